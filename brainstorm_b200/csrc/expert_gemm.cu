@@ -8,20 +8,39 @@
 // out     [L, N] bf16
 // loads   [E] int32 ON THE DEVICE: the kernel never needs them on the host.
 //
-// One persistent CTA per SM walks the list of (expert, 128-row tile, BN-column tile) work
-// items that it derives from `loads` itself.  Roles inside a CTA (192 threads):
+// The weights are the M operand of the MMA and the rows its N operand (the tile computed is
+// out^T): out_features is a multiple of the 128-row half of a tile, while the number of rows of
+// an expert is anything, and N may be any multiple of 16 up to 256.  An expert's rows are cut
+// into ceil(load / 256) equal tiles, so hardly anything is computed for padding; with rows as
+// the M operand every expert's last 128-row tile was computed in full.
+//
+// One persistent CTA pair (kPair = 2: cta_group::2, M = 256, each CTA holds 128 weight rows and
+// half of the tile's rows) or, when out_features is an odd multiple of 128, one CTA (M = 128)
+// walks the list of (expert, row tile, feature tile) work items that it derives from `loads`
+// itself.  Roles inside a CTA (192 threads):
 //   warp 0     one elected lane issues the TMA loads (cp.async.bulk.tensor, 128B swizzle, no
-//              multicast) of the A tile [128 x 64] and the B tile [BN x 64] of every k-block
-//              into a 4-stage shared-memory ring, completion on mbarriers;
-//   warp 1     allocates tensor memory (2 accumulators of 128 lanes x BN fp32 columns), and
-//              one elected lane issues tcgen05.mma (M = 128, N = BN, K = 16, bf16 -> fp32)
-//              four times per k-block, releasing ring slots and publishing finished
-//              accumulators with tcgen05.commit;
-//   warps 2-5  epilogue: tcgen05.ld of the accumulator quarter their warp id selects, optional
-//              ReLU, fp32 -> bf16, 16-byte stores of the rows that exist (row < loads[e]).
+//              multicast) of its weight tile [128 x 64] and of its rows in boxes of 32 x 64 into
+//              a shared-memory ring; the bytes of both CTAs count on the first CTA's mbarrier;
+//   warp 1     allocates tensor memory (2 accumulators of 128 lanes x 256 fp32 columns); one
+//              elected lane of the first CTA issues tcgen05.mma (K = 16) four times per k-block
+//              for the pair, releasing ring slots and publishing accumulators in both CTAs with
+//              tcgen05.commit;
+//   warps 2-5  epilogue: tcgen05.ld of the 32 lanes (features) their warp id selects, optional
+//              ReLU, fp32 -> bf16, transposed through 2 KB of shared memory per warp so that
+//              a row is stored 64 bytes at a time, and only if it exists (row < loads[e]).
 // The second accumulator lets the epilogue of tile i run under the MMAs of tile i + 1.
 // Every mbarrier wait is bounded: after the limit the role records an error and leaves its
-// loop, the CTA frees its tensor memory and returns.
+// loop, the copies in flight are given time to land, the CTAs meet, free their tensor memory
+// and return.
+//
+// What bounds it: HBM reads of the weights for few rows per expert (32 experts of 4 rows, 1024 ->
+// 4096: 48 us, 5.6 TB/s); for many, shared memory and the tensor pipe together: the MMAs of the
+// 1024 -> 4096 layer over 27732 rows take 155 us without their loads, the loads and stores
+// 154 us without the MMAs, both 192 us (1208 TFLOP/s).  Single CTAs with 128 x 256 tiles, rows as
+// the M operand, took 211 us there and moved 2.9 instead of 2.0 GB from L2 to the SMs; 36343
+// rows in 128 very uneven experts, 768 -> 3072, took 222 us and take 185.  The rows come in one
+// box of the size needed: boxes of 32 rows alone cost 12 %.  An L2 prefetch of the weights of
+// the next tile made every shape slower (66 -> 76 us with few rows).
 #include <cuda.h>
 
 #include "common.cuh"
@@ -29,15 +48,23 @@
 namespace brt_b200 {
 namespace {
 
-constexpr int kBM = 128, kBK = 64;  // tile rows; kBK bf16 = one 128-byte swizzle row
-// Tile columns BN are 256 when out_features allows it (the A tile is then used by twice as many
-// multiply-accumulates, which is what keeps the tensor pipe fed from shared memory), else 128.
-constexpr int kStages = 4;
+constexpr int kBM = 128, kBK = 64;  // weight rows per CTA; kBK bf16 = one 128-byte swizzle row
+constexpr int kBN = 256;            // rows of an expert in one tile, at most
+constexpr int kBoxStep = 32;        // the row operand is fetched in one box of 32, 64, 96 or
+constexpr int kBoxSizes = 4;        // 128 rows (two of them when a single CTA needs more)
 constexpr int kUmmaK = 16;
 constexpr int kThreads = 192;
 constexpr int kMaxExperts = 1024;
-constexpr uint32_t kTileBytes = kBM * kBK * 2;  // 16 KB: an A tile, or 128 columns of a B tile
-constexpr int kSpinLimit = 1 << 22;
+constexpr uint32_t kTileBytes = kBM * kBK * 2;         // 16 KB: one CTA's weight tile
+constexpr uint32_t kRowBytes = kBK * 2;                // one row of a k-block
+constexpr unsigned long long kWaitLimitNs = 2000000000ull;  // of one wait
+// ring slots: 32 KB each with a pair (half of the rows per CTA), 48 KB without
+template <int kPair>
+constexpr int kStages = kPair == 2 ? 6 : 4;
+
+struct RowMaps {
+  CUtensorMap box[kBoxSizes];  // box[i]: (i + 1) * kBoxStep rows
+};
 
 struct GemmArgs {
   const int* loads;
@@ -45,7 +72,7 @@ struct GemmArgs {
   int* error;
   int experts;
   int max_path_load;  // 0: packed
-  int n_tiles;        // N / BN
+  int m_tiles;        // N / (128 * kPair)
   int k_blocks;       // K / kBK
   long long N;
   long long total_rows;
@@ -66,10 +93,16 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+__device__ __forceinline__ unsigned long long now_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
 // Bounded wait for the phase with the given parity; false when the limit ran out.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
   const uint32_t addr = smem_u32(bar);
-  for (int spin = 0; spin < kSpinLimit; spin++) {
+  unsigned long long until = 0;
+  for (int spin = 0;; spin++) {
     uint32_t done;
     asm volatile(
         "{\n"
@@ -81,25 +114,56 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
         : "r"(addr), "r"(parity)
         : "memory");
     if (done) return true;
-    if (spin > 64) __nanosleep(32);
+    if (spin > 64) {
+      const unsigned long long now = now_ns();
+      if (until == 0) until = now + kWaitLimitNs;
+      else if (now > until) return false;
+      __nanosleep(32);
+    }
   }
-  return false;
 }
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint64_t* bar,
+// The address of `p`'s twin in the shared memory of CTA `rank` of the cluster.
+__device__ __forceinline__ uint32_t map_to_cta(const void* p, uint32_t rank) {
+  uint32_t addr;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(smem_u32(p)), "r"(rank));
+  return addr;
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr)
+               : "memory");
+}
+// `bar` is a cluster address: with a pair, the copies of both CTAs count on the first one's.
+template <int kPair>
+__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint32_t bar,
                                             int x, int y) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, "
-      "{%3, %4}], [%2];" ::"r"(smem_u32(dst)),
-      "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y)
-      : "memory");
+  if constexpr (kPair == 2)
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2"
+        " [%0], [%1, {%3, %4}], [%2];" ::"r"(smem_u32(dst)),
+        "l"(map), "r"(bar), "r"(x), "r"(y)
+        : "memory");
+  else
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, "
+        "{%3, %4}], [%2];" ::"r"(smem_u32(dst)),
+        "l"(map), "r"(bar), "r"(x), "r"(y)
+        : "memory");
 }
-__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, uint64_t* bar,
+template <int kPair>
+__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, uint32_t bar,
                                             int x, int y, int z) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, "
-      "{%3, %4, %5}], [%2];" ::"r"(smem_u32(dst)),
-      "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z)
-      : "memory");
+  if constexpr (kPair == 2)
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2"
+        " [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_u32(dst)),
+        "l"(map), "r"(bar), "r"(x), "r"(y), "r"(z)
+        : "memory");
+  else
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, "
+        "{%3, %4, %5}], [%2];" ::"r"(smem_u32(dst)),
+        "l"(map), "r"(bar), "r"(x), "r"(y), "r"(z)
+        : "memory");
 }
 
 // Shared-memory matrix descriptor of a K-major tile stored with the 128-byte swizzle (rows of
@@ -115,26 +179,63 @@ __device__ __forceinline__ uint64_t umma_desc(const void* tile) {
   return d;
 }
 // kind::f16 instruction descriptor: fp32 accumulate, bf16 x bf16, both operands K-major.
-template <int BN>
-__device__ __forceinline__ uint32_t umma_idesc() {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) |
-         ((uint32_t)(kBM >> 4) << 24);
+template <int kPair>
+__device__ __forceinline__ uint32_t umma_idesc(int n) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) |
+         ((uint32_t)(kPair * kBM >> 4) << 24);
 }
+template <int kPair>
 __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc,
                                           uint32_t accumulate) {
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
-      "}\n" ::"r"(tmem_d),
-      "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
-      : "memory");
+  if constexpr (kPair == 2)
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "setp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
+        "}\n" ::"r"(tmem_d),
+        "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
+        : "memory");
+  else
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "setp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
+        "}\n" ::"r"(tmem_d),
+        "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
+        : "memory");
 }
+// Arrive on `bar` (with a pair: on both CTAs' barriers at that offset) once every MMA issued
+// before has finished.
+template <int kPair>
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                   smem_u32(bar))
-               : "memory");
+  if constexpr (kPair == 2)
+    asm volatile(
+        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64"
+        " [%0], %1;" ::"r"(smem_u32(bar)),
+        "h"((uint16_t)3)
+        : "memory");
+  else
+    asm volatile(
+        "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+            smem_u32(bar))
+        : "memory");
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// All threads of the pair (or of the CTA).
+template <int kPair>
+__device__ __forceinline__ void group_sync() {
+  if constexpr (kPair == 2) {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  } else {
+    __syncthreads();
+  }
 }
 __device__ __forceinline__ void tmem_load_32(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile(
@@ -150,82 +251,118 @@ __device__ __forceinline__ void tmem_load_32(uint32_t taddr, uint32_t (&r)[32]) 
       : "memory");
 }
 
-template <int BN>
+template <int kPair>
 struct alignas(1024) GemmSmem {
-  unsigned char a[kStages][kTileBytes];
-  unsigned char b[kStages][kTileBytes * (BN / 128)];
-  uint64_t full[kStages];
-  uint64_t empty[kStages];
+  unsigned char a[kStages<kPair>][kTileBytes];
+  unsigned char b[kStages<kPair>][kBN / kPair * kBK * 2];
+  __nv_bfloat16 turn[4][2][32 * 32];  // per epilogue warp, two buffers: [row][feature]
+  uint64_t full[kStages<kPair>];
+  uint64_t empty[kStages<kPair>];
   uint64_t acc_full[2];
   uint64_t acc_empty[2];
   uint32_t tmem_base;
   int first_tile[kMaxExperts + 1];  // exclusive prefix of the tiles per expert
   int row_base[kMaxExperts];
+  int load[kMaxExperts];
 };
 
 struct TileAt {
-  int expert, m_tile, n_tile;
+  int expert, m_tile;
+  int row0, rows;  // within the expert
+  int width;       // columns of the MMA: rows of a tile, rounded up to 16
 };
-template <int BN>
-__device__ __forceinline__ TileAt tile_at(const GemmSmem<BN>& s, int experts, int n_tiles, int t) {
+template <int kPair>
+__device__ __forceinline__ TileAt tile_at(const GemmSmem<kPair>& s, int experts, int m_tiles,
+                                          int t) {
   int lo = 0, hi = experts - 1;  // last expert whose first tile is <= t (empty ones skipped)
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
     if (s.first_tile[mid] <= t) lo = mid; else hi = mid - 1;
   }
   const int local = t - s.first_tile[lo];
+  const int load = s.load[lo];
+  const int parts = (load + kBN - 1) / kBN;
+  const int each = ((load + parts - 1) / parts + 15) & ~15;
+  const int part = local / m_tiles;
   TileAt at;
   at.expert = lo;
-  at.m_tile = local / n_tiles;
-  at.n_tile = local - at.m_tile * n_tiles;
+  at.m_tile = local - part * m_tiles;
+  at.row0 = part * each;
+  at.rows = load - at.row0 < each ? load - at.row0 : each;  // <= 0: rounding left none
+  at.width = each;
   return at;
 }
 
-template <int BN>
+template <int kPair>
 __global__ void __launch_bounds__(kThreads, 1)
-expert_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
-                   const __grid_constant__ CUtensorMap map_b, const GemmArgs g) {
-  constexpr uint32_t kTmemCols = 2 * BN;
-  constexpr uint32_t kStageBytes = kTileBytes + kTileBytes * (BN / 128);
+expert_gemm_kernel(const __grid_constant__ CUtensorMap map_w,
+                   const __grid_constant__ RowMaps map_r, const GemmArgs g) {
+  constexpr uint32_t kTmemCols = 2 * kBN;
+  constexpr int kRing = kStages<kPair>;
   extern __shared__ __align__(1024) unsigned char s_raw[];
-  GemmSmem<BN>& s = *reinterpret_cast<GemmSmem<BN>*>(
+  GemmSmem<kPair>& s = *reinterpret_cast<GemmSmem<kPair>*>(
       (reinterpret_cast<uintptr_t>(s_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
   const int lane = tid & 31;
+  const uint32_t rank = kPair == 2 ? cluster_rank() : 0;
+  const int group = blockIdx.x / kPair;
+  const int groups = gridDim.x / kPair;
 
-  // tiles per expert and the first row of every expert (serial scan: E is small)
-  if (tid == 0) {
+  if (warp == 0) {  // tiles per expert and the first row of every expert
     int tiles = 0, row = 0;
-    for (int e = 0; e < g.experts; e++) {
-      int load = g.loads[e];
+    for (int p = 0; p < g.experts; p += 32) {
+      const int e = p + lane;
+      int load = e < g.experts ? g.loads[e] : 0;
       if (load < 0) load = 0;
       if (g.max_path_load != 0 && load > g.max_path_load) load = g.max_path_load;
-      s.first_tile[e] = tiles;
-      s.row_base[e] = g.max_path_load != 0 ? e * g.max_path_load : row;
-      tiles += (load + kBM - 1) / kBM * g.n_tiles;
-      row += load;
+      const int mine = (load + kBN - 1) / kBN * g.m_tiles;
+      int tiles_incl = mine, rows_incl = load;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int tn = __shfl_up_sync(0xffffffffu, tiles_incl, d);
+        const int rn = __shfl_up_sync(0xffffffffu, rows_incl, d);
+        if (lane >= d) { tiles_incl += tn; rows_incl += rn; }
+      }
+      if (e < g.experts) {
+        s.first_tile[e] = tiles + tiles_incl - mine;
+        s.row_base[e] = g.max_path_load != 0 ? e * g.max_path_load : row + rows_incl - load;
+        s.load[e] = load;
+      }
+      tiles += __shfl_sync(0xffffffffu, tiles_incl, 31);
+      row += __shfl_sync(0xffffffffu, rows_incl, 31);
     }
-    s.first_tile[g.experts] = tiles;
-    for (int i = 0; i < kStages; i++) {
-      mbar_init(&s.full[i], 1);
-      mbar_init(&s.empty[i], 1);
+    if (lane == 0) {
+      s.first_tile[g.experts] = tiles;
+      for (int i = 0; i < kRing; i++) {
+        mbar_init(&s.full[i], 1);
+        mbar_init(&s.empty[i], 1);
+      }
+      for (int i = 0; i < 2; i++) {
+        mbar_init(&s.acc_full[i], 1);
+        mbar_init(&s.acc_empty[i], 4 * kPair);  // one arrival per epilogue warp
+      }
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    for (int i = 0; i < 2; i++) {
-      mbar_init(&s.acc_full[i], 1);
-      mbar_init(&s.acc_empty[i], 4);  // one arrival per epilogue warp
-    }
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     smem_u32(&s.tmem_base)),
-                 "r"(kTmemCols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    if constexpr (kPair == 2) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                       smem_u32(&s.tmem_base)),
+                   "r"(kTmemCols)
+                   : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                       smem_u32(&s.tmem_base)),
+                   "r"(kTmemCols)
+                   : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  group_sync<kPair>();  // the peer's barriers exist
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = s.tmem_base;
   const int total_tiles = s.first_tile[g.experts];
@@ -235,29 +372,43 @@ expert_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
     if (lane == 0) {
       int slot = 0;
       uint32_t phase = 0;
-      for (int t = blockIdx.x; t < total_tiles && !failed; t += gridDim.x) {
-        const TileAt at = tile_at(s, g.experts, g.n_tiles, t);
-        const int row0 = s.row_base[at.expert] + at.m_tile * kBM;
+      for (int t = group; t < total_tiles && !failed; t += groups) {
+        const TileAt at = tile_at(s, g.experts, g.m_tiles, t);
+        const int half = at.width / kPair;  // rows this CTA stages (a multiple of 8)
+        const int boxes = half > kBoxSizes * kBoxStep ? 2 : 1;
+        const int size = (half / boxes + kBoxStep - 1) / kBoxStep;  // half / 2 is a multiple of 8
+        const int box_rows = size * kBoxStep;
+        const CUtensorMap* const map_box = &map_r.box[size - 1];
+        const int row0 = s.row_base[at.expert] + at.row0 + (int)rank * half;
+        const int feature0 = (at.m_tile * kPair + (int)rank) * kBM;
+        const uint32_t bytes = kPair * (kTileBytes + (uint32_t)(boxes * box_rows) * kRowBytes);
         for (int kb = 0; kb < g.k_blocks; kb++) {
           if (!mbar_wait(&s.empty[slot], phase ^ 1)) { failed = true; break; }
-          mbar_expect_tx(&s.full[slot], kStageBytes);
-          tma_load_2d(s.a[slot], &map_a, &s.full[slot], kb * kBK, row0);
-          tma_load_3d(s.b[slot], &map_b, &s.full[slot], kb * kBK, at.n_tile * BN, at.expert);
-          if (++slot == kStages) { slot = 0; phase ^= 1; }
+          if (rank == 0) mbar_expect_tx(&s.full[slot], bytes);
+          const uint32_t bar = kPair == 2 ? map_to_cta(&s.full[slot], 0) : smem_u32(&s.full[slot]);
+          tma_load_3d<kPair>(s.a[slot], &map_w, bar, kb * kBK, feature0, at.expert);
+          for (int b = 0; b < boxes; b++)
+            tma_load_2d<kPair>(s.b[slot] + b * box_rows * kRowBytes, map_box, bar, kb * kBK,
+                               row0 + b * box_rows);
+          if (++slot == kRing) { slot = 0; phase ^= 1; }
         }
       }
+      // copies still in flight land before the CTA's shared memory is given back
+      if (failed)
+        for (int i = 0; i < 1024; i++) __nanosleep(1000);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = umma_idesc<BN>();
+    if (lane == 0 && rank == 0) {
       int slot = 0;
       uint32_t phase = 0;
       int acc = 0;
       uint32_t acc_phase = 0;
-      for (int t = blockIdx.x; t < total_tiles && !failed; t += gridDim.x) {
+      for (int t = group; t < total_tiles && !failed; t += groups) {
+        const TileAt at = tile_at(s, g.experts, g.m_tiles, t);
+        const uint32_t idesc = umma_idesc<kPair>(at.width);
         if (!mbar_wait(&s.acc_empty[acc], acc_phase ^ 1)) { failed = true; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t d = tmem + (uint32_t)acc * BN;
+        const uint32_t d = tmem + (uint32_t)acc * kBN;
         for (int kb = 0; kb < g.k_blocks; kb++) {
           if (!mbar_wait(&s.full[slot], phase)) { failed = true; break; }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -266,67 +417,85 @@ expert_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
 #pragma unroll
           for (int k = 0; k < kBK / kUmmaK; k++) {
             // 16 bf16 = 32 bytes further along K inside the swizzled row: +2 in 16-byte units
-            umma_bf16(d, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
+            umma_bf16<kPair>(d, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
           }
-          umma_commit(&s.empty[slot]);  // the slot is free once these MMAs have read it
-          if (++slot == kStages) { slot = 0; phase ^= 1; }
+          umma_commit<kPair>(&s.empty[slot]);  // free once these MMAs have read the slot
+          if (++slot == kRing) { slot = 0; phase ^= 1; }
         }
         if (failed) break;
-        umma_commit(&s.acc_full[acc]);  // the accumulator is complete once they have finished
+        umma_commit<kPair>(&s.acc_full[acc]);  // complete once they have finished
         if (++acc == 2) { acc = 0; acc_phase ^= 1; }
       }
     }
   } else {
-    // epilogue: this warp reads the 32 accumulator lanes (tile rows) of quarter warp % 4
+    // epilogue: this warp reads the 32 accumulator lanes (features) of quarter warp % 4
     const int quarter = warp & 3;
     int acc = 0;
     uint32_t acc_phase = 0;
-    for (int t = blockIdx.x; t < total_tiles && !failed; t += gridDim.x) {
-      const TileAt at = tile_at(s, g.experts, g.n_tiles, t);
-      int load = g.loads[at.expert];
-      if (g.max_path_load != 0 && load > g.max_path_load) load = g.max_path_load;
-      const int row_in_expert = at.m_tile * kBM + quarter * 32 + lane;
-      const long long row = (long long)s.row_base[at.expert] + row_in_expert;
+    int buffer = 0;
+    const int my_row = lane >> 2;         // of 8 rows stored at a time
+    const int my_piece = (lane & 3) * 8;  // 16 bytes of the row's 64
+    for (int t = group; t < total_tiles && !failed; t += groups) {
+      const TileAt at = tile_at(s, g.experts, g.m_tiles, t);
+      const long long first_row = (long long)s.row_base[at.expert] + at.row0;
+      const long long left = g.total_rows - first_row;
+      const int rows = at.rows < left ? at.rows : (int)(left > 0 ? left : 0);
+      __nv_bfloat16* const out =
+          g.out + first_row * g.N + (long long)(at.m_tile * kPair + (int)rank) * kBM +
+          quarter * 32 + my_piece;
       if (!mbar_wait(&s.acc_full[acc], acc_phase)) { failed = true; break; }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll 1
-      for (int c0 = 0; c0 < BN; c0 += 32) {
+      for (int c0 = 0; c0 < rows; c0 += 32) {
         uint32_t v[32];
-        tmem_load_32(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * BN + c0), v);
+        tmem_load_32(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * kBN + c0), v);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (row_in_expert < load && row < g.total_rows) {
-          uint4* dst = reinterpret_cast<uint4*>(g.out + row * g.N + (long long)at.n_tile * BN + c0);
+        // two buffers: the barrier below also says that everybody has read this one's last rows
+        __nv_bfloat16* const turn = s.turn[quarter][buffer];
+        buffer ^= 1;
 #pragma unroll
-          for (int q = 0; q < 4; q++) {
-            uint32_t w[4];
+        for (int i = 0; i < 16; i++) {
+          float lo = __uint_as_float(v[2 * i]);
+          float hi = __uint_as_float(v[2 * i + 1]);
+          if (g.relu) { lo = fmaxf(lo, 0.f); hi = fmaxf(hi, 0.f); }
+          const __nv_bfloat162 p = __floats2bfloat162_rn(lo, hi);
+          turn[(2 * i) * 32 + lane] = p.x;
+          turn[(2 * i + 1) * 32 + lane] = p.y;
+        }
+        __syncwarp();
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-              float lo = __uint_as_float(v[q * 8 + 2 * i]);
-              float hi = __uint_as_float(v[q * 8 + 2 * i + 1]);
-              if (g.relu) { lo = fmaxf(lo, 0.f); hi = fmaxf(hi, 0.f); }
-              const __nv_bfloat162 p = __floats2bfloat162_rn(lo, hi);
-              w[i] = *reinterpret_cast<const uint32_t*>(&p);
-            }
-            dst[q] = make_uint4(w[0], w[1], w[2], w[3]);
-          }
+        for (int i = 0; i < 4; i++) {
+          const int r = i * 8 + my_row;
+          if (c0 + r < rows)
+            *reinterpret_cast<uint4*>(out + (long long)(c0 + r) * g.N) =
+                *reinterpret_cast<const uint4*>(turn + r * 32 + my_piece);
         }
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
-      if (lane == 0) mbar_arrive(&s.acc_empty[acc]);
+      if (lane == 0) {
+        if (rank == 0) mbar_arrive(&s.acc_empty[acc]);
+        else mbar_arrive_cluster(map_to_cta(&s.acc_empty[acc], 0));
+      }
       if (++acc == 2) { acc = 0; acc_phase ^= 1; }
     }
   }
   if (failed) atomicExch(g.error, BRT_ERR_TIMEOUT);
-  __syncwarp();  // the single-lane roles rejoin their warps before the CTA barrier
+  __syncwarp();  // the single-lane roles rejoin their warps before the barrier
 
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
+  group_sync<kPair>();  // nobody leaves while the peer may still signal its barriers
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  if (warp == 1)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
-                 "r"(kTmemCols)
-                 : "memory");
+  if (warp == 1) {
+    if constexpr (kPair == 2)
+      asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem),
+                   "r"(kTmemCols)
+                   : "memory");
+    else
+      asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
+                   "r"(kTmemCols)
+                   : "memory");
+  }
 }
 
 }  // namespace
@@ -355,6 +524,36 @@ EncodeTiledFn encode_tiled() {
   return fn;
 }
 
+template <int kPair>
+int launch_expert_gemm(const CUtensorMap& map_w, const RowMaps& map_r, const GemmArgs& g,
+                       cudaStream_t st) {
+  const size_t smem = sizeof(GemmSmem<kPair>) + 1024;
+  static thread_local int configured_device = -1;
+  int dev = 0;
+  BRT_CUDA_TRY(cudaGetDevice(&dev));
+  if (configured_device != dev) {
+    BRT_CUDA_TRY(cudaFuncSetAttribute(expert_gemm_kernel<kPair>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    configured_device = dev;
+  }
+  cudaLaunchAttribute cluster;
+  cluster.id = cudaLaunchAttributeClusterDimension;
+  cluster.val.clusterDim.x = kPair;
+  cluster.val.clusterDim.y = 1;
+  cluster.val.clusterDim.z = 1;
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3((unsigned)(sm_count() / kPair * kPair));
+  config.blockDim = dim3(kThreads);
+  config.dynamicSmemBytes = smem;
+  config.stream = st;
+  config.attrs = &cluster;
+  config.numAttrs = 1;
+  const KernelTimer timer("expert_gemm_kernel", st);
+  BRT_CUDA_TRY(cudaLaunchKernelEx(&config, expert_gemm_kernel<kPair>, map_w, map_r, g));
+  note_launch();
+  return BRT_OK;
+}
+
 }  // namespace
 
 extern "C" {
@@ -374,7 +573,9 @@ BRT_API int brt_grouped_expert_gemm(const void* rows, const void* weights, void*
                      "the tensor-core expert GEMM needs in_features %% %d == 0 and "
                      "out_features %% 128 == 0 (got %lld, %lld)",
                      kBK, (long long)in_features, (long long)out_features);
-  const int bn = out_features % 256 == 0 ? 256 : 128;
+  // a pair of CTAs computes 256 features; an odd multiple of 128 leaves half a pair idle on
+  // the last tile, and single CTAs do not
+  const int pair = out_features % 256 == 0 ? 2 : 1;
   if (total_rows == 0) return BRT_OK;
   BRT_REQUIRE(rows != nullptr && weights != nullptr && out != nullptr, "null pointer argument");
   BRT_REQUIRE(aligned_to(rows, 16) && aligned_to(weights, 16) && aligned_to(out, 16),
@@ -384,13 +585,14 @@ BRT_API int brt_grouped_expert_gemm(const void* rows, const void* weights, void*
   if (encode == nullptr)
     return set_error(BRT_ERR_CUDA, "the driver does not offer cuTensorMapEncodeTiled");
 
-  alignas(64) CUtensorMap map_a, map_b;
-  {
+  alignas(64) CUtensorMap map_w;
+  alignas(64) RowMaps map_r;
+  for (int i = 0; i < kBoxSizes; i++) {
     const cuuint64_t dims[2] = {(cuuint64_t)in_features, (cuuint64_t)total_rows};
     const cuuint64_t strides[1] = {(cuuint64_t)in_features * 2};
-    const cuuint32_t box[2] = {kBK, kBM};
+    const cuuint32_t box[2] = {kBK, (cuuint32_t)((i + 1) * kBoxStep)};
     const cuuint32_t elem[2] = {1, 1};
-    const CUresult r = encode(&map_a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
+    const CUresult r = encode(&map_r.box[i], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
                               const_cast<void*>(rows), dims, strides, box, elem,
                               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                               CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -403,9 +605,9 @@ BRT_API int brt_grouped_expert_gemm(const void* rows, const void* weights, void*
                                 (cuuint64_t)path_num};
     const cuuint64_t strides[2] = {(cuuint64_t)in_features * 2,
                                    (cuuint64_t)in_features * out_features * 2};
-    const cuuint32_t box[3] = {kBK, (cuuint32_t)bn, 1};
+    const cuuint32_t box[3] = {kBK, kBM, 1};
     const cuuint32_t elem[3] = {1, 1, 1};
-    const CUresult r = encode(&map_b, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3,
+    const CUresult r = encode(&map_w, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3,
                               const_cast<void*>(weights), dims, strides, box, elem,
                               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                               CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -419,36 +621,15 @@ BRT_API int brt_grouped_expert_gemm(const void* rows, const void* weights, void*
   g.error = static_cast<int*>(error_word);
   g.experts = path_num;
   g.max_path_load = max_path_load;
-  g.n_tiles = (int)(out_features / bn);
+  g.m_tiles = (int)(out_features / (kBM * pair));
   g.k_blocks = (int)(in_features / kBK);
   g.N = out_features;
   g.total_rows = total_rows;
   g.relu = relu != 0;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  int dev = 0;
-  BRT_CUDA_TRY(cudaGetDevice(&dev));
-  const KernelTimer timer("expert_gemm_kernel", st);
-  if (bn == 256) {
-    const size_t smem = sizeof(GemmSmem<256>) + 1024;
-    static thread_local int configured_device = -1;
-    if (configured_device != dev) {
-      BRT_CUDA_TRY(cudaFuncSetAttribute(expert_gemm_kernel<256>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      configured_device = dev;
-    }
-    expert_gemm_kernel<256><<<(unsigned)sm_count(), kThreads, smem, st>>>(map_a, map_b, g),
-        note_launch();
-  } else {
-    const size_t smem = sizeof(GemmSmem<128>) + 1024;
-    static thread_local int configured_device = -1;
-    if (configured_device != dev) {
-      BRT_CUDA_TRY(cudaFuncSetAttribute(expert_gemm_kernel<128>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      configured_device = dev;
-    }
-    expert_gemm_kernel<128><<<(unsigned)sm_count(), kThreads, smem, st>>>(map_a, map_b, g),
-        note_launch();
-  }
+  const int rc = pair == 2 ? launch_expert_gemm<2>(map_w, map_r, g, st)
+                           : launch_expert_gemm<1>(map_w, map_r, g, st);
+  if (rc != BRT_OK) return rc;
   BRT_LAUNCH_CHECK("expert_gemm_kernel");
   return BRT_OK;
 }
