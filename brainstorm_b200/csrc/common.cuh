@@ -69,6 +69,11 @@ __device__ __forceinline__ void cp_async_16(void* smem_dst, const void* gmem_src
   const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem_dst));
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem_src) : "memory");
 }
+// 4 bytes (through L1: the .cg form only takes 16).
+__device__ __forceinline__ void cp_async_4(void* smem_dst, const void* gmem_src) {
+  const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem_dst));
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gmem_src) : "memory");
+}
 // The same copy with an L2 eviction policy (createpolicy) attached to the line it reads.
 __device__ __forceinline__ unsigned long long l2_evict_first_policy() {
   unsigned long long p;
@@ -90,6 +95,12 @@ template <int N>
 __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
+
+// ---- route records: the first routes of a cell, as the index scan leaves them ---------------
+// kRecordRoutes x (path, seat), ascending paths, seat 0 = none; kRecordMore in the first path:
+// the record does not hold all routes of the cell, read its index row instead.
+constexpr int kRecordRoutes = 4;
+constexpr int kRecordMore = 0x40000000;
 
 // ---- device-side conversion between storage types and fp32 ---------------------------------
 

@@ -20,17 +20,18 @@
 // the bit words, so the integer semantics of the reference (index = running sum * mask
 // value) hold for any int32 mask.
 //
-// Two implementations of pack/expand share that plan:
-//   * the tiled path (path_num % 4 == 0, 16-byte aligned arrays): a CTA stages a
-//     [32*k cells, <=256 paths] tile in shared memory with fully coalesced 16-byte loads
-//     (every load of the tile is in flight at once), each warp turns a 32x32 block into
-//     column bit words with a 5-step shuffle transpose, and `expand` is one popcount per
-//     output element with coalesced 16-byte stores.  Whenever the bit words of a CTA's
-//     share of the mask fit in shared memory the three steps run as ONE launch (the
-//     chained path): a CTA packs a run of consecutive tiles, publishes the run's column
-//     sums, adds up the sums of the runs before it (a bounded wait on CTAs that started
-//     earlier) and expands its tiles from shared memory;
-//   * the strip path (any path_num / alignment): a thread walks 32 cells of V paths.
+// Three implementations share that plan:
+//   * the chained path, ONE launch, whenever the bit words of a CTA's share of the mask fit
+//     in shared memory (any path count up to 256, and wider masks of 4 * n aligned paths): a
+//     CTA packs a run of consecutive tiles with asynchronous copies, publishes the run's
+//     column sums, adds up the sums of the runs before it (a bounded wait on CTAs that started
+//     earlier) and writes its indices from shared memory;
+//   * the tiled path for larger masks (path_num % 4 == 0, 16-byte aligned arrays), three
+//     launches: a CTA stages a [32*k cells, <=256 paths] tile in shared memory with fully
+//     coalesced 16-byte loads, each warp turns a 32x32 block into column bit words with a
+//     5-step shuffle transpose, and `expand` is one popcount per output element with coalesced
+//     16-byte stores;
+//   * the strip path for the rest: a thread walks 32 cells of V paths.
 
 #include <atomic>
 #include <cstdlib>
@@ -49,10 +50,18 @@ constexpr int kGroupRows = 32;  // cells per bit word
 
 // Where the launch under way writes the per-path cell counts of the indices it produces
 // (null: nowhere).  Set by the entry points around their call into the launch helpers.
+// The same for the cells' route records (chained path only).
 thread_local int32_t* t_counts_out = nullptr;
+thread_local void* t_records_out = nullptr;
 struct CountsScope {
-  explicit CountsScope(int32_t* p) { t_counts_out = p; }
-  ~CountsScope() { t_counts_out = nullptr; }
+  explicit CountsScope(int32_t* counts, void* records = nullptr) {
+    t_counts_out = counts;
+    t_records_out = records;
+  }
+  ~CountsScope() {
+    t_counts_out = nullptr;
+    t_records_out = nullptr;
+  }
 };
 
 // kMask: write the 0/1 mask itself.  kThrottleSeat: seat indices and loads of the throttled
@@ -606,35 +615,6 @@ __device__ __forceinline__ void pack_staged(const TileCtx& x, const TileSmem& sm
   __syncthreads();
 }
 
-// Start the asynchronous copy of one tile of the mask into `stage` (rows beyond the mask
-// are zero-filled with plain stores) and zero the tile's bit words.  The caller commits the
-// group, waits for it and passes a CTA barrier before pack_staged.
-__device__ __forceinline__ void stage_tile_async(const TileCtx& x, int* stage, int* bits,
-                                                 const int* __restrict__ mask) {
-  const int tid = threadIdx.x;
-  const int col0 = x.chunk * x.ec;
-  const int cols = (x.path_num - col0) < x.ec ? (x.path_num - col0) : x.ec;
-  const int64_t row0 = x.tile * x.rg * kGroupRows;
-  const int tile_rows = x.rg * kGroupRows;
-  const int vec_per_row = cols >> 2;
-  const int total_vecs = tile_rows * vec_per_row;
-  for (int i = tid; i < x.rg * x.ec; i += kTileThreads) bits[i] = 0;
-  const int step_r = kTileThreads / vec_per_row;
-  const int step_q = kTileThreads - step_r * vec_per_row;
-  int r = tid / vec_per_row;
-  int q = tid - r * vec_per_row;
-  for (int idx = tid; idx < total_vecs; idx += kTileThreads) {
-    int* dst = stage + r * x.pitch + 4 * q;
-    if (row0 + r < x.cell_num)
-      cp_async_16(dst, mask + (row0 + r) * x.path_num + col0 + 4 * q);
-    else
-      *reinterpret_cast<int4*>(dst) = make_int4(0, 0, 0, 0);
-    r += step_r;
-    q += step_q;
-    if (q >= vec_per_row) { q -= vec_per_row; r += 1; }
-  }
-}
-
 // Stage one tile of the mask and turn it into column bit words (kept in shared memory at
 // sm.bits, and written to `bits_out` when that is not null).  The tile's column sums are
 // ADDED to sm.sum / sm.extra and a value other than 0/1 sets sm.flag: the caller zeroes the
@@ -853,8 +833,7 @@ __device__ __forceinline__ void expand_general(const TileCtx& x, const int* __re
 // of an earlier tile is no longer read.
 template <Mode MODE>
 __device__ __forceinline__ void expand_binary(const TileCtx& x, const TileSmem& sm, int& run,
-                                              int* __restrict__ out,
-                                              int* __restrict__ mask_out = nullptr) {
+                                              int* __restrict__ out) {
   const int tid = threadIdx.x;
   const int col0 = x.chunk * x.ec;
   const int cols = (x.path_num - col0) < x.ec ? (x.path_num - col0) : x.ec;
@@ -891,10 +870,6 @@ __device__ __forceinline__ void expand_binary(const TileCtx& x, const TileSmem& 
       const int seat = b[j] + __popc(w[j] & low);
       if constexpr (MODE == Mode::kThrottle)
         v[j] = (bit && seat <= sm.thr[4 * q + j]) ? 1 : 0;
-      else if constexpr (MODE == Mode::kThrottleSeat)
-        v[j] = (bit && seat <= sm.thr[4 * q + j]) ? seat : 0;
-      else if constexpr (MODE == Mode::kMask)
-        v[j] = bit;
       else
         v[j] = bit ? seat : 0;
     }
@@ -908,11 +883,6 @@ __device__ __forceinline__ void expand_binary(const TileCtx& x, const TileSmem& 
     } else {
       __stcs(reinterpret_cast<int4*>(out + row * x.path_num + col0 + 4 * q),
              make_int4(v[0], v[1], v[2], v[3]));
-      if constexpr (MODE == Mode::kThrottleSeat || MODE == Mode::kSeat) {
-        if (mask_out != nullptr)  // the (throttled) 0/1 mask itself, for callers that want both
-          __stcs(reinterpret_cast<int4*>(mask_out + row * x.path_num + col0 + 4 * q),
-                 make_int4(v[0] != 0, v[1] != 0, v[2] != 0, v[3] != 0));
-      }
     }
     r += step_r;
     q += step_q;
@@ -1042,120 +1012,198 @@ __device__ __forceinline__ float key_score(unsigned key) {
   return __uint_as_float(u);
 }
 
-// PER scores per lane, L lanes per row (L < 32 only with PER == 1: 32 / L rows per warp).
-// A pick costs two warp reductions: the largest key among the row's unpicked scores, then
-// the lowest path that holds it.
-template <int PER, int L>
-__device__ __forceinline__ void gate_rows_as(const TileCtx& x, const int* stage, int* bits,
-                                             int* sums, const GateArgs& g) {
-  constexpr int kRowsPerWarp = 32 / L;
-  const int lane = threadIdx.x & 31;
-  const int warp = threadIdx.x >> 5;
-  const int sub = lane / L;
-  const int l = lane - sub * L;
-  const unsigned members = L == 32 ? 0xffffffffu : (((1u << L) - 1u) << (sub * L));
+// One row per kTileThreads / (rows of the tile) neighbouring threads, 4 to 32 paths per thread
+// (a tile holds 32 * rg rows of at most 256 / rg paths), so the decision is made in registers
+// and a few shuffles.  (A warp per row with two warp reductions per pick took 300
+// instructions per row of 128 paths; this takes 30.)
+//
+// A thread's paths are read as int4 in an order rotated by its place in the row, so that the
+// 8 lanes of a shared-memory phase hit different banks (the pitch is 4 modulo 32 for the wide
+// rows).  A pick: the largest key of every int4 is kept, the largest of those is met over the
+// row's threads, and its owner (the lowest path wins) looks into the int4 again.
+// Leaves the row's picks as words of 32 paths at row_words[row * words per row + word] and,
+// with gates_out, the renormalised gates in the staged tile.
+__device__ __forceinline__ void gate_rows(const TileCtx& x, int* stage, unsigned* row_words,
+                                          const GateArgs& g) {
+  const int tid = threadIdx.x;
+  const int lane = tid & 31;
   const int cols = x.path_num;  // a gated tile spans every path
-  const int64_t row0 = x.tile * x.rg * kGroupRows;
-  const int tile_rows = x.rg * kGroupRows;
-  // column bit words of the 32-cell group this lane is in, for the rows it has seen so far;
-  // handed to shared memory (where the other warps' rows of the group meet) when the group
-  // changes
-  unsigned word[PER];
+  const int per_row = kTileWarps / x.rg;  // threads per row: 1, 2, 4 or 8
+  const int r = tid / per_row;
+  const int p = tid - r * per_row;
+  // paths per thread: the smallest power of two from 4 on that covers the row
+  int per_thread = 4;
+  while (per_thread * per_row < cols) per_thread <<= 1;
+  const int vecs = per_thread >> 2;
+  const int c0 = p * per_thread;
+  const int rot = (c0 >> 5) * (8 / per_row);
+  int* const row = stage + r * x.pitch + c0;
+  const unsigned members = ((1u << per_row) - 1u) << (lane - p);
+  unsigned word = 0;
+  float denom = 0.f;
+  if (g.kind == 1) {
+    unsigned top[8];
 #pragma unroll
-  for (int i = 0; i < PER; i++) word[i] = 0;
-  int group = 0;
-  auto flush = [&]() {
-#pragma unroll
-    for (int i = 0; i < PER; i++) {
-      if (word[i] != 0) {
-        const int c = l + L * i;
-        atomicOr(reinterpret_cast<unsigned*>(bits) + group * x.ec + c, word[i]);
-        atomicAdd(sums + c, __popc(word[i]));
-        word[i] = 0;
+    for (int q = 0; q < 8; q++) {
+      const int at = 4 * ((q + rot) & (vecs - 1));
+      top[q] = 0u;
+      if (q < vecs && c0 + at < cols) {
+        const int4 v = *reinterpret_cast<const int4*>(row + at);
+        top[q] = max(max(score_key(v.x), score_key(v.y)), max(score_key(v.z), score_key(v.w)));
       }
     }
-  };
-  for (int r = warp * kRowsPerWarp + sub; r < tile_rows; r += kTileWarps * kRowsPerWarp) {
-    const int64_t row = row0 + r;
-    if (row >= x.cell_num) break;  // uniform per row group; later rows were staged as zeros
-    if ((r >> 5) != group) {
-      flush();
-      group = r >> 5;
-    }
-    const int* p = stage + r * x.pitch;
-    unsigned key[PER];
+    for (int t = 0; t < g.top_k; t++) {
+      unsigned mine = top[0];
 #pragma unroll
-    for (int i = 0; i < PER; i++) {
-      const int c = l + L * i;
-      key[i] = c < cols ? score_key(p[c]) : 0u;
-    }
-    unsigned picked = 0;
-    float denom = 0.f;
-    if (g.kind == 1) {
-      for (int t = 0; t < g.top_k; t++) {
-        unsigned mine = 0;
+      for (int q = 1; q < 8; q++) mine = max(mine, top[q]);
+      unsigned best = mine;
+      for (int d = 1; d < per_row; d <<= 1)
+        best = max(best, __shfl_xor_sync(0xffffffffu, best, d));
+      if (best != 0u) denom = __fadd_rn(denom, key_score(best));  // 0: fewer paths than top_k
+      const unsigned holders = __ballot_sync(0xffffffffu, mine == best && best != 0u) & members;
+      if (holders != 0u && lane == __ffs(holders) - 1) {
+        int at = 32;
 #pragma unroll
-        for (int i = 0; i < PER; i++)
-          if (!((picked >> i) & 1u) && key[i] > mine) mine = key[i];
-        const unsigned best = __reduce_max_sync(members, mine);
-        if (best == 0u) break;  // fewer paths than top_k
-        unsigned my_col = 0xffffffffu;
+        for (int q = 0; q < 8; q++) {
+          const int here = 4 * ((q + rot) & (vecs - 1));
+          if (q < vecs && top[q] == best && here < at) at = here;
+        }
+        const int4 v = *reinterpret_cast<const int4*>(row + at);
+        const unsigned key[4] = {score_key(v.x), score_key(v.y), score_key(v.z), score_key(v.w)};
+        const unsigned taken = word >> at;
+        unsigned rest = 0u;
+        bool found = false;
 #pragma unroll
-        for (int i = PER - 1; i >= 0; i--)
-          if (!((picked >> i) & 1u) && key[i] == best) my_col = l + L * i;
-        const unsigned col = __reduce_min_sync(members, my_col);
-        if (col == my_col) picked |= 1u << (col / L);
-        denom = __fadd_rn(denom, key_score(best));
+        for (int j = 0; j < 4; j++) {
+          if ((taken >> j) & 1u) continue;
+          if (!found && key[j] == best) {
+            found = true;
+            word |= 1u << (at + j);
+          } else {
+            rest = max(rest, key[j]);
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < 8; q++)
+          if (q < vecs && 4 * ((q + rot) & (vecs - 1)) == at) top[q] = rest;
       }
-    } else {
-#pragma unroll
-      for (int i = 0; i < PER; i++)
-        if (l + L * i < cols && key_score(key[i]) > g.threshold) picked |= 1u << i;
-      if (g.residual_path >= 0 && __ballot_sync(members, picked != 0) == 0 &&
-          (g.residual_path % L) == l)
-        picked |= 1u << (g.residual_path / L);
     }
-    const int rr = r & 31;
+  } else {
 #pragma unroll
-    for (int i = 0; i < PER; i++) word[i] |= ((picked >> i) & 1u) << rr;
-    if (g.gates_out != nullptr) {
-      denom = fmaxf(denom, 1.1920928955078125e-07f);
+    for (int q = 0; q < 8; q++) {
+      const int at = 4 * ((q + rot) & (vecs - 1));
+      if (q < vecs && c0 + at < cols) {
+        const int4 v = *reinterpret_cast<const int4*>(row + at);
+        unsigned four = __int_as_float(v.x) > g.threshold ? 1u : 0u;
+        four |= __int_as_float(v.y) > g.threshold ? 2u : 0u;
+        four |= __int_as_float(v.z) > g.threshold ? 4u : 0u;
+        four |= __int_as_float(v.w) > g.threshold ? 8u : 0u;
+        word |= four << at;
+      }
+    }
+    const unsigned anyone = __ballot_sync(0xffffffffu, word != 0u) & members;
+    if (g.residual_path >= 0 && anyone == 0u && g.residual_path / per_thread == p)
+      word = 1u << (g.residual_path & (per_thread - 1));
+  }
+  if (x.tile * x.rg * kGroupRows + r >= x.cell_num) word = 0u;  // a row the tile only pads
+  unsigned joined = word << (c0 & 31);
+  for (int d = 1; d * per_thread < 32 && d < per_row; d <<= 1)
+    joined |= __shfl_xor_sync(0xffffffffu, joined, d);
+  if ((c0 & 31) == 0 && c0 < cols) row_words[r * ((cols + 31) >> 5) + (c0 >> 5)] = joined;
+  if (g.gates_out != nullptr) {
+    denom = fmaxf(denom, 1.1920928955078125e-07f);
 #pragma unroll
-      for (int i = 0; i < PER; i++) {
-        const int c = l + L * i;
-        if (c < cols)
-          __stcs(g.gates_out + row * x.path_num + c,
-                 ((picked >> i) & 1u) ? __fdiv_rn(key_score(key[i]), denom) : 0.f);
+    for (int q = 0; q < 8; q++) {
+      const int at = 4 * ((q + rot) & (vecs - 1));
+      if (q < vecs && c0 + at < cols) {
+        int4 out = make_int4(0, 0, 0, 0);
+        const unsigned four = (word >> at) & 15u;
+        if (four != 0u) {
+          const int4 v = *reinterpret_cast<const int4*>(row + at);
+          if (four & 1u) out.x = __float_as_int(__fdiv_rn(__int_as_float(v.x), denom));
+          if (four & 2u) out.y = __float_as_int(__fdiv_rn(__int_as_float(v.y), denom));
+          if (four & 4u) out.z = __float_as_int(__fdiv_rn(__int_as_float(v.z), denom));
+          if (four & 8u) out.w = __float_as_int(__fdiv_rn(__int_as_float(v.w), denom));
+        }
+        *reinterpret_cast<int4*>(row + at) = out;
       }
     }
   }
-  flush();
 }
 
-// Decide the routes of a staged tile of scores and leave the result as column bit words in
-// `bits` (zeroed beforehand) and per-path counts added to `sums`: what pack_staged produces
-// from a staged mask, without a mask in between.  The caller passes a CTA barrier next.
-__device__ __forceinline__ void gate_rows(const TileCtx& x, const int* stage, int* bits,
-                                          int* sums, const GateArgs& g) {
-  const int cols = x.path_num;  // <= 256, warp-uniform
-  if (cols <= 8) gate_rows_as<1, 8>(x, stage, bits, sums, g);
-  else if (cols <= 16) gate_rows_as<1, 16>(x, stage, bits, sums, g);
-  else if (cols <= 32) gate_rows_as<1, 32>(x, stage, bits, sums, g);
-  else if (cols <= 64) gate_rows_as<2, 32>(x, stage, bits, sums, g);
-  else if (cols <= 128) gate_rows_as<4, 32>(x, stage, bits, sums, g);
-  else gate_rows_as<8, 32>(x, stage, bits, sums, g);
+// The tile's picks as column bit words and counts: what pack_words produces from a staged mask.
+// Opens and ends with a CTA barrier.
+__device__ __forceinline__ void gate_words(const TileCtx& x, int* stage, int* bits, int* sums,
+                                           int* routed, unsigned* row_words, const GateArgs& g) {
+  gate_rows(x, stage, row_words, g);
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5;
+  const int col_blocks = (x.path_num + 31) >> 5;
+  if (warp < x.rg * col_blocks) {  // one 32x32 block per warp, never more than 8
+    const int group = warp / col_blocks;
+    const int cb = warp - group * col_blocks;
+    const int col = cb * 32 + lane;
+    const unsigned mine = row_words[(group * 32 + lane) * col_blocks + cb];
+    const int any = __reduce_add_sync(0xffffffffu, __popc(mine));
+    const uint32_t colw = warp_transpose32(mine, lane);
+    if (col < x.path_num) {
+      bits[group * x.ec + col] = static_cast<int>(colw);
+      const int n = __popc(colw);
+      if (n != 0) atomicAdd(&sums[col], n);
+    }
+    if (lane == 0 && any != 0) atomicAdd(routed, any);
+  }
+  if (g.gates_out != nullptr) {
+    const int vec_per_row = x.path_num >> 2;
+    const int64_t row0 = x.tile * x.rg * kGroupRows;
+    const int64_t left = x.cell_num - row0;
+    const int rows = left < x.rg * kGroupRows ? (int)left : x.rg * kGroupRows;
+    const int total = rows * vec_per_row;
+    int4* const out = reinterpret_cast<int4*>(g.gates_out + row0 * x.path_num);
+    const int step_r = kTileThreads / vec_per_row;
+    const int step_q = kTileThreads - step_r * vec_per_row;
+    int r = threadIdx.x / vec_per_row;
+    int q = threadIdx.x - r * vec_per_row;
+    for (int i = threadIdx.x; i < total; i += kTileThreads) {
+      __stcs(out + i, *reinterpret_cast<const int4*>(stage + r * x.pitch + 4 * q));
+      r += step_r;
+      q += step_q;
+      if (q >= vec_per_row) { q -= vec_per_row; r += 1; }
+    }
+  }
+  __syncthreads();
 }
 
 // ---------------------------------------------------------------------------- chained path
 // One launch, no grid-wide barrier.  A CTA takes a ticket; ticket k owns a run of
 // consecutive tiles of one path chunk.  It packs them all (the bit words stay in shared
 // memory), publishes the run's column sums, adds up the sums published by the tickets before
-// it and then writes its tiles.  A ticket only ever waits for SMALLER tickets, whose CTAs
-// have started by construction, so the kernel needs no co-residency guarantee.
+// it and then writes its indices.  A ticket only ever waits for SMALLER tickets, whose CTAs
+// have started by construction, so the kernel needs no co-residency guarantee.  A mask that
+// one CTA takes needs neither tickets nor published sums (nor the memset that prepares them).
+//
+// Almost all of the output of a sparse mask is zero and known before any sum is: a tile with at
+// most 1/kSparse of its elements routed is zeroed while the next one is loaded, so that the
+// reads and most of the writes share the memory system, and what is left after the wait is
+// one 4-byte store per route.  Denser tiles are written whole, 16 bytes at a time, after the
+// wait.  (All tiles written after the wait: 262144 x 128 in 78 us, reads and writes one after
+// the other; now 60 us: 51 for reads and zeros, 5.2 TB/s, the rest for the wait and the routes.
+// From scores, top-1: 112 us with a warp per row in the gate, now 71.)
+//
+// Any path count: V = 4 stages 16 bytes at a time and wants path_num % 4 == 0 and 16-byte
+// aligned arrays, V = 1 stages element by element.
+//
+// Beside the indices it can leave, per cell, a route record: the first kRecordRoutes routes
+// as (path, seat) in ascending path order, seat 0 where there are fewer, kRecordMore set in
+// the first path when the record does not hold them all (then the index row has to be read).
+// Dispatch and combine read 32 bytes per cell in place of its index row.
 struct ChainArgs {
   TiledArgs t;
   GateArgs gate;
-  unsigned long long* status;  // [ranges][path_num]: (1 << 32) | column sum once published
+  unsigned long long* status;  // [ranges][path_num]: column sum << 8 | 1 once published
+  unsigned long long* block;   // [ranges / kBlockRuns][path_num]: the sums of kBlockRuns runs
+                               // added up, how many of them in the low byte; null: none kept
   int* ticket;
   int* error;       // set to 1 when a wait ran out
   int* host_error;  // host-mapped word that receives BRT_ERR_TIMEOUT then (may be null)
@@ -1163,14 +1211,27 @@ struct ChainArgs {
   int first_ticket; // 0; a test passes 1 so that the first run is never published
   int tiles_per_cta;
   int ranges;
+  uint4* records;   // may be null; path_num <= 256 only
 };
 
-constexpr int kChainFly = 16;            // status words a thread keeps in flight
+constexpr int kChainFly = 8;    // words a thread keeps in flight
+constexpr int kBlockRuns = 16;  // a run then adds up at most ranges / 16 + 15 words per column
 constexpr int kChainSpinLimit = 1 << 20;  // default number of polls
+constexpr int kSparse = 8;  // 4-byte stores into zeroed sectors beat whole vectors below this
 
+// A published word: the sum (any int32) above a byte that counts the runs in it.
+__device__ __forceinline__ unsigned long long status_word(int value) {
+  return (static_cast<unsigned long long>(static_cast<long long>(value)) << 8) | 1ull;
+}
+__device__ __forceinline__ int status_value(unsigned long long w) {
+  return static_cast<int>(static_cast<long long>(w) >> 8);
+}
 __device__ __forceinline__ void status_publish(unsigned long long* p, int value) {
-  const unsigned long long w = (1ull << 32) | static_cast<unsigned>(value);
-  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(w) : "memory");
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(status_word(value)) : "memory");
+}
+__device__ __forceinline__ void status_add(unsigned long long* p, int value) {
+  asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(status_word(value))
+               : "memory");
 }
 __device__ __forceinline__ unsigned long long status_peek(const unsigned long long* p) {
   unsigned long long w;
@@ -1178,18 +1239,301 @@ __device__ __forceinline__ unsigned long long status_peek(const unsigned long lo
   return w;
 }
 
-template <Mode MODE, bool GATED>
+// Shared memory of the chained kernel, in ints.  The base seats of every 32-cell group take
+// the place of the staged tiles once those are packed.
+struct ChainSmem {
+  int* sum;             // [ec] column sums of the run
+  int* extra;           // [ec] what values other than 0/1 add to them
+  int* flag;            // [8]  flag[0]: such a value was seen
+  int* before;          // [ec] column sums of the earlier runs
+  int* thr;             // [ec]
+  int* routed;          // [tiles rounded up to 4] elements routed per tile
+  unsigned* row_words;  // [kTileThreads] picks of a gated tile
+  int* bits;            // [tiles][rg][ec] column bit words
+  int* stages;          // 2 x [rg * 32][pitch]
+  int stage_ints;
+  int* base;            // [tiles][rg][ec], over the stages
+  __device__ __forceinline__ int* stage(int i) const { return stages + (i & 1) * stage_ints; }
+};
+__host__ __device__ inline int round4(int n) { return (n + 3) & ~3; }
+__host__ __device__ inline size_t chain_smem_ints(int ec, int rg, int pitch, int tiles) {
+  const size_t words = (size_t)tiles * rg * ec;
+  const size_t stages = 2 * (size_t)rg * kGroupRows * pitch;
+  return 4 * (size_t)ec + 8 + round4(tiles) + kTileThreads + words +
+         (stages > words ? stages : words);
+}
+__device__ __forceinline__ ChainSmem carve_chain_smem(int* s, int ec, int rg, int pitch,
+                                                      int tiles) {
+  ChainSmem m;
+  m.sum = s;
+  m.extra = s + ec;
+  m.flag = s + 2 * ec;
+  m.before = m.flag + 8;
+  m.thr = m.before + ec;
+  m.routed = m.thr + ec;
+  m.row_words = reinterpret_cast<unsigned*>(m.routed + round4(tiles));
+  m.bits = m.routed + round4(tiles) + kTileThreads;
+  m.stages = m.bits + tiles * rg * ec;
+  m.stage_ints = rg * kGroupRows * pitch;
+  m.base = m.stages;
+  return m;
+}
+
+// Visit (row, column) of a tile's elements `step` columns wide, thread by thread: the pair
+// advances by a fixed step with one carry, without a division per element.
+struct TileWalk {
+  int r, q, step_r, step_q, per_row;
+  __device__ __forceinline__ explicit TileWalk(int per_row_) : per_row(per_row_) {
+    step_r = kTileThreads / per_row;
+    step_q = kTileThreads - step_r * per_row;
+    r = threadIdx.x / per_row;
+    q = threadIdx.x - r * per_row;
+  }
+  __device__ __forceinline__ void next() {
+    r += step_r;
+    q += step_q;
+    if (q >= per_row) { q -= per_row; r += 1; }
+  }
+};
+__device__ __forceinline__ int rows_of(const TileCtx& x) {
+  const int64_t left = x.cell_num - x.tile * x.rg * kGroupRows;
+  const int rows = x.rg * kGroupRows;
+  return left < rows ? (int)left : rows;
+}
+
+// Start the asynchronous copy of one tile into `stage` (rows beyond the mask are zero-filled
+// with plain stores) and zero its bit words.  The caller commits the group, waits for it and
+// passes a CTA barrier before the tile is read.
+template <int V>
+__device__ __forceinline__ void stage_tile_async(const TileCtx& x, int cols, int* stage,
+                                                 int* bits, const int* __restrict__ mask) {
+  const int rows = rows_of(x);
+  const int* const src = mask + x.tile * x.rg * kGroupRows * x.path_num + (int64_t)x.chunk * x.ec;
+  for (int i = threadIdx.x; i < x.rg * x.ec; i += kTileThreads) bits[i] = 0;
+  TileWalk w(cols / V);
+  for (; w.r < x.rg * kGroupRows; w.next()) {
+    int* const dst = stage + w.r * x.pitch + V * w.q;
+    if constexpr (V == 4) {
+      if (w.r < rows) cp_async_16(dst, src + (int64_t)w.r * x.path_num + 4 * w.q);
+      else *reinterpret_cast<int4*>(dst) = make_int4(0, 0, 0, 0);
+    } else {
+      if (w.r < rows) cp_async_4(dst, src + (int64_t)w.r * x.path_num + w.q);
+      else *dst = 0;
+    }
+  }
+}
+
+// Turn a staged tile into column bit words at `bits` (zeroed), adding its column sums to
+// sm.sum / sm.extra and its routed elements to *routed; a value other than 0/1 sets sm.flag.
+// Ends with a CTA barrier.
+template <int V>
+__device__ __forceinline__ void pack_words(const TileCtx& x, int cols, const ChainSmem& sm,
+                                           const int* stage, int* bits, int* routed) {
+  const int lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5;
+  const int col_blocks = (cols + 31) >> 5;
+  for (int b = warp; b < x.rg * col_blocks; b += kTileWarps) {
+    const int g = b / col_blocks;
+    const int c_begin = (b - g * col_blocks) * 32;
+    if ((x.tile * x.rg + g) * kGroupRows >= x.cell_num) continue;  // warp-uniform
+    const int c_count = (cols - c_begin) < 32 ? (cols - c_begin) : 32;
+    const int* rowp = stage + (g * kGroupRows + lane) * x.pitch + c_begin;
+    uint32_t roww = 0;
+    int seen = 0;
+    if constexpr (V == 4) {
+#pragma unroll
+      for (int q = 0; q < 8; q++) {
+        if (4 * q < c_count) {
+          const int4 v = *reinterpret_cast<const int4*>(rowp + 4 * q);
+          roww += ((uint32_t)v.x << (4 * q)) + ((uint32_t)v.y << (4 * q + 1)) +
+                  ((uint32_t)v.z << (4 * q + 2)) + ((uint32_t)v.w << (4 * q + 3));
+          seen |= v.x | v.y | v.z | v.w;
+        }
+      }
+    } else {
+#pragma unroll 8
+      for (int c = 0; c < c_count; c++) {
+        const int v = rowp[c];
+        roww += (uint32_t)v << c;
+        seen |= v;
+      }
+    }
+    if (__any_sync(0xffffffffu, (seen & ~1) != 0)) {  // values other than 0/1: once more
+      roww = 0;
+      for (int c = 0; c < c_count; c++) {
+        const int v = rowp[c];
+        roww |= (v != 0 ? 1u : 0u) << c;
+        if ((v & ~1) != 0) atomicAdd(&sm.extra[c_begin + c], v - 1);
+      }
+      if (lane == 0) atomicOr(sm.flag, 1);
+    }
+    const int any = __reduce_add_sync(0xffffffffu, __popc(roww));
+    const uint32_t colw = warp_transpose32(roww, lane);
+    if (lane < c_count) {
+      bits[g * x.ec + c_begin + lane] = static_cast<int>(colw);
+      const int n = __popc(colw);
+      if (n != 0) atomicAdd(&sm.sum[c_begin + lane], n);
+    }
+    if (lane == 0 && any != 0) atomicAdd(routed, any);
+  }
+  __syncthreads();
+}
+
+// Zeros over the rows of a tile that exist.
+template <int V>
+__device__ __forceinline__ void zero_tile(const TileCtx& x, int cols, int* __restrict__ out) {
+  const int rows = rows_of(x);
+  int* const dst = out + x.tile * x.rg * kGroupRows * x.path_num + (int64_t)x.chunk * x.ec;
+  if (x.chunks == 1) {  // the rows are contiguous
+    const int n = rows * cols;
+    if constexpr (V == 4) {
+      for (int i = threadIdx.x; i < n >> 2; i += kTileThreads)
+        __stcs(reinterpret_cast<int4*>(dst) + i, make_int4(0, 0, 0, 0));
+    } else {
+      for (int i = threadIdx.x; i < n; i += kTileThreads) __stcs(dst + i, 0);
+    }
+    return;
+  }
+  TileWalk w(cols / V);
+  for (; w.r < rows; w.next()) {
+    int* const p = dst + (int64_t)w.r * x.path_num + V * w.q;
+    if constexpr (V == 4) __stcs(reinterpret_cast<int4*>(p), make_int4(0, 0, 0, 0));
+    else __stcs(p, 0);
+  }
+}
+
+// What a routed element with the given seat becomes (0: throttled away).
+template <Mode MODE>
+__device__ __forceinline__ int value_of(int seat, int thr) {
+  if constexpr (MODE == Mode::kThrottle) return seat <= thr ? 1 : 0;
+  if constexpr (MODE == Mode::kThrottleSeat) return seat <= thr ? seat : 0;
+  if constexpr (MODE == Mode::kMask) return 1;
+  return seat;
+}
+
+// A whole tile from its bit words and base seats.
+template <Mode MODE, int V>
+__device__ __forceinline__ void write_tile(const TileCtx& x, int cols, const int* bits,
+                                           const int* base, const int* thr,
+                                           int* __restrict__ out, int* __restrict__ mask_out) {
+  const int rows = rows_of(x);
+  const int64_t at0 = x.tile * x.rg * kGroupRows * x.path_num + (int64_t)x.chunk * x.ec;
+  TileWalk w(cols / V);
+  for (; w.r < rows; w.next()) {
+    const int rr = w.r & 31;
+    const uint32_t low = 0xffffffffu >> (31 - rr);  // bits 0..rr
+    const int c = V * w.q;
+    const int* wp = bits + (w.r >> 5) * x.ec + c;
+    const int* bp = base + (w.r >> 5) * x.ec + c;
+    int words[V], seats[V], v[V];
+    if constexpr (V == 4) {
+      const int4 w4 = *reinterpret_cast<const int4*>(wp);
+      const int4 b4 = *reinterpret_cast<const int4*>(bp);
+      words[0] = w4.x; words[1] = w4.y; words[2] = w4.z; words[3] = w4.w;
+      seats[0] = b4.x; seats[1] = b4.y; seats[2] = b4.z; seats[3] = b4.w;
+    } else {
+      words[0] = *wp;
+      seats[0] = *bp;
+    }
+#pragma unroll
+    for (int j = 0; j < V; j++) {
+      const uint32_t word = static_cast<uint32_t>(words[j]);
+      const int seat = seats[j] + __popc(word & low);
+      constexpr bool kLimited = MODE == Mode::kThrottle || MODE == Mode::kThrottleSeat;
+      v[j] = ((word >> rr) & 1u) ? value_of<MODE>(seat, kLimited ? thr[c + j] : 0) : 0;
+    }
+    const int64_t at = at0 + (int64_t)w.r * x.path_num + c;
+    if constexpr (V == 4) {
+      __stcs(reinterpret_cast<int4*>(out + at), make_int4(v[0], v[1], v[2], v[3]));
+      if (mask_out != nullptr)
+        __stcs(reinterpret_cast<int4*>(mask_out + at),
+               make_int4(v[0] != 0, v[1] != 0, v[2] != 0, v[3] != 0));
+    } else {
+      __stcs(out + at, v[0]);
+      if (mask_out != nullptr) __stcs(mask_out + at, v[0] != 0 ? 1 : 0);
+    }
+  }
+}
+
+// The routes of the 32 cells of a group, one cell per lane: their elements into a zeroed output
+// (`scatter`) and the cells' records.  Called by a whole warp.
+template <Mode MODE>
+__device__ __forceinline__ void write_routes(const ChainArgs& c, const TileCtx& x, int cols,
+                                             int64_t group, const int* bits, const int* base,
+                                             const int* thr, bool scatter) {
+  const int lane = threadIdx.x & 31;
+  const int64_t row = group * kGroupRows + lane;
+  const uint32_t low = 0xffffffffu >> (31 - lane);
+  const int64_t at = row * x.path_num + (int64_t)x.chunk * x.ec;
+  const bool records = (MODE == Mode::kSeat || MODE == Mode::kThrottleSeat) && c.records != nullptr;
+  int n = 0;
+  int path[kRecordRoutes], seats[kRecordRoutes];
+#pragma unroll
+  for (int k = 0; k < kRecordRoutes; k++) { path[k] = 0; seats[k] = 0; }
+  // 128 paths at a time: four transposes in flight, and one turn of the loop takes a route of
+  // every lane wherever in the 128 it lies
+  for (int c0 = 0; c0 < cols; c0 += 128) {
+    uint32_t mine[4];  // this lane's cell, 32 paths each
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const int col = c0 + 32 * j + lane;
+      mine[j] = col < cols ? static_cast<uint32_t>(bits[col]) : 0u;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+      if (c0 + 32 * j < cols) mine[j] = warp_transpose32(mine[j], lane);
+    for (;;) {
+      uint32_t word = mine[0];
+      int block = 0;
+#pragma unroll
+      for (int j = 1; j < 4; j++)
+        if (word == 0u) { word = mine[j]; block = j; }
+      if (word == 0u) break;
+      const int col = c0 + 32 * block + __ffs(word) - 1;
+      word &= word - 1;
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+        if (block == j) mine[j] = word;
+      constexpr bool kLimited = MODE == Mode::kThrottle || MODE == Mode::kThrottleSeat;
+      const int seat = base[col] + __popc(static_cast<uint32_t>(bits[col]) & low);
+      const int v = value_of<MODE>(seat, kLimited ? thr[col] : 0);
+      if (v == 0) continue;
+      if constexpr (MODE == Mode::kTag) {
+        if (seat <= x.cell_num)
+          c.t.out[(int64_t)(seat - 1) * x.path_num + (int64_t)x.chunk * x.ec + col] =
+              (int)(row + 1);
+      } else if (scatter) {
+        c.t.out[at + col] = v;
+        if (c.t.mask_out != nullptr) c.t.mask_out[at + col] = 1;
+      }
+      if (records) {
+#pragma unroll
+        for (int k = 0; k < kRecordRoutes; k++)
+          if (n == k) { path[k] = col; seats[k] = v; }
+        n++;
+      }
+    }
+  }
+  if (records && row < x.cell_num) {
+    if (n > kRecordRoutes) path[0] |= kRecordMore;
+    c.records[2 * row] = make_uint4(path[0], seats[0], path[1], seats[1]);
+    c.records[2 * row + 1] = make_uint4(path[2], seats[2], path[3], seats[3]);
+  }
+}
+
+template <Mode MODE, bool GATED, int V>
 __global__ void __launch_bounds__(kTileThreads, 2) index_chain_kernel(const ChainArgs c) {
   extern __shared__ __align__(16) int s_dyn[];
   __shared__ int s_ticket;
   const TiledArgs& a = c.t;
   const int tid = threadIdx.x;
-  if (tid == 0) s_ticket = atomicAdd(c.ticket, 1);
-  TileSmem sm = carve_tile_smem(s_dyn, a.ec, a.rg, a.pitch, true);
-  int* bits_all = s_dyn + tile_smem_ints(a.ec, a.rg, a.pitch, true);
+  const bool alone = c.ranges == 1;
+  if (!alone && tid == 0) s_ticket = atomicAdd(c.ticket, 1);
+  const ChainSmem sm = carve_chain_smem(s_dyn, a.ec, a.rg, a.pitch, c.tiles_per_cta);
   for (int i = tid; i < 2 * a.ec + 1; i += kTileThreads) sm.sum[i] = 0;
+  for (int i = tid; i < c.tiles_per_cta; i += kTileThreads) sm.routed[i] = 0;
   __syncthreads();
-  const int ticket = s_ticket + c.first_ticket;
+  const int ticket = alone ? (int)blockIdx.x : s_ticket + c.first_ticket;
   const int range = ticket / a.chunks;
   if (range >= c.ranges) return;  // only with first_ticket != 0: nothing left to own
   TileCtx x;
@@ -1219,49 +1563,57 @@ __global__ void __launch_bounds__(kTileThreads, 2) index_chain_kernel(const Chai
     sm.thr[tid] = MODE == Mode::kThrottleSeat ? thr - start : thr;
   }
 
-  // two staging buffers: the copy of tile t + 1 is in flight while tile t is packed
-  int* const stage[2] = {sm.tile, bits_all + (size_t)c.tiles_per_cta * words_per_tile};
+  // two staging buffers: the copy of tile t + 1 is in flight while tile t is packed and zeroed
   x.tile = tile0;
-  stage_tile_async(x, stage[0], bits_all, a.mask);
+  stage_tile_async<V>(x, cols, sm.stage(0), sm.bits, a.mask);
   cp_async_commit();
   for (int64_t t = tile0; t < tile1; t++) {
     const int i = (int)(t - tile0);
     if (t + 1 < tile1) {
       x.tile = t + 1;
-      stage_tile_async(x, stage[(i + 1) & 1], bits_all + (size_t)(i + 1) * words_per_tile, a.mask);
+      stage_tile_async<V>(x, cols, sm.stage(i + 1), sm.bits + (i + 1) * words_per_tile,
+                          a.mask);
     }
     cp_async_commit();
     cp_async_wait<1>();
     __syncthreads();
     x.tile = t;
-    TileSmem cur = sm;
-    cur.tile = stage[i & 1];
-    cur.bits = bits_all + (size_t)i * words_per_tile;
-    if constexpr (GATED) {  // the staged tile holds scores: straight to bit words and counts
-      gate_rows(x, cur.tile, cur.bits, sm.sum, c.gate);
-      __syncthreads();
-    } else {
-      pack_staged(x, cur, nullptr);
+    int* const bits = sm.bits + i * words_per_tile;
+    if constexpr (GATED)  // the staged tile holds scores
+      gate_words(x, sm.stage(i), bits, sm.sum, sm.routed + i, sm.row_words, c.gate);
+    else
+      pack_words<V>(x, cols, sm, sm.stage(i), bits, sm.routed + i);
+    // (the tag output is zeroed as a whole before the launch: its rows are not the tile's)
+    if (MODE != Mode::kTag && sm.routed[i] * kSparse <= rows_of(x) * cols) {
+      zero_tile<V>(x, cols, a.out);
+      if (a.mask_out != nullptr) zero_tile<V>(x, cols, a.mask_out);
     }
   }
   const int own = tid < cols ? sm.sum[tid] + sm.extra[tid] : 0;
   const bool general = *sm.flag != 0;
-  __threadfence();
-  if (tid < cols) status_publish(c.status + (int64_t)range * a.path_num + col0 + tid, own);
+  for (int i = tid; i < a.ec; i += kTileThreads) sm.before[i] = 0;
 
-  // sum of the tickets before this one: thread (part, path) takes every parts-th of them,
-  // kChainFly loads in flight at a time
-  int* s_before = sm.base;  // free until the first expand
-  for (int i = tid; i < a.ec; i += kTileThreads) s_before[i] = 0;
-  __syncthreads();
-  {
+  if (!alone) {
+    __threadfence();
+    const int my_block = c.block != nullptr ? range / kBlockRuns : 0;
+    if (tid < cols) {
+      status_publish(c.status + (int64_t)range * a.path_num + col0 + tid, own);
+      if (c.block != nullptr && (my_block + 1) * kBlockRuns <= c.ranges)
+        status_add(c.block + (int64_t)my_block * a.path_num + col0 + tid, own);
+    }
+    __syncthreads();
+    // sum of the runs before this one: whole blocks of them, then those of this run's block.
+    // Thread (part, path) takes every parts-th word, kChainFly loads in flight at a time.
     const int parts = kTileThreads / cols;
     const int part = tid / cols;
     const int path = tid - part * cols;
-    if (part < parts && range > 0) {
-      const unsigned long long* column = c.status + col0 + path;
+    const int words = my_block + (range - my_block * kBlockRuns);
+    if (part < parts && words > 0) {
+      const unsigned long long* const blocks = c.block + col0 + path;
+      const unsigned long long* const runs =
+          c.status + (int64_t)my_block * (kBlockRuns - 1) * a.path_num + col0 + path;
       int acc = 0;
-      for (int j0 = part; j0 < range; j0 += parts * kChainFly) {
+      for (int j0 = part; j0 < words; j0 += parts * kChainFly) {
         unsigned long long w[kChainFly];
         int spins = 0;
         for (;;) {
@@ -1269,10 +1621,15 @@ __global__ void __launch_bounds__(kTileThreads, 2) index_chain_kernel(const Chai
 #pragma unroll
           for (int u = 0; u < kChainFly; u++) {
             const int j = j0 + u * parts;
-            w[u] = j < range ? status_peek(column + (int64_t)j * a.path_num) : (1ull << 32);
+            // word j is block j, or run my_block * kBlockRuns + (j - my_block)
+            w[u] = j < words ? status_peek((j < my_block ? blocks : runs) + (int64_t)j * a.path_num)
+                             : (unsigned long long)kBlockRuns;
           }
 #pragma unroll
-          for (int u = 0; u < kChainFly; u++) ready = ready && (w[u] >> 32) != 0;
+          for (int u = 0; u < kChainFly; u++) {
+            const int need = j0 + u * parts < my_block ? kBlockRuns : 1;
+            ready = ready && (int)(w[u] & 0xffu) >= need;
+          }
           if (ready) break;
           if (++spins > c.spin_limit) {  // give up: report it and carry on with what is there
             *c.error = 1;
@@ -1285,16 +1642,16 @@ __global__ void __launch_bounds__(kTileThreads, 2) index_chain_kernel(const Chai
           __nanosleep(64);
         }
 #pragma unroll
-        for (int u = 0; u < kChainFly; u++) acc += static_cast<int>(static_cast<unsigned>(w[u]));
+        for (int u = 0; u < kChainFly; u++) acc += status_value(w[u]);
       }
-      if (acc != 0) atomicAdd(&s_before[path], acc);
+      if (acc != 0) atomicAdd(&sm.before[path], acc);
     }
   }
   __syncthreads();
-  int run = tid < cols ? s_before[tid] + (MODE == Mode::kThrottle ? start : 0) : 0;
+  int run = tid < cols ? sm.before[tid] + (MODE == Mode::kThrottle ? start : 0) : 0;
 
   if (range == c.ranges - 1 && tid < cols) {
-    const int total = s_before[tid] + own;
+    const int total = sm.before[tid] + own;
     __threadfence();
     if constexpr (kThrottles) {
       const int thr = MODE == Mode::kThrottleSeat ? sm.thr[tid] + start : sm.thr[tid];
@@ -1322,14 +1679,51 @@ __global__ void __launch_bounds__(kTileThreads, 2) index_chain_kernel(const Chai
     }
   }
 
-  for (int64_t t = tile0; t < tile1; t++) {
-    x.tile = t;
-    if (general) {
+  if (general) {
+    for (int64_t t = tile0; t < tile1; t++) {
+      x.tile = t;
       expand_general<MODE>(x, a.mask, run, a.out, a.threshold);
-    } else {
-      TileSmem cur = sm;
-      cur.bits = bits_all + (t - tile0) * words_per_tile;
-      expand_binary<MODE>(x, cur, run, a.out, a.mask_out);
+      if (c.records != nullptr)  // seats of such a mask are not counts: read the index rows
+        for (int r = tid; r < rows_of(x); r += kTileThreads) {
+          const int64_t row = t * a.rg * kGroupRows + r;
+          c.records[2 * row] = make_uint4((unsigned)kRecordMore, 0u, 0u, 0u);
+          c.records[2 * row + 1] = make_uint4(0u, 0u, 0u, 0u);
+        }
+    }
+    return;
+  }
+  const int tiles = (int)(tile1 - tile0);
+  const int groups = tiles * a.rg;
+  if (tid < cols) {  // base seats of every group of the run, one path per thread
+    for (int g0 = 0; g0 < groups; g0 += 8) {
+      int n[8];
+#pragma unroll
+      for (int u = 0; u < 8; u++)
+        n[u] = g0 + u < groups ? __popc(static_cast<uint32_t>(sm.bits[(g0 + u) * a.ec + tid])) : 0;
+#pragma unroll
+      for (int u = 0; u < 8; u++) {
+        if (g0 + u < groups) sm.base[(g0 + u) * a.ec + tid] = run;
+        run += n[u];
+      }
+    }
+  }
+  __syncthreads();
+  const bool with_records = c.records != nullptr;
+  for (int g = tid >> 5; g < groups; g += kTileWarps) {
+    const int i = g / a.rg;
+    x.tile = tile0 + i;
+    const bool scatter =
+        MODE == Mode::kTag || sm.routed[i] * kSparse <= rows_of(x) * cols;  // warp-uniform
+    if (scatter || with_records)
+      write_routes<MODE>(c, x, cols, tile0 * a.rg + g, sm.bits + g * a.ec, sm.base + g * a.ec,
+                         sm.thr, scatter);
+  }
+  if constexpr (MODE != Mode::kTag) {
+    for (int i = 0; i < tiles; i++) {
+      x.tile = tile0 + i;
+      if (sm.routed[i] * kSparse > rows_of(x) * cols)
+        write_tile<MODE, V>(x, cols, sm.bits + i * words_per_tile, sm.base + i * words_per_tile,
+                            sm.thr, a.out, a.mask_out);
     }
   }
 }
@@ -1383,14 +1777,14 @@ std::atomic<int> g_spin_limit{kChainSpinLimit};
 std::atomic<int> g_first_ticket{0};
 thread_local bool t_may_allocate = true;  // false inside the entry point that must not
 
-template <Mode MODE, bool GATED>
+template <Mode MODE, bool GATED, int V>
 int launch_chain_mode(const ChainArgs& c, unsigned grid, size_t smem, cudaStream_t stream) {
   static thread_local std::map<int, size_t> configured;  // device -> opted-in bytes
   if (smem > 48 * 1024) {
     int dev = 0;
     BRT_CUDA_TRY(cudaGetDevice(&dev));
     if (configured[dev] < smem) {
-      BRT_CUDA_TRY(cudaFuncSetAttribute(index_chain_kernel<MODE, GATED>,
+      BRT_CUDA_TRY(cudaFuncSetAttribute(index_chain_kernel<MODE, GATED, V>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)kChainSmemLimit));
       configured[dev] = kChainSmemLimit;
@@ -1401,17 +1795,60 @@ int launch_chain_mode(const ChainArgs& c, unsigned grid, size_t smem, cudaStream
                                 : MODE == Mode::kThrottleSeat ? "throttle_index_chain_kernel"
                                                               : "index_chain_kernel",
                           stream);
-  index_chain_kernel<MODE, GATED><<<grid, kTileThreads, smem, stream>>>(c), note_launch();
+  index_chain_kernel<MODE, GATED, V><<<grid, kTileThreads, smem, stream>>>(c), note_launch();
   BRT_LAUNCH_CHECK("index_chain_kernel");
   return BRT_OK;
 }
 
-int launch_chain(Mode mode, const TileGeom& g, int tiles_per_cta, int ranges, size_t smem,
-                 const int32_t* mask, int32_t* out, int32_t* loads, int64_t cell_num,
-                 int path_num, const int32_t* caps, int ncap, int capacity_padding,
-                 int path_wise, int32_t* prefix, const int32_t* threshold, void* scratch,
-                 cudaStream_t stream, const GateArgs* gate = nullptr,
+// How the chained launch cuts a mask; smem == 0: it does not fit.
+struct ChainPlan {
+  TileGeom geom;
+  int tiles_per_cta, ranges;
+  size_t smem;
+};
+
+// Masks of at most this many full tiles are scanned by one CTA (per 256 paths): what it saves is
+// the memset in front of the launch, the ticket and the wait.  (256 x 32: 4.7 us of GPU time;
+// 2048 x 32 with 64 CTAs takes 6.0 plus 1.4 for the memset)
+constexpr int64_t kAloneTiles = 2;
+
+ChainPlan plan_chain(int64_t cell_num, int path_num, bool wide) {
+  ChainPlan plan;
+  TileGeom& g = plan.geom;
+  g = make_tile_geom(cell_num, path_num, max_row_groups(path_num < 256 ? path_num : 256));
+  const bool alone = g.num_tiles <= kAloneTiles;
+  if (!alone) g = make_tile_geom(cell_num, path_num);
+  if (!wide) {  // element by element: an odd pitch keeps a column walk free of bank conflicts
+    g.ec = round4(g.ec);
+    g.pitch = path_num | 1;
+  }
+  int64_t target = alone ? 1 : (int64_t)sm_count() * kChainCtasPerSm / g.col_chunks;
+  if (target < 1) target = 1;
+  const int64_t ranges0 = g.num_tiles < target ? g.num_tiles : target;
+  const int64_t tiles_per_cta = (g.num_tiles + ranges0 - 1) / ranges0;
+  plan.smem = 0;
+  if (tiles_per_cta > (int64_t)kChainSmemLimit) return plan;
+  plan.tiles_per_cta = (int)tiles_per_cta;
+  plan.ranges = (int)((g.num_tiles + tiles_per_cta - 1) / tiles_per_cta);
+  const size_t smem = chain_smem_ints(g.ec, g.rg, g.pitch, plan.tiles_per_cta) * sizeof(int);
+  if (smem <= kChainSmemLimit && (wide || g.col_chunks == 1)) plan.smem = smem;
+  return plan;
+}
+
+bool forced_split() {
+  static const bool forced = [] {
+    const char* const v = getenv("BRT_INDEX_PATH");
+    return v != nullptr && strcmp(v, "split") == 0;
+  }();
+  return forced;
+}
+
+int launch_chain(Mode mode, const ChainPlan& plan, bool wide, const int32_t* mask, int32_t* out,
+                 int32_t* loads, int64_t cell_num, int path_num, const int32_t* caps, int ncap,
+                 int capacity_padding, int path_wise, int32_t* prefix, const int32_t* threshold,
+                 void* scratch, cudaStream_t stream, const GateArgs* gate = nullptr,
                  int32_t* mask_out = nullptr) {
+  const TileGeom& g = plan.geom;
   ChainArgs c;
   c.gate = gate != nullptr ? *gate : GateArgs{0, 0, 0.f, -1, nullptr};
   char* p = static_cast<char*>(scratch);
@@ -1422,8 +1859,15 @@ int launch_chain(Mode mode, const TileGeom& g, int tiles_per_cta, int ranges, si
   c.spin_limit = g_spin_limit.load(std::memory_order_relaxed);
   c.first_ticket = g_first_ticket.load(std::memory_order_relaxed);
   c.status = reinterpret_cast<unsigned long long*>(p + 256);
-  c.tiles_per_cta = tiles_per_cta;
-  c.ranges = ranges;
+  // the sums of blocks of runs, where the scratch (whose size the caller was told) has room
+  const size_t run_bytes = (size_t)plan.ranges * path_num * 8;
+  const size_t block_bytes = (size_t)(plan.ranges / kBlockRuns) * path_num * 8;
+  const bool blocks = plan.ranges > 2 * kBlockRuns &&
+                      256 + run_bytes + block_bytes <= scratch_bytes_for(cell_num, path_num);
+  c.block = blocks ? c.status + (size_t)plan.ranges * path_num : nullptr;
+  c.tiles_per_cta = plan.tiles_per_cta;
+  c.ranges = plan.ranges;
+  c.records = static_cast<uint4*>(t_records_out);
   c.t.tile_flags = nullptr;
   c.t.tile_sums = nullptr;
   c.t.bits = nullptr;
@@ -1445,25 +1889,34 @@ int launch_chain(Mode mode, const TileGeom& g, int tiles_per_cta, int ranges, si
   c.t.pitch = g.pitch;
   c.t.num_tiles = g.num_tiles;
   c.t.chunks = g.col_chunks;
-  BRT_CUDA_TRY(cudaMemsetAsync(p, 0, 256 + (size_t)ranges * path_num * 8, stream));
+  if (plan.ranges > 1)
+    BRT_CUDA_TRY(cudaMemsetAsync(p, 0, 256 + run_bytes + (blocks ? block_bytes : 0), stream));
   if (mode == Mode::kTag)
     BRT_CUDA_TRY(cudaMemsetAsync(out, 0, (size_t)cell_num * path_num * 4, stream));
-  const unsigned grid = (unsigned)ranges * (unsigned)g.col_chunks;
+  const unsigned grid = (unsigned)plan.ranges * (unsigned)g.col_chunks;
+  const size_t smem = plan.smem;
   if (gate != nullptr) {
     switch (mode) {
-      case Mode::kSeat: return launch_chain_mode<Mode::kSeat, true>(c, grid, smem, stream);
-      case Mode::kMask: return launch_chain_mode<Mode::kMask, true>(c, grid, smem, stream);
+      case Mode::kSeat: return launch_chain_mode<Mode::kSeat, true, 4>(c, grid, smem, stream);
+      case Mode::kMask: return launch_chain_mode<Mode::kMask, true, 4>(c, grid, smem, stream);
       case Mode::kThrottleSeat:
-        return launch_chain_mode<Mode::kThrottleSeat, true>(c, grid, smem, stream);
-      default: return launch_chain_mode<Mode::kThrottle, true>(c, grid, smem, stream);
+        return launch_chain_mode<Mode::kThrottleSeat, true, 4>(c, grid, smem, stream);
+      default: return launch_chain_mode<Mode::kThrottle, true, 4>(c, grid, smem, stream);
+    }
+  }
+  if (!wide) {
+    switch (mode) {
+      case Mode::kSeat: return launch_chain_mode<Mode::kSeat, false, 1>(c, grid, smem, stream);
+      case Mode::kTag: return launch_chain_mode<Mode::kTag, false, 1>(c, grid, smem, stream);
+      default: return launch_chain_mode<Mode::kThrottle, false, 1>(c, grid, smem, stream);
     }
   }
   switch (mode) {
-    case Mode::kSeat: return launch_chain_mode<Mode::kSeat, false>(c, grid, smem, stream);
-    case Mode::kTag: return launch_chain_mode<Mode::kTag, false>(c, grid, smem, stream);
+    case Mode::kSeat: return launch_chain_mode<Mode::kSeat, false, 4>(c, grid, smem, stream);
+    case Mode::kTag: return launch_chain_mode<Mode::kTag, false, 4>(c, grid, smem, stream);
     case Mode::kThrottleSeat:
-      return launch_chain_mode<Mode::kThrottleSeat, false>(c, grid, smem, stream);
-    default: return launch_chain_mode<Mode::kThrottle, false>(c, grid, smem, stream);
+      return launch_chain_mode<Mode::kThrottleSeat, false, 4>(c, grid, smem, stream);
+    default: return launch_chain_mode<Mode::kThrottle, false, 4>(c, grid, smem, stream);
   }
 }
 
@@ -1472,30 +1925,14 @@ int launch_tiled(Mode mode, const int32_t* mask, int32_t* out, int32_t* loads, i
                  int path_wise, int32_t* prefix, const int32_t* threshold, void* scratch,
                  cudaStream_t stream, const GateArgs* gate = nullptr,
                  int32_t* mask_out = nullptr) {
-  TileGeom g = make_tile_geom(cell_num, path_num);
-  BRT_REQUIRE(g.num_tiles <= 0x7fffffffLL && g.col_chunks <= 65535,
-              "mask of %lld x %d cells is too large for one launch", (long long)cell_num,
-              path_num);
   // One chained launch when the bit words of a CTA's tiles fit in shared memory, else three
   // launches (pack, scan, expand).  BRT_INDEX_PATH=split forces the latter (for tests).
-  static const bool forced_split = [] {
-    const char* const forced = getenv("BRT_INDEX_PATH");
-    return forced != nullptr && strcmp(forced, "split") == 0;
-  }();
-  if (gate != nullptr || !forced_split || mode == Mode::kThrottleSeat) {
-    int64_t target = (int64_t)sm_count() * kChainCtasPerSm / g.col_chunks;
-    if (target < 1) target = 1;
-    const int64_t ranges0 = g.num_tiles < target ? g.num_tiles : target;
-    const int64_t tiles_per_cta = (g.num_tiles + ranges0 - 1) / ranges0;
-    const int64_t ranges = (g.num_tiles + tiles_per_cta - 1) / tiles_per_cta;
-    const size_t smem = (tile_smem_ints(g.ec, g.rg, g.pitch, true) +
-                         (size_t)tiles_per_cta * g.rg * g.ec +
-                         (size_t)g.rg * kGroupRows * g.pitch) *
-                        sizeof(int);
-    if (smem <= kChainSmemLimit)
-      return launch_chain(mode, g, (int)tiles_per_cta, (int)ranges, smem, mask, out, loads,
-                          cell_num, path_num, caps, ncap, capacity_padding, path_wise, prefix,
-                          threshold, scratch, stream, gate, mask_out);
+  if (gate != nullptr || !forced_split() || mode == Mode::kThrottleSeat) {
+    const ChainPlan plan = plan_chain(cell_num, path_num, true);
+    if (plan.smem != 0)
+      return launch_chain(mode, plan, true, mask, out, loads, cell_num, path_num, caps, ncap,
+                          capacity_padding, path_wise, prefix, threshold, scratch, stream, gate,
+                          mask_out);
   }
   if (gate != nullptr)
     return set_error(BRT_ERR_UNSUPPORTED,
@@ -1505,6 +1942,11 @@ int launch_tiled(Mode mode, const int32_t* mask, int32_t* out, int32_t* loads, i
     return set_error(BRT_ERR_UNSUPPORTED,
                      "a %lld x %d mask does not fit the single-launch scan; throttle and index "
                      "it in two steps", (long long)cell_num, path_num);
+  BRT_REQUIRE(t_records_out == nullptr, "this mask gets no route records");
+  const TileGeom g = make_tile_geom(cell_num, path_num);
+  BRT_REQUIRE(g.num_tiles <= 0x7fffffffLL && g.col_chunks <= 65535,
+              "mask of %lld x %d cells is too large for one launch", (long long)cell_num,
+              path_num);
   TiledArgs a;
   char* p = static_cast<char*>(scratch);
   a.flags = reinterpret_cast<int*>(p);
@@ -1621,6 +2063,16 @@ int run_scan(Mode mode, const int32_t* mask, int32_t* out, int32_t* loads, int64
   if (path_num % 4 == 0 && aligned_to(mask, 16) && aligned_to(out, 16))
     return launch_tiled(mode, mask, out, loads, cell_num, path_num, caps, ncap,
                         capacity_padding, path_wise, prefix, threshold, scratch, stream);
+  // any other path count or alignment: the same chained launch, element by element, up to 256
+  // paths (9001 x 30: memset and three strip launches took 16.8 us of GPU time, memset and this
+  // one 10.4)
+  if (!forced_split()) {
+    const ChainPlan plan = plan_chain(cell_num, path_num, false);
+    if (plan.smem != 0)
+      return launch_chain(mode, plan, false, mask, out, loads, cell_num, path_num, caps, ncap,
+                          capacity_padding, path_wise, prefix, threshold, scratch, stream);
+  }
+  BRT_REQUIRE(t_records_out == nullptr, "this mask gets no route records");
   const bool a16 = aligned_to(mask, 16) && aligned_to(out, 16) &&
                    (threshold == nullptr || aligned_to(threshold, 16));
   const bool a8 = aligned_to(mask, 8) && aligned_to(out, 8) &&

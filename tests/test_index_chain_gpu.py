@@ -1,0 +1,117 @@
+"""The single-launch index scan and gate at the edges of their tiles: cell counts around 32, a
+tile, a CTA's run and the one-CTA limit, path counts with and without 16-byte rows, masks that
+are written whole and masks that are zeroed and scattered into.  Whole values, compared bit for
+bit with the checker."""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+CELLS = [1, 31, 33, 256, 257, 513, 1025, 9001, 40961]
+PATHS = [1, 3, 5, 16, 30, 33, 36, 97, 129, 250, 256, 260]
+
+
+def mask_of(rng, cells, paths, kind):
+    if kind == "top1":
+        mask = np.zeros((cells, paths), dtype=np.int32)
+        mask[np.arange(cells), rng.integers(0, paths, cells)] = 1
+        return mask
+    if kind == "mixed":  # dense and sparse tiles in one mask
+        odds = np.repeat(rng.choice([0.01, 0.12, 0.13, 0.9], (cells + 63) // 64), 64)[:cells, None]
+        return (rng.random((cells, paths)) < odds).astype(np.int32)
+    if kind == "ones":
+        return np.ones((cells, paths), dtype=np.int32)
+    # integer semantics; not below zero: the reference leaves a path at the first 1024 cells
+    # whose sum passes its threshold, which a falling sum would tell from a cell by cell rule
+    return rng.integers(0, 4, (cells, paths)).astype(np.int32)
+
+
+@pytest.mark.parametrize("kind", ["top1", "mixed", "ones", "integers"])
+@pytest.mark.parametrize("paths", PATHS)
+@pytest.mark.parametrize("cells", CELLS)
+def test_scan_edges(cells, paths, kind):
+    from brainstorm_b200._C import router as R
+
+    rng = np.random.default_rng(cells * 1000 + paths)
+    mask = mask_of(rng, cells, paths, kind)
+    dev = torch.from_numpy(mask).cuda()
+    caps = [max(1, cells // 3)]
+    caps_dev = torch.tensor(caps, dtype=torch.int32, device="cuda")
+    for tag in (False, True):
+        if kind == "integers" and tag:
+            continue  # several cells may name one tag row; which of them stays is not defined
+        got = R.generate_indices_and_loads(dev, caps_dev, False, False, tag)
+        want = oracle.generate_indices_and_loads(mask, caps, False, False, tag)
+        assert np.array_equal(got[0].cpu().numpy(), want[0]), tag
+        assert np.array_equal(got[1].cpu().numpy(), want[1]), tag
+    limit = rng.integers(0, cells + 2, paths).astype(np.int32)
+    start = rng.integers(0, 3, paths).astype(np.int32)
+    prefix = torch.from_numpy(start.copy()).cuda()
+    got, _ = R.throttle_hotmask(dev, prefix, torch.from_numpy(limit).cuda())
+    start_np = start.copy()
+    want, _ = oracle.throttle_hotmask(mask, start_np, limit)
+    assert np.array_equal(got.cpu().numpy(), want)
+    assert np.array_equal(prefix.cpu().numpy(), start_np)
+    if kind != "integers":
+        prefix = torch.from_numpy(start.copy()).cuda()
+        idx, loads, _, throttled = R.throttle_and_generate_indices(
+            dev, prefix, torch.from_numpy(limit).cuda(), caps_dev, with_mask=True)
+        want_idx, want_loads = oracle.generate_indices_and_loads(want, caps)
+        assert np.array_equal(throttled.cpu().numpy(), want)
+        assert np.array_equal(idx.cpu().numpy(), want_idx)
+        assert np.array_equal(loads.cpu().numpy(), want_loads)
+        assert np.array_equal(prefix.cpu().numpy(), start_np)
+
+
+def test_scan_of_an_array_that_is_only_4_byte_aligned():
+    from brainstorm_b200._C import router as R
+
+    rng = np.random.default_rng(3)
+    mask = mask_of(rng, 3000, 32, "mixed")
+    room = torch.zeros(3000 * 32 + 1, dtype=torch.int32, device="cuda")
+    view = room[1:].view(3000, 32)
+    view.copy_(torch.from_numpy(mask))
+    idx, loads = R.generate_indices_and_loads(view)
+    want = oracle.generate_indices_and_loads(mask)
+    assert np.array_equal(idx.cpu().numpy(), want[0])
+    assert np.array_equal(loads.cpu().numpy(), want[1])
+
+
+def picks_by_key(score, k):
+    """The k first of every row in descending order of the bits (NaN above everything), lower
+    paths first among equals."""
+    bits = score.view(np.uint32).astype(np.int64)
+    key = np.where(bits & 0x80000000, 0xffffffff - bits, bits + 0x80000000)
+    order = np.argsort(-key, axis=1, kind="stable")[:, :k]
+    mask = np.zeros(score.shape, dtype=np.int32)
+    np.put_along_axis(mask, order, 1, axis=1)
+    return mask
+
+
+@pytest.mark.parametrize("paths", [4, 8, 12, 20, 32, 36, 64, 68, 100, 128, 132, 200, 256])
+@pytest.mark.parametrize("cells", [1, 33, 300, 5003, 40000])
+def test_gate_edges(cells, paths):
+    from brainstorm_b200._C import router as R
+
+    rng = np.random.default_rng(cells + paths)
+    score = rng.choice(np.array([0.0, -0.0, 0.25, 1.0, -3.0, np.inf, -np.inf,
+                                 np.finfo(np.float32).min, 1e-40], dtype=np.float32),
+                       (cells, paths))
+    score[::2] = rng.standard_normal((score[::2].shape)).astype(np.float32)
+    score[rng.random(score.shape) < 0.01] = np.nan
+    dev = torch.from_numpy(score).cuda()
+    for k in sorted({1, 2, min(5, paths), paths}):
+        want = picks_by_key(score, k)
+        idx, loads, mask = R.route_scores(dev, "topk", k, output="seat_indices", with_mask=True)
+        assert np.array_equal(mask.cpu().numpy(), want), k
+        want_idx, want_loads = oracle.generate_indices_and_loads(want)
+        assert np.array_equal(idx.cpu().numpy(), want_idx), k
+        assert np.array_equal(loads.cpu().numpy(), want_loads), k
+    for residual in (-1, 0, paths - 1):
+        with np.errstate(invalid="ignore"):
+            want = oracle.threshold_hot_mask(score, 0.5, residual)
+        got = R.route_scores(dev, "threshold", threshold=0.5, residual_path=residual)[0]
+        assert np.array_equal(got.cpu().numpy(), want), residual
