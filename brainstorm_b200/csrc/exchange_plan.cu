@@ -273,7 +273,10 @@ int forward_begin(brt_p2p_ctx* c, const void* rows, const FusedDispatch* fused,
   if (n > 1024 || (size_t)c->world * n > kBoardInts)
     return set_error(BRT_ERR_UNSUPPORTED, "%d buckets are too many for the peer exchange", n);
   if (stages == 0) stages = BRT_P2P_STAGE_ALL;
-  if (int rc = check_alive(c)) return rc;
+  // the landing kernel of this very exchange may report rows that do not fit before its last
+  // stage is issued: an exchange under way is carried through, the next one is refused
+  if ((stages & BRT_P2P_STAGE_POST) || c->host_status[0] != BRT_ERR_UNSUPPORTED)
+    if (int rc = check_alive(c)) return rc;
   BRT_REQUIRE(!c->replaying || !(stages & BRT_P2P_STAGE_SIZES),
               "exchanges issued for replay keep their sizes on the device "
               "(brt_p2p_forward_device_sizes); the SIZES stage brings them to the host");
