@@ -1835,6 +1835,8 @@ ChainPlan plan_chain(int64_t cell_num, int path_num, bool wide) {
   return plan;
 }
 
+constexpr int64_t kRecordMinElements = 1 << 21;
+
 bool forced_split() {
   static const bool forced = [] {
     const char* const v = getenv("BRT_INDEX_PATH");
@@ -2134,8 +2136,35 @@ BRT_API size_t brt_index_scratch_bytes(int64_t cell_num, int path_num) {
   return scratch_bytes_for(cell_num, path_num);
 }
 
+BRT_API size_t brt_route_record_bytes(int64_t cell_num, int path_num) {
+  // Up to 16 paths an index row is no longer than two records.  Below 8 MB of indices the rows
+  // come out of L2 and the records save little for what their allocation costs the host (4 us):
+  // 64 x 32, a step of 57 us took 64 with them; 32768 x 32, 84 us took 83, but the gate alone
+  // 27 -> 32.
+  if (cell_num * path_num < kRecordMinElements) return 0;
+  if (cell_num <= 0 || path_num <= 16 || path_num > 256 || forced_split()) return 0;
+  if (plan_chain(cell_num, path_num, false).smem == 0) return 0;
+  if (path_num % 4 == 0 && plan_chain(cell_num, path_num, true).smem == 0) return 0;
+  return (size_t)cell_num * kRecordRoutes * 8;
+}
+
 BRT_API int brt_generate_indices_and_loads(const int32_t* hot_mask, int32_t* indices,
                                            int32_t* loads, int32_t* path_counts,
+                                           int64_t cell_num, int path_num,
+                                           const int32_t* supported_capacities,
+                                           int supported_capacity_num, int capacity_padding,
+                                           int path_wise_padding, int is_tag_index,
+                                           void* scratch, size_t scratch_bytes, void* stream) {
+  return brt_generate_indices_loads_records(hot_mask, indices, loads, path_counts, nullptr,
+                                            cell_num, path_num, supported_capacities,
+                                            supported_capacity_num, capacity_padding,
+                                            path_wise_padding, is_tag_index, scratch,
+                                            scratch_bytes, stream);
+}
+
+BRT_API int brt_generate_indices_loads_records(const int32_t* hot_mask, int32_t* indices,
+                                           int32_t* loads, int32_t* path_counts,
+                                           void* route_records,
                                            int64_t cell_num, int path_num,
                                            const int32_t* supported_capacities,
                                            int supported_capacity_num, int capacity_padding,
@@ -2165,7 +2194,9 @@ BRT_API int brt_generate_indices_and_loads(const int32_t* hot_mask, int32_t* ind
     return BRT_OK;
   }
   BRT_REQUIRE(hot_mask != nullptr && indices != nullptr, "hot_mask or indices is null");
-  const CountsScope counts(path_counts);
+  BRT_REQUIRE(route_records == nullptr || (!is_tag_index && aligned_to(route_records, 16)),
+              "route_records go with seat indices and must be 16-byte aligned");
+  const CountsScope counts(path_counts, route_records);
   return run_scan(is_tag_index ? Mode::kTag : Mode::kSeat, hot_mask, indices, loads, cell_num,
                   path_num, supported_capacities, supported_capacity_num, capacity_padding,
                   path_wise, nullptr, nullptr, scratch, scratch_bytes, st);
@@ -2188,6 +2219,18 @@ BRT_API int brt_throttle_hotmask(const int32_t* hotmask, int32_t* throttled, int
 BRT_API int brt_throttle_and_generate_indices(
     const int32_t* hot_mask, int32_t* indices, int32_t* loads, int32_t* path_counts,
     int32_t* prefix, const int32_t* threshold, int32_t* throttled_mask, int64_t cell_num,
+    int path_num, const int32_t* supported_capacities, int supported_capacity_num,
+    int capacity_padding, int path_wise_padding, void* scratch, size_t scratch_bytes,
+    void* stream) {
+  return brt_throttle_and_generate_records(
+      hot_mask, indices, loads, path_counts, nullptr, prefix, threshold, throttled_mask, cell_num,
+      path_num, supported_capacities, supported_capacity_num, capacity_padding,
+      path_wise_padding, scratch, scratch_bytes, stream);
+}
+
+BRT_API int brt_throttle_and_generate_records(
+    const int32_t* hot_mask, int32_t* indices, int32_t* loads, int32_t* path_counts,
+    void* route_records, int32_t* prefix, const int32_t* threshold, int32_t* throttled_mask, int64_t cell_num,
     int path_num,
     const int32_t* supported_capacities, int supported_capacity_num, int capacity_padding,
     int path_wise_padding, void* scratch, size_t scratch_bytes, void* stream) {
@@ -2225,7 +2268,8 @@ BRT_API int brt_throttle_and_generate_indices(
   if (scratch_bytes < need)
     return set_error(BRT_ERR_SCRATCH_TOO_SMALL, "scratch holds %zu bytes, %zu needed",
                      scratch_bytes, need);
-  const CountsScope counts(path_counts);
+  BRT_REQUIRE(aligned_to(route_records, 16), "route_records must be 16-byte aligned");
+  const CountsScope counts(path_counts, route_records);
   return launch_tiled(Mode::kThrottleSeat, hot_mask, indices, loads, cell_num, path_num,
                       supported_capacities, supported_capacity_num, capacity_padding, path_wise,
                       prefix, threshold, scratch, st, nullptr, throttled_mask);
@@ -2234,6 +2278,21 @@ BRT_API int brt_throttle_and_generate_indices(
 BRT_API int brt_route_scores(const float* scores, int64_t cell_num, int path_num, int decision,
                              int top_k, float threshold, int residual_path, int output,
                              int32_t* out, int32_t* loads, int32_t* path_counts,
+                             const int32_t* capacities, int capacity_num, int capacity_padding,
+                             int path_wise_padding, int32_t* prefix,
+                             const int32_t* throttle_capacity, float* gates_out,
+                             int32_t* mask_out, void* scratch, size_t scratch_bytes,
+                             void* stream) {
+  return brt_route_scores_records(scores, cell_num, path_num, decision, top_k, threshold,
+                                  residual_path, output, out, loads, path_counts, nullptr,
+                                  capacities, capacity_num, capacity_padding, path_wise_padding,
+                                  prefix, throttle_capacity, gates_out, mask_out, scratch,
+                                  scratch_bytes, stream);
+}
+
+BRT_API int brt_route_scores_records(const float* scores, int64_t cell_num, int path_num, int decision,
+                             int top_k, float threshold, int residual_path, int output,
+                             int32_t* out, int32_t* loads, int32_t* path_counts, void* route_records,
                              const int32_t* capacities,
                              int capacity_num, int capacity_padding, int path_wise_padding,
                              int32_t* prefix, const int32_t* throttle_capacity, float* gates_out,
@@ -2268,6 +2327,10 @@ BRT_API int brt_route_scores(const float* scores, int64_t cell_num, int path_num
   BRT_REQUIRE(path_counts == nullptr || output == BRT_ROUTE_SEAT_INDICES ||
                   output == BRT_ROUTE_THROTTLED_SEAT_INDICES,
               "path_counts goes with the seat-index outputs only");
+  BRT_REQUIRE(route_records == nullptr ||
+                  ((output == BRT_ROUTE_SEAT_INDICES ||
+                    output == BRT_ROUTE_THROTTLED_SEAT_INDICES) && aligned_to(route_records, 16)),
+              "route_records go with the seat-index outputs and must be 16-byte aligned");
   if (cell_num == 0) {
     if (output != BRT_ROUTE_THROTTLED_MASK)
       BRT_CUDA_TRY(cudaMemsetAsync(loads, 0, (size_t)path_num * 4, static_cast<cudaStream_t>(stream)));
@@ -2296,7 +2359,7 @@ BRT_API int brt_route_scores(const float* scores, int64_t cell_num, int path_num
                     : output == BRT_ROUTE_THROTTLED_MASK ? Mode::kThrottle
                     : output == BRT_ROUTE_THROTTLED_SEAT_INDICES ? Mode::kThrottleSeat
                                                                  : Mode::kSeat;
-  const CountsScope counts(path_counts);
+  const CountsScope counts(path_counts, route_records);
   return launch_tiled(mode, reinterpret_cast<const int32_t*>(scores), out, loads, cell_num,
                       path_num, capacities, capacity_num, capacity_padding, path_wise_padding,
                       prefix, throttle_capacity, scratch, static_cast<cudaStream_t>(stream), &gate,
