@@ -11,6 +11,7 @@ deliberate:
   identical when the current stream is the default one);
 * outputs are never pre-zeroed by a separate memset: the kernels write every byte.
 """
+import ctypes
 import os
 from typing import List, Optional
 
@@ -398,6 +399,13 @@ def dispatch_with_indices_and_loads(
     is_tag_index: bool = False,
 ) -> List[torch.Tensor]:
     """src/backend/torch/router.cc:131-273."""
+    return _dispatch(in_data, route_indices, loads, gates, tag_generating, tags,
+                     max_path_padding, max_path_load, is_1d_routing, is_tag_index)
+
+
+def _dispatch(in_data, route_indices, loads, gates, tag_generating, tags, max_path_padding,
+              max_path_load, is_1d_routing, is_tag_index=False, host_loads=None):
+    """The dispatch operator; ``host_loads``: the loads as the caller has already read them."""
     _check_cuda(in_data, "in_data")
     _check_cuda(route_indices, "route_indices")
     dev = in_data.device
@@ -433,7 +441,8 @@ def dispatch_with_indices_and_loads(
             total = mpl * path_num
         else:
             mpl = 0
-            total = int(loads.sum().item())
+            # the loads themselves cross over: a sum on the device takes two launches first
+            total = sum(loads.tolist() if host_loads is None else host_loads)
         shape = list(in_data.shape)
         if is_1d_routing:
             shape[0] = total
@@ -496,6 +505,11 @@ def split_fused_cells_to_paths(
     tags: Optional[torch.Tensor] = None,
 ):
     """src/backend/torch/router.cc:285-335: per-path views of the fused tensor."""
+    return _split(in_data, loads, max_path_padding, is_load_split, is_tag_split, tags)
+
+
+def _split(in_data, loads, max_path_padding, is_load_split, is_tag_split, tags=None,
+           host_loads=None):
     path_num = loads.numel()
     if is_tag_split:
         is_load_split = True
@@ -511,10 +525,11 @@ def split_fused_cells_to_paths(
             if is_tag_split:
                 tags_l.append(tags.narrow(0, i * mpl, mpl))
     else:
-        cpu_loads = loads.cpu().tolist()
+        if host_loads is None:
+            host_loads = loads.tolist()
         start = 0
         for i in range(path_num):
-            n = int(cpu_loads[i])
+            n = int(host_loads[i])
             datas.append(in_data.narrow(0, start, n))
             if is_load_split:
                 loads_l.append(loads.narrow(0, i, 1))
@@ -548,6 +563,58 @@ def fuse_split_cells_from_paths(
         new_tags, inverse = torch.unique(all_tags, sorted=True, return_inverse=True)
         return [out, new_tags, inverse]
     return [out]
+
+
+def _merge_paths_by_tag(in_data: List[torch.Tensor], tags: List[torch.Tensor], ever_padded: bool):
+    """``fuse_split_cells_from_paths`` with tags followed by the tag-index combine of its result,
+    without fusing the cells: the sum reads them where they are.  None when the paths are not
+    plain (then the two ops take them)."""
+    first = in_data[0]
+    if first.dtype not in _DT or not first.is_cuda or not 1 <= len(in_data) <= 128 or \
+            first.dim() < 1:
+        return None
+    dev, cell = first.device, first.shape[1:]
+    for data, tag in zip(in_data, tags):
+        if tag is None or data.device != dev or tag.device != dev or data.dtype != first.dtype \
+                or tag.dtype != torch.int32 or tag.dim() != 1 or data.shape[1:] != cell or \
+                not data.is_contiguous() or not tag.is_contiguous() or \
+                tag.size(0) != data.size(0):
+            return None
+    rows = [data.size(0) for data in in_data]
+    total, n = sum(rows), len(rows)
+    cell_size = cell.numel()
+    if total < 2 or cell_size == 0:
+        return None
+    datas_c = (ctypes.c_void_p * n)(*[data.data_ptr() for data in in_data])
+    rows_c = (ctypes.c_int64 * n)(*rows)
+    with _lib.device_guard(dev):
+        stream = _stream(dev)
+        nbytes = _lib.query("brt_tag_group_bytes", total)
+        if nbytes:
+            tags_c = (ctypes.c_void_p * n)(*[tag.data_ptr() for tag in tags])
+            groups = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+            new_tags = torch.empty(total, dtype=torch.int32, device=dev)
+            out_load = torch.empty(1, dtype=torch.int32, device=dev)
+            _lib.call("brt_group_pieces_by_tag", datas_c, tags_c, rows_c, n, cell_size,
+                      _DT[first.dtype], int(bool(ever_padded)), _ptr(new_tags), _ptr(out_load),
+                      _ptr(groups), nbytes, stream)
+            rows_out = int(out_load.item())  # the output's size: the one host read
+            out = torch.empty((rows_out,) + tuple(cell), dtype=first.dtype, device=dev)
+            _lib.call("brt_sum_grouped_pieces", datas_c, rows_c, n, _ptr(groups), _ptr(out),
+                      rows_out, cell_size, _DT[first.dtype], stream)
+            return [out, new_tags.narrow(0, 0, rows_out), out_load]
+        new_tags, inverse = torch.unique(torch.cat(tags, 0), sorted=True, return_inverse=True)
+        rows_out = new_tags.size(0)
+        out = torch.empty((rows_out,) + tuple(cell), dtype=first.dtype, device=dev)
+        index = inverse.to(torch.int32)
+        nbytes = _lib.query("brt_sum_rows_scratch_bytes", total, rows_out)
+        scratch = _scratch.get("row_sum", dev, nbytes)
+        _lib.call("brt_sum_pieces_by_index", datas_c, rows_c, n, _ptr(index), _ptr(out), rows_out,
+                  cell_size, _DT[first.dtype], _ptr(scratch), scratch.numel(), stream)
+        if ever_padded and int(new_tags[0].item()) == 0:
+            out, new_tags = out.narrow(0, 1, rows_out - 1), new_tags.narrow(0, 1, rows_out - 1)
+        out_load = torch.tensor([new_tags.numel()], dtype=torch.int32, device=dev)
+        return [out, new_tags, out_load]
 
 
 def combine_with_indices_and_loads(

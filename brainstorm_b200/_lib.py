@@ -43,6 +43,12 @@ SIGNATURES = {
                _int, _vp, _vp, _sz, _vp]),
     "brt_combine_with_records": (
         _int, [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _int, _i32, _int, _int, _int, _vp]),
+    "brt_sum_pieces_by_index": (
+        _int, [_vp, _vp, _int, _vp, _vp, _i64, _i64, _int, _vp, _sz, _vp]),
+    "brt_tag_group_bytes": (_sz, [_i64]),
+    "brt_group_pieces_by_tag": (
+        _int, [_vp, _vp, _vp, _int, _i64, _int, _int, _vp, _vp, _vp, _sz, _vp]),
+    "brt_sum_grouped_pieces": (_int, [_vp, _vp, _int, _vp, _vp, _i64, _i64, _int, _vp]),
     "brt_static_index_scratch_bytes": (_sz, []),
     "brt_generate_indices_and_loads_static": (
         _int, [_vp, _vp, _vp, _i64, _int, _vp, _int, _int, _int, _int, _vp]),

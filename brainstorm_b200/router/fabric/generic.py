@@ -78,38 +78,43 @@ class DispatchFabric(FabricBase):
             all_out_flows = all_out_flows[0]
         return all_out_flows, score
 
-    def _route(self, flow_data, route_indices, loads, score, flow_idx, flow_tag):
+    def _route(self, flow_data, route_indices, loads, score, flow_idx, flow_tag,
+               host_loads=None):
         # positional layout of the operator: (data, indices, loads, gates, tag_generating, tags,
         # max_path_padding, max_path_load, is_1d_routing)
-        return c_router.dispatch_with_indices_and_loads(
+        return c_router._dispatch(
             flow_data, route_indices, loads, score if self.transforms[flow_idx] else None,
             self.is_tag_index, flow_tag, self.max_path_padding, self.max_path_load,
-            self.route_logics[flow_idx] == "1d")
+            self.route_logics[flow_idx] == "1d", host_loads=host_loads)
 
     def dispatch(self, in_flows: List[GridTensor], route_indices: torch.Tensor,
                  loads: torch.Tensor, score: torch.Tensor
                  ) -> Tuple[List[List[GridTensor]], torch.Tensor]:
         all_out_flows = []
         path_num = route_indices.size(1)
+        # packed paths: the loads are read once for the sizes of the outputs and for the cuts
+        # between the paths, which the host then makes while the cells move
+        host_loads = None if self.max_path_padding else loads.tolist()
         for flow_idx in range(self.flow_num):
             data, tag_stack, load_stack, extra = to_torch_tensor(in_flows[flow_idx],
                                                                  retrieve_attr=True)
             flow_tag = tag_stack[-1]
             tag_stack, load_stack = tag_stack[:-1], load_stack[:-1]
-            routed = self._route(data, route_indices, loads, score, flow_idx, flow_tag)
+            routed = self._route(data, route_indices, loads, score, flow_idx, flow_tag,
+                                 host_loads)
             if self.is_tag_index:
                 routed_data, routed_tags = routed
-                datas, split_loads, split_tags = c_router.split_fused_cells_to_paths(
+                datas, split_loads, split_tags = c_router._split(
                     routed_data, loads, self.max_path_padding, is_load_split=True,
-                    is_tag_split=True, tags=routed_tags)
+                    is_tag_split=True, tags=routed_tags, host_loads=host_loads)
                 out_flows = [
                     init_grid_tensor(datas[i], tag_stack + [split_tags[i]],
                                      load_stack + [split_loads[i]], extra)
                     for i in range(path_num)]
             else:
-                (datas,) = c_router.split_fused_cells_to_paths(
+                (datas,) = c_router._split(
                     routed[0], loads, self.max_path_padding, is_load_split=False,
-                    is_tag_split=False)
+                    is_tag_split=False, host_loads=host_loads)
                 out_flows = [
                     init_grid_tensor(datas[i], tag_stack + [route_indices], load_stack + [loads],
                                      extra)
@@ -158,6 +163,14 @@ class CombineFabric(FabricBase):
                 load_stack[-1] = torch.tensor([data.shape[0]], dtype=torch.int32,
                                               device=data.device)
                 out_flows.append(init_grid_tensor(data, tag_stack, load_stack, extra))
+                continue
+            result = None
+            if self.is_tag_index and residual is None:
+                result = c_router._merge_paths_by_tag(datas, tags, self.ever_padded)
+            if result is not None:
+                out_data, out_tag, out_load = result
+                out = init_grid_tensor(out_data, tag_stack[:-1], load_stack[:-1], extra)
+                out_flows.append(out.pack(out_tag, out_load))
                 continue
             if self.is_tag_index:
                 fused, fused_tags, route_indices = c_router.fuse_split_cells_from_paths(

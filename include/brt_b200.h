@@ -353,6 +353,38 @@ BRT_API int brt_sum_rows_by_index(const void* in_rows, const int32_t* row_index,
                                   int64_t rows_in, int64_t rows_out, int64_t cell_size,
                                   int dtype, void* scratch, size_t scratch_bytes, void* stream);
 
+/*
+ * The same over rows that lie in up to 128 pieces (one tensor per path, numbered through in the
+ * order given): in_pieces[i] holds piece_rows[i] rows; both arrays are host memory, read before
+ * the call returns.  Scratch: brt_sum_rows_scratch_bytes of all rows.
+ */
+BRT_API int brt_sum_pieces_by_index(const void* const* in_pieces, const int64_t* piece_rows,
+                                    int pieces, const int32_t* row_index, void* out_rows,
+                                    int64_t rows_out, int64_t cell_size, int dtype,
+                                    void* scratch, size_t scratch_bytes, void* stream);
+
+/*
+ * Merging paths by tag in two calls with one host read between them (the number of distinct tags
+ * sizes the output): what the reference's combine fabric does with torch.cat, torch.unique and
+ * scatter_reduce (src/backend/torch/router.cc:348-369,449-472).
+ *
+ * brt_group_pieces_by_tag  tag_pieces[i]: int32 tags of the piece_rows[i] rows of in_pieces[i].
+ *                          tags_out (room for all rows) <- the distinct tags, ascending;
+ *                          count[0] <- how many; groups (brt_tag_group_bytes, 256-byte aligned)
+ *                          <- what the second call reads.  drop_zero != 0 leaves tag 0 out.
+ *                          BRT_ERR_UNSUPPORTED outside 2 .. 4096 rows.
+ * brt_sum_grouped_pieces   out_rows[g] <- the sum of the rows of the g-th tag, ascending rows,
+ *                          fp32, rounded once; rows_out = count[0].  The same pieces as before.
+ */
+BRT_API size_t brt_tag_group_bytes(int64_t rows_in);
+BRT_API int brt_group_pieces_by_tag(const void* const* in_pieces, const void* const* tag_pieces,
+                                    const int64_t* piece_rows, int pieces, int64_t cell_size,
+                                    int dtype, int drop_zero, int32_t* tags_out, int32_t* count,
+                                    void* groups, size_t group_bytes, void* stream);
+BRT_API int brt_sum_grouped_pieces(const void* const* in_pieces, const int64_t* piece_rows,
+                                   int pieces, const void* groups, void* out_rows,
+                                   int64_t rows_out, int64_t cell_size, int dtype, void* stream);
+
 /* ------------------------------------------------------------------ experts: grouped GEMM */
 
 /*
