@@ -10,6 +10,10 @@ deliberate:
 * kernels are enqueued on the *current* stream (the reference uses the default stream;
   identical when the current stream is the default one);
 * outputs are never pre-zeroed by a separate memset: the kernels write every byte.
+
+The hot operators first offer the call to ``_lib.host_ops()``, which takes plain calls
+(contiguous CUDA tensors of the right types on the current device) in native code and
+declines everything else; the Python below is the whole operator.
 """
 import ctypes
 import os
@@ -169,6 +173,11 @@ def generate_indices_and_loads(
 ):
     """src/backend/torch/router.cc:48-80."""
     _check_cuda(hot_mask, "hot_mask")
+    if not is_tag_index:
+        done = _lib.host_ops().scan(hot_mask, None, None, supported_capacities,
+                                    capacity_padding, path_wise_padding, False)
+        if done is not None:
+            return done
     check_index_status()
     hot_mask = _int32c(hot_mask, "hot_mask")
     T, E = hot_mask.shape
@@ -217,6 +226,11 @@ def throttle_and_generate_indices(
     _check_cuda(hot_mask, "hot_mask")
     _check_cuda(prefix, "prefix")
     _check_cuda(threshold, "threshold")
+    done = _lib.host_ops().scan(hot_mask, prefix, threshold, supported_capacities,
+                                capacity_padding, path_wise_padding, with_mask)
+    if done is not None:
+        indices, loads, throttled = done
+        return (indices, loads, prefix, throttled) if with_mask else (indices, loads, prefix)
     check_index_status()
     if hot_mask.size(1) != prefix.size(0) or hot_mask.size(1) != threshold.size(0):
         raise RuntimeError("CHECK_EQ fails.")
@@ -295,6 +309,22 @@ def route_scores(
     ``NotImplementedError`` when the scores do not fit the single-launch kernel; callers then
     route in two steps."""
     _check_cuda(score, "score")
+    if decision in _GATE and output in _ROUTE_OUT:
+        done = _lib.host_ops().route_scores(
+            score, _GATE[decision], top_k, threshold, residual_path, _ROUTE_OUT[output],
+            supported_capacities, capacity_padding, path_wise_padding, prefix,
+            throttle_capacity, with_gates, with_mask)
+        if done is not None:
+            out, loads, gates, mask_out = done
+            if output == "throttled_seat_indices":
+                res = (out, loads, prefix)
+            else:
+                res = (out, prefix if output == "throttled_mask" else loads)
+            if with_gates:
+                res += (gates,)
+            if with_mask:
+                res += (mask_out,)
+            return res
     check_index_status()
     if decision not in _GATE or output not in _ROUTE_OUT:
         raise RuntimeError(f"unknown decision {decision!r} or output {output!r}")
@@ -408,6 +438,18 @@ def _dispatch(in_data, route_indices, loads, gates, tag_generating, tags, max_pa
     """The dispatch operator; ``host_loads``: the loads as the caller has already read them."""
     _check_cuda(in_data, "in_data")
     _check_cuda(route_indices, "route_indices")
+    if is_1d_routing and _USE_DENSE and not tag_generating and not is_tag_index and \
+            in_data.size(0) > 0:
+        if not max_path_padding:
+            if host_loads is None:
+                host_loads = loads.tolist()
+            slot, total = 0, sum(host_loads)
+        else:
+            slot, total = max_path_load, max_path_load * route_indices.size(1)
+        if slot > 0 or not max_path_padding:
+            done = _lib.host_ops().dispatch(in_data, route_indices, loads, gates, slot, total)
+            if done is not None:
+                return [done]
     dev = in_data.device
     with _lib.device_guard(dev):
         cell_num = in_data.size(0)
@@ -631,6 +673,11 @@ def combine_with_indices_and_loads(
     """src/backend/torch/router.cc:372-473."""
     _check_cuda(in_data, "in_data")
     _check_cuda(route_indices, "route_indices")
+    if not is_tag_index and loads is not None and _USE_DENSE:
+        done = _lib.host_ops().combine(in_data, route_indices, loads, gates, out_data,
+                                       max_path_padding)
+        if done is not None:
+            return [done]
     dev = in_data.device
     with _lib.device_guard(dev):
         cell_num = route_indices.size(0)

@@ -150,6 +150,23 @@ def load():
     return lib
 
 
+_host = None
+
+
+def host_ops():
+    """The native host side of the hot operators (``csrc/host_ops.cpp``); raises if missing."""
+    global _host
+    if _host is None:
+        load()
+        try:
+            from . import _host_ops
+        except ImportError as exc:
+            raise BrtError(f"{_PKG / '_host_ops.so'} does not load ({exc}): build it with "
+                           "`python -m brainstorm_b200.build`") from None
+        _host = _host_ops
+    return _host
+
+
 def exported(name: str) -> bool:
     return hasattr(load(), name)
 

@@ -4,7 +4,8 @@
     python -m brainstorm_b200.build [--force] [--verbose]
 
 The library has no Python or torch dependency; ``brainstorm_b200._lib`` loads it
-with ctypes.  nvcc cross-compiles without a GPU.
+with ctypes.  nvcc cross-compiles without a GPU.  ``_host_ops.so``, the native host side of the
+router's hot operators, is a small extension module on top of it (g++, torch's headers).
 """
 import os
 import shutil
@@ -17,6 +18,8 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 INCLUDE = PKG.parent / "include"
 LIB = PKG / "libbrt_b200.so"
+HOST_SRC = CSRC / "host_ops.cpp"
+HOST_LIB = PKG / "_host_ops.so"
 OBJ_DIR = PKG / "build"
 
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -65,9 +68,39 @@ def _stale() -> bool:
     return LIB.stat().st_mtime < newest
 
 
+def build_host(force: bool = False) -> Path:
+    if not force and HOST_LIB.exists() and \
+            HOST_LIB.stat().st_mtime >= max(p.stat().st_mtime for p in
+                                            [HOST_SRC, LIB, *INCLUDE.glob("*.h")]):
+        return HOST_LIB
+    import sysconfig
+
+    import torch
+
+    base = Path(torch.__file__).resolve().parent
+    cuda = Path(_nvcc()).resolve().parent.parent
+    cxx = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else "g++"
+    cmd = [cxx, "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           f"-I{base / 'include'}", f"-I{base / 'include/torch/csrc/api/include'}",
+           f"-I{sysconfig.get_paths()['include']}", f"-I{cuda / 'include'}", str(HOST_SRC),
+           "-o", str(HOST_LIB), f"-L{base / 'lib'}", "-ltorch_python", "-ltorch", "-ltorch_cpu",
+           "-ltorch_cuda", "-lc10", "-lc10_cuda", f"-L{PKG}", f"-l:{LIB.name}",
+           "-Wl,-rpath,$ORIGIN"]
+    proc = subprocess.run(cmd, capture_output=True, text=True)
+    if proc.returncode != 0:
+        raise RuntimeError(f"$ {' '.join(cmd)}\n{proc.stdout}\n{proc.stderr}")
+    return HOST_LIB
+
+
 def build(force: bool = False, verbose: bool = False) -> Path:
-    if not force and not _stale():
-        return LIB
+    if force or _stale():
+        build_library(verbose)
+    build_host(force)
+    return LIB
+
+
+def build_library(verbose: bool = False) -> Path:
     nvcc = _nvcc()
     OBJ_DIR.mkdir(exist_ok=True)
     nccl_inc, nccl_link = _nccl_flags()

@@ -1,0 +1,157 @@
+"""The native host side of the router operators against the Python operators alone, over the forms
+of calls that programs make: plain ones (which it takes), and other orders, strides, types,
+devices and kinds of tensors (which it has to decline), errors included."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+class Declines:
+    def __getattr__(self, name):
+        return lambda *args: None
+
+
+@pytest.fixture
+def both(monkeypatch):
+    """Run a function natively and without the native side; results and errors must agree."""
+    from brainstorm_b200 import _lib
+
+    native = _lib.host_ops()
+
+    def outcome(make):
+        try:
+            return flat(make()), None
+        except Exception as exc:  # noqa: BLE001 - whatever an operator raises
+            return None, (type(exc), str(exc))
+
+    def flat(value):
+        if isinstance(value, torch.Tensor):
+            return [value]
+        return [t for v in value for t in flat(v)]
+
+    def run(make):
+        monkeypatch.setattr(_lib, "host_ops", lambda: native)
+        got, error = outcome(make)
+        monkeypatch.setattr(_lib, "host_ops", lambda: Declines())
+        want, expected = outcome(make)
+        monkeypatch.setattr(_lib, "host_ops", lambda: native)
+        assert error == expected
+        if want is not None:
+            assert len(got) == len(want)
+            for a, b in zip(got, want):
+                assert a.dtype == b.dtype and a.shape == b.shape and a.device == b.device
+                assert a.stride() == b.stride() and type(a) is type(b)
+                assert torch.equal(a, b)
+        return got, error
+
+    return run
+
+
+def masks(cells, paths):
+    g = torch.Generator(device="cuda").manual_seed(cells + paths)
+    m = (torch.rand((cells, paths), generator=g, device="cuda") < 0.2).to(torch.int32)
+    wide = torch.zeros((cells, paths + 4), dtype=torch.int32, device="cuda")
+    wide[:, :paths] = m
+    return {"plain": m, "transposed": m.t().contiguous().t(), "slice": wide[:, :paths],
+            "int64": m.long(), "cpu": m.cpu(), "empty": m[:0]}
+
+
+@pytest.mark.parametrize("form", ["plain", "transposed", "slice", "int64", "cpu", "empty"])
+@pytest.mark.parametrize("cells,paths", [(64, 32), (1000, 30), (65536, 32)])
+def test_scans(both, cells, paths, form):
+    from brainstorm_b200._C import router as R
+
+    mask = masks(cells, paths)[form]
+    caps = torch.tensor([3, 9], dtype=torch.int32, device="cuda")
+    each = torch.full((paths,), 7, dtype=torch.int32, device="cuda")
+    for args in [(mask,), (mask, caps), (mask, caps, True), (mask, each, True, True),
+                 (mask, None, True), (mask, caps.long()), (mask, each[:2], True, True),
+                 (mask, caps, False, False, True)]:
+        both(lambda: R.generate_indices_and_loads(*args))
+    limit = torch.full((paths,), 5, dtype=torch.int32, device="cuda")
+    for with_mask in (False, True):
+        for thr in (limit, limit.long(), limit[:-1], limit.cpu()):
+            both(lambda: R.throttle_and_generate_indices(
+                mask, torch.ones(paths, dtype=torch.int32, device="cuda"), thr, caps,
+                with_mask=with_mask))
+
+
+@pytest.mark.parametrize("cells,paths", [(64, 32), (1000, 30), (65536, 32), (5, 260)])
+def test_gates(both, cells, paths):
+    from brainstorm_b200._C import router as R
+
+    score = torch.rand((cells, paths), device="cuda",
+                       generator=torch.Generator(device="cuda").manual_seed(cells))
+    limit = torch.full((paths,), 5, dtype=torch.int32, device="cuda")
+    for s in (score, score.double(), score.t().contiguous().t(), score.cpu(), score[:0]):
+        for output in ("mask", "throttled_mask", "seat_indices", "throttled_seat_indices", "none"):
+            for k in (1, 2, 0, paths + 1):
+                for extras in (False, True):
+                    both(lambda: R.route_scores(
+                        s, "topk", k, output=output, supported_capacities=limit,
+                        prefix=torch.zeros(paths, dtype=torch.int32, device="cuda"),
+                        throttle_capacity=limit, with_gates=extras, with_mask=extras))
+        both(lambda: R.route_scores(s, "threshold", threshold=0.5, residual_path=0))
+        both(lambda: R.route_scores(s, "threshold", threshold=1, residual_path=paths))
+        both(lambda: R.route_scores(s, "topk", 1, output="throttled_mask"))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16, torch.float64])
+@pytest.mark.parametrize("width", [(16,), (3,), (2, 5, 4)])
+@pytest.mark.parametrize("cells,paths", [(64, 32), (1, 4), (65536, 33)])
+def test_moves(both, cells, paths, dtype, width):
+    from brainstorm_b200 import Annotator
+    from brainstorm_b200._C import router as R
+
+    mask = masks(cells, paths)["plain"]
+    mask[0, 0] = 1
+    x = torch.randn((cells,) + width, device="cuda").to(dtype)
+    gates = torch.rand((cells, paths), device="cuda")
+    indices, loads = R.generate_indices_and_loads(mask)
+    slot = int(loads.max())
+    strided = torch.zeros((cells, 2) + width, device="cuda", dtype=dtype)[:, 0]
+    strided.copy_(x)
+    for data in (x, strided, Annotator([0])(x.clone()), x.cpu(), x[:0]):
+        for idx in (indices, indices.clone()):
+            for lo in (loads, loads.cpu(), loads.long()):
+                for gate in (None, gates.to(dtype), gates.half()):
+                    for padded, mpl in ((True, slot), (True, 0), (False, 0), (True, -1)):
+                        if data.is_cuda and data.size(0) and mpl < 0:
+                            continue  # a slot of no rows is not defined
+                        both(lambda: R.dispatch_with_indices_and_loads(
+                            data, idx, lo, gate, False, None, padded, mpl))
+    if dtype == torch.float64 or (dtype == torch.float16 and width == (3,)):
+        return  # refused above, natively and not
+    (rows,) = R.dispatch_with_indices_and_loads(x, indices, loads, None, False, None, True, slot)
+    base = torch.randn((cells,) + width, device="cuda").to(dtype)
+    for data in (rows, rows.cpu(), torch.cat([rows, rows])[::2] * 0 + rows):
+        for lo in (loads, loads.cpu(), loads.long(), None):
+            for gate in (None, gates, gates.to(dtype), gates.double(), gates.t().contiguous().t()):
+                for out in (False, True):
+                    both(lambda: R.combine_with_indices_and_loads(
+                        data, indices, lo, gate, base.clone() if out else None, True))
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        both(lambda: R.combine_with_indices_and_loads(rows, indices, loads, gates, None, True))
+        both(lambda: R.dispatch_with_indices_and_loads(x, indices, loads, None, False, None, True,
+                                                       slot))
+    side.synchronize()
+    with torch.inference_mode():
+        both(lambda: R.generate_indices_and_loads(mask))
+        idx, lo = R.generate_indices_and_loads(mask)
+        both(lambda: R.dispatch_with_indices_and_loads(x, idx, lo, None, False, None, True, slot))
+        both(lambda: R.combine_with_indices_and_loads(rows, idx, lo, gates, None, True))
+
+
+def test_residual_is_returned_itself_and_notes_travel():
+    from brainstorm_b200._C import router as R
+
+    indices, loads = R.generate_indices_and_loads(masks(65536, 32)["plain"])
+    assert getattr(indices, R._DENSE).data_ptr() == loads.data_ptr() + 4 * 32
+    assert R._records_of(indices, 65536, 32) is not None
+    rows = torch.randn((int(loads.sum()), 8), device="cuda")
+    base = torch.randn((65536, 8), device="cuda")
+    (out,) = R.combine_with_indices_and_loads(rows, indices, loads, None, base)
+    assert out is base
