@@ -27,6 +27,7 @@
 // through a slower serial walk of the index row, so any number of routes is correct.
 #include "row_move.cuh"
 
+#include <algorithm>
 #include <cstdlib>
 #include <cstring>
 #include <initializer_list>
@@ -48,9 +49,9 @@ __global__ void __launch_bounds__(kThreads, 4) dispatch_seat_kernel(const MoveAr
   int* s_base = s_mem + a.path_num;
   int* s_written = s_base + a.path_num;
   int* s_fill = s_written + a.path_num;
-  setup_paths(a.loads, a.path_num, a.max_path_load, s_loads, s_base);
+  setup_tables(a.loads, a.dense_counts, a.path_num, a.max_path_load, s_loads, s_base, s_written,
+               s_fill);
   const bool dense = a.dense_counts != nullptr;
-  if (dense) setup_fill(a.dense_counts, a.path_num, a.max_path_load, s_loads, s_written, s_fill);
 
   const int lane = threadIdx.x & 31;
   const int64_t warp = (int64_t)blockIdx.x * kWarps + (threadIdx.x >> 5);
@@ -209,7 +210,7 @@ __global__ void __launch_bounds__(kThreads) dispatch_tag_kernel(const MoveArgs a
   extern __shared__ int s_mem[];
   int* s_loads = s_mem;
   int* s_base = s_mem + a.path_num;
-  setup_paths(a.loads, a.path_num, a.max_path_load, s_loads, s_base);
+  setup_tables(a.loads, nullptr, a.path_num, a.max_path_load, s_loads, s_base, nullptr, nullptr);
 
   const int lane = threadIdx.x & 31;
   const int64_t warp = (int64_t)blockIdx.x * kWarps + (threadIdx.x >> 5);
@@ -276,7 +277,7 @@ __global__ void __launch_bounds__(kThreads) dispatch_tag_kernel(const MoveArgs a
 // GMODE: 0 = no gates, 1 = fp32 gates, 2 = gates stored in the data type.
 // 16-byte rows only (VB == 16).  IV: paths per lane of an index row scan, or 0: the routes come
 // from the cells' records, 32 bytes per cell in place of an index and a gate row, and only the
-// gates of kept routes are read (262144 x 128, top-1, rows of 1.5 KB: 127 us -> 93).
+// gates of kept routes are read (262144 x 128, top-1, rows of 1.5 KB: 127 us -> 92).
 template <int IV>
 struct FoldStageOf {
   using type = FoldStage;
@@ -297,7 +298,7 @@ __global__ void __launch_bounds__(kThreads, 3) combine_seat_async_kernel(const M
   Stage* s_stage = reinterpret_cast<Stage*>(s_raw);  // [kWarps][kStages]
   int* s_loads = reinterpret_cast<int*>(s_raw + sizeof(Stage) * kWarps * kStages);
   int* s_base = s_loads + a.path_num;
-  setup_paths(a.loads, a.path_num, a.max_path_load, s_loads, s_base);
+  setup_tables(a.loads, nullptr, a.path_num, a.max_path_load, s_loads, s_base, nullptr, nullptr);
 
   const int lane = threadIdx.x & 31;
   const int warp_in_cta = threadIdx.x >> 5;
@@ -481,7 +482,8 @@ __global__ void __launch_bounds__(kThreads, 3) combine_seat_async_kernel(const M
 // copy of the warp's NEXT item is in flight while the current one is stored to its routes,
 // and cells that no path kept are never read.  IV: paths per lane of an index row scan, or 0: the
 // routes come from the cells' records (262144 x 128, top-1, rows of 1.5 KB: 192 us ->
-// 181, of which the 748 MB of zero rows take 140).
+// 181; with the CTAs in order, see plan_dispatch, 145: 5.9 TB/s).  Zero rows are written before
+// the wait for the item's own row.
 template <int DT, bool WEIGHTED, int IV>
 __global__ void __launch_bounds__(kThreads, WEIGHTED ? 3 : 4) dispatch_seat_async_kernel(const MoveArgs a) {
   constexpr int VB = 16;
@@ -496,22 +498,15 @@ __global__ void __launch_bounds__(kThreads, WEIGHTED ? 3 : 4) dispatch_seat_asyn
   int* s_base = s_loads + a.path_num;
   int* s_written = s_base + a.path_num;
   int* s_fill = s_written + a.path_num;
-  setup_paths(a.loads, a.path_num, a.max_path_load, s_loads, s_base);
-  const bool dense = a.dense_counts != nullptr;
-  if (dense) setup_fill(a.dense_counts, a.path_num, a.max_path_load, s_loads, s_written, s_fill);
 
   const int lane = threadIdx.x & 31;
   const int warp_in_cta = threadIdx.x >> 5;
-  const int64_t warp = (int64_t)blockIdx.x * kWarps + warp_in_cta;
-  const int64_t warps = (int64_t)gridDim.x * kWarps;
-  const int64_t items = a.cell_num * a.pieces_per_row;
+  WarpItems items(a);
   const V* __restrict__ src = static_cast<const V*>(a.src);
   V* __restrict__ dst = static_cast<V*>(a.dst);
   const int E = a.path_num;
   CopyStage* my = s_stage + warp_in_cta * kStages;
   const unsigned long long evict_first = l2_evict_first_policy();
-  FillPacer pace(items, dense ? (int64_t)s_fill[E] * a.pieces_per_row : 0, warp, warps);
-
   int seat[kScan];
   float gate[kScan];
   uint2 record = make_uint2(0u, 0u);
@@ -574,13 +569,13 @@ __global__ void __launch_bounds__(kThreads, WEIGHTED ? 3 : 4) dispatch_seat_asyn
     cp_async_commit();
   };
 
-  const ItemStep step = step_of(warps, a.pieces_per_row);
-  ItemCursor at = cursor_at(warp < items ? warp : 0, a.pieces_per_row);
-  if (warp >= items) at.cell = a.cell_num;
-  ItemCursor ahead = advance(at, step);
-  ItemCursor ahead2 = advance(ahead, step);
+  ItemCursor at = items.next(), ahead = items.next(), ahead2 = items.next();
   int stage = 0;
-  fetch(at);
+  fetch(at);  // under way while the tables are made
+  setup_tables(a.loads, a.dense_counts, a.path_num, a.max_path_load, s_loads, s_base, s_written,
+               s_fill);
+  const bool dense = a.dense_counts != nullptr;
+  WarpFill<VB> fill(dense ? (int64_t)s_fill[E] * a.pieces_per_row : 0, a.turns);
   issue(my[0], at);
   fetch(ahead);
   while (at.cell < a.cell_num) {
@@ -590,6 +585,7 @@ __global__ void __launch_bounds__(kThreads, WEIGHTED ? 3 : 4) dispatch_seat_asyn
     }
     issue(my[stage ^ 1], ahead);
     fetch(ahead2);
+    if (dense) fill.run(a, fill.per_turn, s_base, s_written, s_fill, lane);
     cp_async_wait<1>();
     if constexpr (kRecords && WEIGHTED)
       if (held_slot_of[0] >= 0) my[stage].route[held_slot_of[0]].gate = held_gate_of[0];
@@ -649,18 +645,14 @@ __global__ void __launch_bounds__(kThreads, WEIGHTED ? 3 : 4) dispatch_seat_asyn
         }
       }
     }
-    if (dense)
-      for (int n = pace.due(); n > 0 && pace.next < pace.end; n--, pace.next += pace.stride)
-        fill_item<VB>(a, s_base, s_written, s_fill, pace.next, lane);
     __syncwarp();
     at = ahead;
     ahead = ahead2;
-    ahead2 = advance(ahead2, step);
+    ahead2 = items.next();
     stage ^= 1;
   }
   cp_async_wait<0>();
-  for (; pace.next < pace.end; pace.next += pace.stride)
-    fill_item<VB>(a, s_base, s_written, s_fill, pace.next, lane);
+  if (dense) fill.run(a, 0x7fffffff, s_base, s_written, s_fill, lane);
 }
 
 // Register-only combine for rows that cannot be moved 16 bytes at a time.
@@ -671,7 +663,7 @@ __global__ void __launch_bounds__(kThreads) combine_seat_kernel(const MoveArgs a
   extern __shared__ int s_mem[];
   int* s_loads = s_mem;
   int* s_base = s_mem + a.path_num;
-  setup_paths(a.loads, a.path_num, a.max_path_load, s_loads, s_base);
+  setup_tables(a.loads, nullptr, a.path_num, a.max_path_load, s_loads, s_base, nullptr, nullptr);
 
   const int lane = threadIdx.x & 31;
   const int64_t warp = (int64_t)blockIdx.x * kWarps + (threadIdx.x >> 5);
@@ -788,6 +780,33 @@ unsigned grid_for_resident(int64_t items, int ctas_per_sm) {
   return (unsigned)blocks;
 }
 
+// The grid of the pipelined dispatch, and in a.turns how many items each warp takes.  A CTA
+// owns a few consecutive items per warp and ends: the hardware launches CTAs in order, so all
+// SMs work inside one narrow window that advances through memory.  CTAs that stay and stride
+// over the grid's width drift apart, which costs DRAM bandwidth (a plain fill of 800 MB: 5.8 TB/s
+// striding, 7.1 in order).  How many items: enough to hide a CTA's start, few enough to keep the
+// window narrow.  Measured, striding / 2 / 4 / 8 items per warp: 65536 x 64 packed rows of 4 KB
+// 147 / 129 / 133 / 136 us; 64 samples of 3 MiB 185 / 166 / 171 / 185; with capacity padding, where
+// a turn is mostly zero rows, 262144 x 128 181 / 173 / 145 / 150 and 32768 x 32 36.4 / 35.6 / 35.0 /
+// 35.0.  So 2 for packed rows, 4 with slots of a fixed size; when that leaves SMs idle although
+// there are rows to zero, the items are spread over one resident wave.
+// (The combine was measured in the same way and keeps its resident CTAs: 26 / 33 / 31 / 33 us at
+// 32768 x 32, 92 / 157 / 127 / 115 at 262144 x 128: its three CTAs per SM have little beside them
+// to cover a start, and it reads more than it writes.)
+unsigned plan_dispatch(MoveArgs& a, int ctas_per_sm) {
+  const int64_t items = a.cell_num * a.pieces_per_row;
+  const int64_t fills = a.dense_counts != nullptr ? a.total_rows * a.pieces_per_row : 0;
+  a.turns = a.max_path_load != 0 ? 4 : 2;
+  int64_t ctas = (items + kWarps * a.turns - 1) / (kWarps * a.turns);
+  const int64_t resident = (int64_t)sm_count() * ctas_per_sm;
+  const int64_t useful = std::min((std::max(items, fills) + kWarps - 1) / kWarps, resident);
+  if (ctas < useful) {
+    ctas = useful;
+    a.turns = (int)std::max((items + ctas * kWarps - 1) / (ctas * kWarps), (int64_t)1);
+  }
+  return (unsigned)std::max(ctas, (int64_t)1);
+}
+
 // 16-byte scans of index (and gate) rows need path_num % 4 == 0 and aligned arrays.
 bool wide_rows(const int* indices, const void* gates, int gate_elem_bytes, int path_num) {
   if (path_num % 4 != 0 || !aligned_to(indices, 16)) return false;
@@ -820,21 +839,20 @@ void launch_dispatch(const MoveArgs& a, bool is_tag, cudaStream_t st) {
   } else if (VB == 16 && IS_1D) {
     if constexpr (VB == 16 && IS_1D) {
       const size_t smem_async = sizeof(CopyStage) * kWarps * kStages + smem;
-      const int64_t work = (a.cell_num + (a.dense_counts != nullptr ? a.total_rows : 0)) *
-                           a.pieces_per_row;
-      const unsigned grid = grid_for_resident(work, WEIGHTED ? 3 : 4);
+      MoveArgs b = a;
+      const unsigned grid = plan_dispatch(b, WEIGHTED ? 3 : 4);
       if (a.records != nullptr) {
         configure_smem<dispatch_seat_async_kernel<DT, WEIGHTED, 0>>(sizeof(CopyStage) * kWarps *
                                                                     kStages);
-        dispatch_seat_async_kernel<DT, WEIGHTED, 0><<<grid, kThreads, smem_async, st>>>(a), note_launch();
+        dispatch_seat_async_kernel<DT, WEIGHTED, 0><<<grid, kThreads, smem_async, st>>>(b), note_launch();
       } else if (wide_rows(a.indices, a.gates, dtype_size(DT), a.path_num)) {
         configure_smem<dispatch_seat_async_kernel<DT, WEIGHTED, 4>>(sizeof(CopyStage) * kWarps *
                                                                     kStages);
-        dispatch_seat_async_kernel<DT, WEIGHTED, 4><<<grid, kThreads, smem_async, st>>>(a), note_launch();
+        dispatch_seat_async_kernel<DT, WEIGHTED, 4><<<grid, kThreads, smem_async, st>>>(b), note_launch();
       } else {
         configure_smem<dispatch_seat_async_kernel<DT, WEIGHTED, 1>>(sizeof(CopyStage) * kWarps *
                                                                     kStages);
-        dispatch_seat_async_kernel<DT, WEIGHTED, 1><<<grid, kThreads, smem_async, st>>>(a), note_launch();
+        dispatch_seat_async_kernel<DT, WEIGHTED, 1><<<grid, kThreads, smem_async, st>>>(b), note_launch();
       }
     }
   } else {

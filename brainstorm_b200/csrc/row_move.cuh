@@ -141,6 +141,66 @@ __device__ __forceinline__ void setup_fill(const int* __restrict__ counts, int p
   __syncthreads();
 }
 
+// Both tables at once, by all threads of the CTA: one path per thread and round, the loads and
+// counts of a round in flight together.  s_written / s_fill are left alone without counts.
+// (A CTA of a large dispatch lives for some ten microseconds; one warp walking 128 paths, one
+// dependent load after the other, took three of them.)
+__device__ __forceinline__ void setup_tables(const int* __restrict__ loads,
+                                             const int* __restrict__ counts, int path_num,
+                                             int max_path_load, int* s_loads, int* s_base,
+                                             int* s_written, int* s_fill) {
+  __shared__ int s_part[2][kWarps];
+  const int lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5;
+  const bool dense = counts != nullptr;
+  int carry_rows = 0, carry_empty = 0;
+  for (int p = 0; p < path_num; p += kThreads) {
+    const int e = p + threadIdx.x;
+    const int load = e < path_num ? loads[e] : 0;
+    const int count = dense && e < path_num ? counts[e] : 0;
+    const int have = count > 0 ? count : 0;
+    const int room = load > 0 ? load : 0;
+    const int written = have < room ? have : room;
+    const int slot = max_path_load != 0 ? max_path_load : room;
+    const int empty = dense && e < path_num && slot > written ? slot - written : 0;
+    int rows_incl = load, empty_incl = empty;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int rn = __shfl_up_sync(0xffffffffu, rows_incl, d);
+      const int en = __shfl_up_sync(0xffffffffu, empty_incl, d);
+      if (lane >= d) { rows_incl += rn; empty_incl += en; }
+    }
+    if (lane == 31) {
+      s_part[0][warp] = rows_incl;
+      s_part[1][warp] = empty_incl;
+    }
+    __syncthreads();
+    int rows_before = carry_rows, empty_before = carry_empty;
+#pragma unroll
+    for (int w = 0; w < kWarps; w++) {
+      if (w < warp) {
+        rows_before += s_part[0][w];
+        empty_before += s_part[1][w];
+      }
+      carry_rows += s_part[0][w];
+      carry_empty += s_part[1][w];
+    }
+    if (e < path_num) {
+      s_loads[e] = load;
+      s_base[e] = max_path_load != 0 ? e * max_path_load : rows_before + rows_incl - load;
+      if (dense) {
+        s_written[e] = written;
+        s_fill[e] = empty_before + empty_incl - empty;
+      }
+    }
+    __syncthreads();
+  }
+  if (dense) {
+    if (threadIdx.x == 0) s_fill[path_num] = carry_empty;
+    __syncthreads();
+  }
+}
+
 template <int VB, int DT>
 struct Lanes {
   using V = typename Chunk<VB>::type;
@@ -238,6 +298,7 @@ struct MoveArgs {
   int path_num;
   int max_path_load;
   int64_t total_rows;  // dispatch: output rows
+  int turns = 0;       // pipelined dispatch: items per warp; a CTA owns kWarps * turns of them
   int is_residual;     // combine only
 };
 
@@ -367,6 +428,79 @@ __device__ __forceinline__ void fill_item(const MoveArgs& a, const int* s_base,
   }
   if (piece == 0 && lane == 0 && a.new_tags != nullptr) a.new_tags[row] = 0;
 }
+
+// The items of a warp in a grid whose CTAs own kWarps * turns consecutive ones each, in order:
+// the CTA's first + warp, + kWarps, ...  A cursor past the last one has cell == cell_num.
+struct WarpItems {
+  ItemStep step;
+  int64_t cell_num;
+  int mine, given;  // items of this warp; how many have been handed out
+  ItemCursor last;
+  __device__ __forceinline__ explicit WarpItems(const MoveArgs& a) {
+    const int64_t items = a.cell_num * a.pieces_per_row;
+    step = step_of(kWarps, a.pieces_per_row);
+    cell_num = a.cell_num;
+    const int64_t span = (int64_t)kWarps * a.turns;
+    const int64_t first = blockIdx.x * span + (threadIdx.x >> 5);
+    const int64_t end = min((int64_t)(blockIdx.x + 1) * span, items);
+    mine = first < end ? (int)((end - first + kWarps - 1) / kWarps) : 0;
+    given = 0;
+    last = cursor_at(mine > 0 ? first : 0, a.pieces_per_row);
+  }
+  __device__ __forceinline__ ItemCursor next() {
+    if (given > 0 && given < mine) last = advance(last, step);
+    if (given >= mine) last.cell = cell_num;
+    given++;
+    return last;
+  }
+};
+
+// The empty-row pieces of a dense dispatch in such a grid: every CTA zeroes an even, consecutive
+// share, its warps in turn, a few pieces for every move item so that the zeros mix with the row
+// traffic.  A warp's pieces only move forward, and so does the path they have reached.
+template <int VB>
+struct WarpFill {
+  int64_t next, end;
+  int per_turn, path;
+  __device__ __forceinline__ WarpFill(int64_t fill_items, int turns) {
+    const int64_t per = (fill_items + gridDim.x - 1) / gridDim.x;
+    next = per * blockIdx.x + (threadIdx.x >> 5);
+    end = min(per * (blockIdx.x + 1), fill_items);
+    per_turn = (int)((per + kWarps * turns - 1) / (kWarps * turns));
+    path = 0;
+  }
+  __device__ __forceinline__ void run(const MoveArgs& a, int count, const int* s_base,
+                                      const int* s_written, const int* s_fill, int lane) {
+    using V = typename Chunk<VB>::type;
+    for (; count > 0 && next < end; count--, next += kWarps) {
+      int64_t nth = next;
+      int piece = 0;
+      if (a.pieces_per_row != 1) {
+        nth = next / a.pieces_per_row;
+        piece = (int)(next - nth * a.pieces_per_row);
+      }
+      if (path == 0) {  // the first time: last path whose first empty row is <= nth
+        int lo = 0, hi = a.path_num - 1;
+        while (lo < hi) {
+          const int mid = (lo + hi + 1) >> 1;
+          if ((int64_t)s_fill[mid] <= nth) lo = mid; else hi = mid - 1;
+        }
+        path = lo;
+      }
+      while (path + 1 < a.path_num && (int64_t)s_fill[path + 1] <= nth) path++;
+      const int64_t row = (int64_t)s_base[path] + s_written[path] + (nth - s_fill[path]);
+      V* dp = static_cast<V*>(a.dst) + row * a.row_vecs;
+      const V zero = zero_chunk<V>();
+      const int64_t v0 = (int64_t)piece * kPieceVecs + lane;
+#pragma unroll
+      for (int u = 0; u < kCopyUnroll; u++) {
+        const int64_t v = v0 + u * 32;
+        if (v < a.row_vecs) store_stream(dp + v, zero);
+      }
+      if (piece == 0 && lane == 0 && a.new_tags != nullptr) a.new_tags[row] = 0;
+    }
+  }
+};
 
 // A warp's share of the empty-row pieces, spread evenly between its move items so that the
 // writes of zeros mix with the row traffic instead of trailing it.

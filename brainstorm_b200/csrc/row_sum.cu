@@ -245,7 +245,9 @@ void launch_row_sum(int vb, const void* const* rows, void* out, const int* seg,
                     int64_t rows_out, int64_t row_bytes, cudaStream_t st) {
   const int64_t row_vecs = row_bytes / vb;
   int64_t blocks = (rows_out * row_vecs + kThreads - 1) / kThreads;
-  const int64_t cap = (int64_t)sm_count() * 16;
+  // one piece per thread, CTAs in launch order: 64 x 3 MiB from 270 rows 158 us, 167 with resident
+  // CTAs that stride (DRAM likes the narrow window of CTAs launched in order)
+  const int64_t cap = 0x7fffffff;
   if (blocks > cap) blocks = cap;
   if (blocks < 1) blocks = 1;
   const KernelTimer timer("row_sum_kernel", st);
