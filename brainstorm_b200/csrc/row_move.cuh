@@ -13,6 +13,12 @@ constexpr int kWarps = kThreads / 32;
 constexpr int kMaxPaths = 4096;
 constexpr int kPieceVecs = 128;    // vectors per dispatch item (2 KB at 16 bytes)
 constexpr int kCopyUnroll = kPieceVecs / 32;
+// Vectors per lane of an item when a row cannot be moved 16 bytes at a time: still 2 KB (1 KB in
+// 2-byte steps), so that a row of 2004 bytes is one item with 16 loads per lane in flight and
+// one walk of its index row, not four of each.
+constexpr int unroll_of(int vec_bytes) {
+  return vec_bytes == 16 ? kCopyUnroll : vec_bytes == 8 ? 8 : 16;
+}
 constexpr int kMaxRoutes = 2;      // routes per combine item staged in shared memory (the
                                    // fold below is written out for exactly two)
 constexpr int kFoldVecs = 128;     // vectors per combine item (2 KB at 16 bytes)
@@ -77,37 +83,12 @@ __device__ __forceinline__ void load_gate_chunk(const void* __restrict__ gates, 
   }
 }
 
-// s_loads[e], s_base[e] for every path; called by all threads of the CTA.
-__device__ __forceinline__ void setup_paths(const int* __restrict__ loads, int path_num,
-                                            int max_path_load, int* s_loads, int* s_base) {
-  if (threadIdx.x < 32) {
-    const int lane = threadIdx.x;
-    int carry = 0;
-    for (int p = 0; p < path_num; p += 32) {
-      const int e = p + lane;
-      const int v = e < path_num ? loads[e] : 0;
-      int incl = v;
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const int n = __shfl_up_sync(0xffffffffu, incl, d);
-        if (lane >= d) incl += n;
-      }
-      if (e < path_num) {
-        s_loads[e] = v;
-        s_base[e] = max_path_load != 0 ? e * max_path_load : carry + incl - v;
-      }
-      carry += __shfl_sync(0xffffffffu, incl, 31);
-    }
-  }
-  __syncthreads();
-}
-
 // Dense seat columns (what the index kernels write): column e holds every seat
 // 1 .. counts[e] exactly once, so the rows of path e that receive a cell are exactly the first
 // min(counts[e], loads[e]) of its slot and the rest of the slot is known to stay empty
 // without looking at the indices.  s_written[e] = rows of path e that get a cell,
 // s_fill[e] = exclusive prefix of the empty rows per path (s_fill[path_num] = their total).
-// Called by all threads of the CTA after setup_paths.
+// Called by all threads of the CTA once s_loads is there.
 __device__ __forceinline__ void setup_fill(const int* __restrict__ counts, int path_num,
                                            int max_path_load, const int* s_loads,
                                            int* s_written, int* s_fill) {
@@ -403,32 +384,6 @@ __device__ __forceinline__ int record_routes(uint2 mine, const int* s_loads, con
   return __popc(kept);
 }
 
-// Zero one (empty row, 2 KB piece) of a dense dispatch; `item` counts the pieces of the empty
-// rows in path order.  Called by a whole warp.
-template <int VB>
-__device__ __forceinline__ void fill_item(const MoveArgs& a, const int* s_base,
-                                          const int* s_written, const int* s_fill, int64_t item,
-                                          int lane) {
-  using V = typename Chunk<VB>::type;
-  const int64_t nth = item / a.pieces_per_row;
-  const int piece = (int)(item - nth * a.pieces_per_row);
-  int lo = 0, hi = a.path_num - 1;  // last path whose first empty row is <= nth
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if ((int64_t)s_fill[mid] <= nth) lo = mid; else hi = mid - 1;
-  }
-  const int64_t row = (int64_t)s_base[lo] + s_written[lo] + (nth - s_fill[lo]);
-  V* dp = static_cast<V*>(a.dst) + row * a.row_vecs;
-  const V zero = zero_chunk<V>();
-  const int64_t v0 = (int64_t)piece * kPieceVecs + lane;
-#pragma unroll
-  for (int u = 0; u < kCopyUnroll; u++) {
-    const int64_t v = v0 + u * 32;
-    if (v < a.row_vecs) store_stream(dp + v, zero);
-  }
-  if (piece == 0 && lane == 0 && a.new_tags != nullptr) a.new_tags[row] = 0;
-}
-
 // The items of a warp in a grid whose CTAs own kWarps * turns consecutive ones each, in order:
 // the CTA's first + warp, + kWarps, ...  A cursor past the last one has cell == cell_num.
 struct WarpItems {
@@ -460,6 +415,7 @@ struct WarpItems {
 // traffic.  A warp's pieces only move forward, and so does the path they have reached.
 template <int VB>
 struct WarpFill {
+  static constexpr int U = unroll_of(VB);
   int64_t next, end;
   int per_turn, path;
   __device__ __forceinline__ WarpFill(int64_t fill_items, int turns) {
@@ -491,9 +447,9 @@ struct WarpFill {
       const int64_t row = (int64_t)s_base[path] + s_written[path] + (nth - s_fill[path]);
       V* dp = static_cast<V*>(a.dst) + row * a.row_vecs;
       const V zero = zero_chunk<V>();
-      const int64_t v0 = (int64_t)piece * kPieceVecs + lane;
+      const int64_t v0 = (int64_t)piece * (32 * U) + lane;
 #pragma unroll
-      for (int u = 0; u < kCopyUnroll; u++) {
+      for (int u = 0; u < U; u++) {
         const int64_t v = v0 + u * 32;
         if (v < a.row_vecs) store_stream(dp + v, zero);
       }
