@@ -39,10 +39,9 @@ using namespace rows;
 
 
 // ---------------------------------------------------------------------------------- dispatch
-template <int VB, int DT, bool WEIGHTED, bool IS_1D, int IV>
+template <int VB, int DT, bool WEIGHTED, bool IS_1D, int IV, int U>
 __global__ void __launch_bounds__(kThreads, 4) dispatch_seat_kernel(const MoveArgs a) {
   using V = typename Chunk<VB>::type;
-  constexpr int U = unroll_of(VB);
   constexpr int GK = WEIGHTED ? 2 : 0;
   extern __shared__ int s_mem[];
   int* s_loads = s_mem;
@@ -64,7 +63,7 @@ __global__ void __launch_bounds__(kThreads, 4) dispatch_seat_kernel(const MoveAr
   setup_tables(a.loads, a.dense_counts, a.path_num, a.max_path_load, s_loads, s_base, s_written,
                s_fill);
   const bool dense = a.dense_counts != nullptr;
-  WarpFill<VB> fill(dense ? (int64_t)s_fill[E] * a.pieces_per_row : 0, a.turns);
+  WarpFill<VB, U> fill(dense ? (int64_t)s_fill[E] * a.pieces_per_row : 0, a.turns);
   while (at.cell < a.cell_num) {
     int nxt[IV];
 #pragma unroll
@@ -76,6 +75,7 @@ __global__ void __launch_bounds__(kThreads, 4) dispatch_seat_kernel(const MoveAr
     const int64_t v0 = (int64_t)piece * (32 * U) + lane;
     const int left = (int)min(a.row_vecs - (int64_t)piece * (32 * U), (int64_t)(32 * U));
     const int live = (left + 31) >> 5;  // rounds of this piece that hold anything
+    constexpr int kRounds = U == kCopyUnroll ? 1 : 4;  // looked at so many at a time
     V regs[U];
     bool loaded = false;
     for (int c = 0; c < chunks; c++) {
@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(kThreads, 4) dispatch_seat_kernel(const MoveAr
               const V* sp = src + src_row * a.row_vecs;
 #pragma unroll
               for (int u = 0; u < U; u++) {
-                if (u % 4 == 0 && u >= live) break;
+                if (u % kRounds == 0 && u >= live) break;
                 if (u * 32 + lane < left) regs[u] = load_stream(sp + v0 + u * 32);
               }
               loaded = true;
@@ -126,14 +126,14 @@ __global__ void __launch_bounds__(kThreads, 4) dispatch_seat_kernel(const MoveAr
               const float g = __shfl_sync(0xffffffffu, gate[j], l);
 #pragma unroll
               for (int u = 0; u < U; u++) {
-                if (u % 4 == 0 && u >= live) break;
+                if (u % kRounds == 0 && u >= live) break;
                 if (u * 32 + lane < left)
                   store_stream(dp + v0 + u * 32, scale_chunk<VB, DT>(regs[u], g));
               }
             } else {
 #pragma unroll
               for (int u = 0; u < U; u++) {
-                if (u % 4 == 0 && u >= live) break;
+                if (u % kRounds == 0 && u >= live) break;
                 if (u * 32 + lane < left) store_stream(dp + v0 + u * 32, regs[u]);
               }
             }
@@ -569,7 +569,7 @@ __global__ void __launch_bounds__(kThreads, WEIGHTED ? 3 : 4) dispatch_seat_asyn
   setup_tables(a.loads, a.dense_counts, a.path_num, a.max_path_load, s_loads, s_base, s_written,
                s_fill);
   const bool dense = a.dense_counts != nullptr;
-  WarpFill<VB> fill(dense ? (int64_t)s_fill[E] * a.pieces_per_row : 0, a.turns);
+  WarpFill<VB, kCopyUnroll> fill(dense ? (int64_t)s_fill[E] * a.pieces_per_row : 0, a.turns);
   issue(my[0], at);
   fetch(ahead);
   while (at.cell < a.cell_num) {
@@ -652,11 +652,10 @@ __global__ void __launch_bounds__(kThreads, WEIGHTED ? 3 : 4) dispatch_seat_asyn
 // Register-only combine for rows that cannot be moved 16 bytes at a time.  (9001 rows of 2004
 // bytes, 2 of 30 paths: 14.0 -> 11.1 us, and the dispatch of the same rows 19.0 -> 11.5, both
 // against items of 512 bytes, one load per lane at a time.)
-template <int VB, int DT, int GMODE>
+template <int VB, int DT, int GMODE, int U>
 __global__ void __launch_bounds__(kThreads) combine_seat_kernel(const MoveArgs a) {
   using L = Lanes<VB, DT>;
   using V = typename L::V;
-  constexpr int U = unroll_of(VB);
   extern __shared__ int s_mem[];
   int* s_loads = s_mem;
   int* s_base = s_mem + a.path_num;
@@ -676,6 +675,7 @@ __global__ void __launch_bounds__(kThreads) combine_seat_kernel(const MoveArgs a
     const int64_t v0 = piece * (32 * U) + lane;
     const int left = (int)min(a.row_vecs - piece * (32 * U), (int64_t)(32 * U));
     const int live = (left + 31) >> 5;  // rounds of this piece that hold anything
+    constexpr int kRounds = U == kCopyUnroll ? 1 : 4;  // looked at so many at a time
     float acc[U][L::N];
 #pragma unroll
     for (int u = 0; u < U; u++)
@@ -699,12 +699,12 @@ __global__ void __launch_bounds__(kThreads) combine_seat_kernel(const MoveArgs a
         V row[U];
 #pragma unroll
         for (int u = 0; u < U; u++) {
-          if (u % 4 == 0 && u >= live) break;
+          if (u % kRounds == 0 && u >= live) break;
           row[u] = u * 32 + lane < left ? load_stream(sp + u * 32) : zero_chunk<V>();
         }
 #pragma unroll
         for (int u = 0; u < U; u++) {
-          if (u % 4 == 0 && u >= live) break;
+          if (u % kRounds == 0 && u >= live) break;
           fold_chunk<VB, DT, GMODE>(acc[u], row[u], g);
         }
         routed = true;
@@ -713,7 +713,7 @@ __global__ void __launch_bounds__(kThreads) combine_seat_kernel(const MoveArgs a
     if (routed || !a.is_residual) {
 #pragma unroll
       for (int u = 0; u < U; u++) {
-        if (u % 4 == 0 && u >= live) break;
+        if (u % kRounds == 0 && u >= live) break;
         if (u * 32 + lane < left)
           store_stream(dst + cell * a.row_vecs + v0 + u * 32, pack_chunk<VB, DT>(acc[u]));
       }
@@ -794,22 +794,40 @@ unsigned grid_for_resident(int64_t items, int ctas_per_sm) {
 // window narrow.  Measured, striding / 2 / 4 / 8 items per warp: 65536 x 64 packed rows of 4 KB
 // 147 / 129 / 133 / 136 us; 64 samples of 3 MiB 185 / 166 / 171 / 185; with capacity padding, where
 // a turn is mostly zero rows, 262144 x 128 181 / 173 / 145 / 150 and 32768 x 32 36.4 / 35.6 / 35.0 /
-// 35.0.  So 2 for packed rows, 4 with slots of a fixed size; when that leaves SMs idle although
-// there are rows to zero, the items are spread over one resident wave.
+// 35.0.  So 2 for packed rows, 4 with slots of a fixed size, and more when an item is less than 2 KB.
+// A grid of a few waves takes the count near that which leaves the last wave fullest (20000 rows of
+// 4000 bytes, 32 slots: 4 items make 2.1 waves, 34.9 us; 8 make 1.06, 38.5; 5 make 2.8, 32.5).  When SMs would stay
+// idle although there are rows to move or to zero, the items are spread over one resident wave.
 // (The combine was measured in the same way and keeps its resident CTAs: 26 / 33 / 31 / 33 us at
 // 32768 x 32, 92 / 157 / 127 / 115 at 262144 x 128: its three CTAs per SM have little beside them
 // to cover a start, and it reads more than it writes.)
 unsigned plan_dispatch(MoveArgs& a, int ctas_per_sm) {
   const int64_t items = a.cell_num * a.pieces_per_row;
   const int64_t fills = a.dense_counts != nullptr ? a.total_rows * a.pieces_per_row : 0;
-  a.turns = a.max_path_load != 0 ? 4 : 2;
-  int64_t ctas = (items + kWarps * a.turns - 1) / (kWarps * a.turns);
   const int64_t resident = (int64_t)sm_count() * ctas_per_sm;
+  const int64_t item_bytes = std::min<int64_t>(a.row_bytes, 2048);
+  const int64_t scale = std::min<int64_t>(2048 / item_bytes, 32);
+  const int64_t usual = (a.max_path_load != 0 ? 4 : 2) * scale;
+  auto ctas_for = [&](int64_t turns) { return (items + kWarps * turns - 1) / (kWarps * turns); };
+  int64_t turns = usual, ctas = ctas_for(usual);
+  if (ctas < 8 * resident) {
+    double fullest = 0;
+    for (int64_t t = std::max<int64_t>(usual * 3 / 4, 2); t <= usual * 2; t++) {
+      const int64_t waves = (ctas_for(t) + resident - 1) / resident;
+      const double full = (double)items / ((double)waves * resident * kWarps * t);
+      if (full > fullest * 1.02) {
+        fullest = full;
+        turns = t;
+      }
+    }
+    ctas = ctas_for(turns);
+  }
   const int64_t useful = std::min((std::max(items, fills) + kWarps - 1) / kWarps, resident);
   if (ctas < useful) {
     ctas = useful;
-    a.turns = (int)std::max((items + ctas * kWarps - 1) / (ctas * kWarps), (int64_t)1);
+    turns = std::max((items + ctas * kWarps - 1) / (ctas * kWarps), (int64_t)1);
   }
+  a.turns = (int)turns;
   return (unsigned)std::max(ctas, (int64_t)1);
 }
 
@@ -864,10 +882,20 @@ void launch_dispatch(const MoveArgs& a, bool is_tag, cudaStream_t st) {
   } else {
     MoveArgs b = a;
     const unsigned grid = plan_dispatch(b, 4);
-    if (wide_rows(a.indices, a.gates, dtype_size(DT), a.path_num))
-      dispatch_seat_kernel<VB, DT, WEIGHTED, IS_1D, 4><<<grid, kThreads, smem, st>>>(b), note_launch();
-    else
-      dispatch_seat_kernel<VB, DT, WEIGHTED, IS_1D, 1><<<grid, kThreads, smem, st>>>(b), note_launch();
+    const bool wide = wide_rows(a.indices, a.gates, dtype_size(DT), a.path_num);
+    constexpr int U = unroll_of(VB);
+    if (U != kCopyUnroll && a.row_vecs <= kShortRow) {
+      if (wide)
+        dispatch_seat_kernel<VB, DT, WEIGHTED, IS_1D, 4, kCopyUnroll>
+            <<<grid, kThreads, smem, st>>>(b), note_launch();
+      else
+        dispatch_seat_kernel<VB, DT, WEIGHTED, IS_1D, 1, kCopyUnroll>
+            <<<grid, kThreads, smem, st>>>(b), note_launch();
+    } else if (wide) {
+      dispatch_seat_kernel<VB, DT, WEIGHTED, IS_1D, 4, U><<<grid, kThreads, smem, st>>>(b), note_launch();
+    } else {
+      dispatch_seat_kernel<VB, DT, WEIGHTED, IS_1D, 1, U><<<grid, kThreads, smem, st>>>(b), note_launch();
+    }
   }
 }
 
@@ -934,8 +962,11 @@ int launch_combine(const MoveArgs& a, cudaStream_t st) {
   } else {
     const size_t smem = (size_t)a.path_num * 2 * sizeof(int);
     const KernelTimer timer("combine_kernel", st);
-    combine_seat_kernel<VB, DT, GMODE>
-        <<<grid_for_items(a.cell_num * a.pieces_per_row), kThreads, smem, st>>>(a), note_launch();
+    const unsigned grid = grid_for_items(a.cell_num * a.pieces_per_row);
+    if (a.row_vecs <= kShortRow)
+      combine_seat_kernel<VB, DT, GMODE, kCopyUnroll><<<grid, kThreads, smem, st>>>(a), note_launch();
+    else
+      combine_seat_kernel<VB, DT, GMODE, unroll_of(VB)><<<grid, kThreads, smem, st>>>(a), note_launch();
     return BRT_OK;
   }
 }
@@ -1031,6 +1062,7 @@ BRT_API int brt_dispatch_with_records(
   a.loads_evict_first = dispatch_loads_evict_first() ? 1 : 0;
   a.newest_first = 0;
   a.cell_num = cell_num;
+  a.row_bytes = row_bytes;
   a.row_vecs = row_bytes / vb;
   a.pieces_per_row = (a.row_vecs + 32 * unroll_of(vb) - 1) / (32 * unroll_of(vb));
   a.path_num = path_num;
@@ -1117,6 +1149,7 @@ BRT_API int brt_combine_with_records(
   a.loads_evict_first = 0;
   a.newest_first = combine_newest_first() ? 1 : 0;
   a.cell_num = cell_num;
+  a.row_bytes = row_bytes;
   a.row_vecs = row_bytes / vb;
   a.pieces_per_row = (a.row_vecs + 32 * unroll_of(vb) - 1) / (32 * unroll_of(vb));
   a.path_num = path_num;

@@ -19,6 +19,9 @@ constexpr int kCopyUnroll = kPieceVecs / 32;
 constexpr int unroll_of(int vec_bytes) {
   return vec_bytes == 16 ? kCopyUnroll : vec_bytes == 8 ? 8 : 16;
 }
+// Rows of at most this many vectors take the variants with kCopyUnroll rounds (one piece either
+// way; 16 rounds that mostly hold nothing cost rows of 36 and 72 bytes a third of their time).
+constexpr int kShortRow = 32 * kCopyUnroll;
 constexpr int kMaxRoutes = 2;      // routes per combine item staged in shared memory (the
                                    // fold below is written out for exactly two)
 constexpr int kFoldVecs = 128;     // vectors per combine item (2 KB at 16 bytes)
@@ -279,6 +282,7 @@ struct MoveArgs {
   int path_num;
   int max_path_load;
   int64_t total_rows;  // dispatch: output rows
+  int64_t row_bytes = 0;
   int turns = 0;       // pipelined dispatch: items per warp; a CTA owns kWarps * turns of them
   int is_residual;     // combine only
 };
@@ -413,9 +417,8 @@ struct WarpItems {
 // The empty-row pieces of a dense dispatch in such a grid: every CTA zeroes an even, consecutive
 // share, its warps in turn, a few pieces for every move item so that the zeros mix with the row
 // traffic.  A warp's pieces only move forward, and so does the path they have reached.
-template <int VB>
+template <int VB, int U>
 struct WarpFill {
-  static constexpr int U = unroll_of(VB);
   int64_t next, end;
   int per_turn, path;
   __device__ __forceinline__ WarpFill(int64_t fill_items, int turns) {
