@@ -101,26 +101,35 @@ def _new_records(cells: int, paths: int, device) -> Optional[torch.Tensor]:
 
 
 def _mark_records(indices: torch.Tensor, records: Optional[torch.Tensor]) -> None:
-    """Remember on the tensor itself the route records that came with ``indices``, and the
-    tensor's version: an edit in place (of it or of a view) makes the note void.  Inference
-    tensors do not count their edits, so they get no note."""
+    """Remember on the tensor itself the route records that came with ``indices``, with the
+    tensor's version (an edit in place, of it or of a view, makes the note void), its memory,
+    the stream and the capture they were made in.  Inference tensors do not count their
+    edits, so they get no note."""
     if records is not None and not indices.is_inference():
-        setattr(indices, _RECORDS, (records, indices._version,
-                                    _lib.raw_stream(indices.device)))
+        stream = _lib.raw_stream(indices.device)
+        setattr(indices, _RECORDS, (records, indices._version, stream, indices.data_ptr(),
+                                    _lib.query("brt_stream_capture_id", stream)))
 
 
 def _records_of(indices: torch.Tensor, cells: int, paths: int) -> Optional[torch.Tensor]:
-    """The route records of ``indices`` as long as they describe it.  The caller of a stream
-    they were not made on only vouches for ``indices``; their memory is held for it here."""
+    """The route records of ``indices`` as long as they describe it.  A launch that is captured
+    takes them from its own capture only, and one that is not takes none of a capture: a
+    replay finds in the tensor what was copied there since, which the records would not show.
+    The caller of a stream they were not made on only vouches for ``indices``; their memory
+    is held for it here."""
     note = getattr(indices, _RECORDS, None)
     if note is None or not _USE_DENSE or getattr(indices, _DENSE, None) is None:
         return None
-    records, version, stream = note
-    if indices._version != version or records.device != indices.device or \
+    records, version, stream, address, capture = note
+    if indices._version != version or indices.data_ptr() != address or \
+            records.device != indices.device or \
             indices.size(0) != cells or indices.size(1) != paths or \
             records.numel() != cells * 8:
         return None
-    if _lib.raw_stream(indices.device) != stream:
+    here = _lib.raw_stream(indices.device)
+    if _lib.query("brt_stream_capture_id", here) != capture:
+        return None
+    if here != stream:
         records.record_stream(torch.cuda.current_stream(indices.device))
     return records
 

@@ -30,6 +30,7 @@ SIGNATURES = {
     "brt_generate_indices_and_loads": (
         _int, [_vp, _vp, _vp, _vp, _i64, _int, _vp, _int, _int, _int, _int, _vp, _sz, _vp]),
     "brt_route_record_bytes": (_sz, [_i64, _int]),
+    "brt_stream_capture_id": (ctypes.c_uint64, [_vp]),
     "brt_generate_indices_loads_records": (
         _int, [_vp, _vp, _vp, _vp, _vp, _i64, _int, _vp, _int, _int, _int, _int, _vp, _sz, _vp]),
     "brt_throttle_and_generate_records": (

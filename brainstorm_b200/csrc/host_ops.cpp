@@ -66,6 +66,10 @@ bool same_device(const at::Tensor& a, const at::Tensor* b) {
   return b == nullptr || a.get_device() == b->get_device();
 }
 
+unsigned long long address(const void* p) {
+  return (unsigned long long)reinterpret_cast<uintptr_t>(p);
+}
+
 // The notes of an index operator on the tensor it returns, see _C/router.py.
 bool mark(PyObject* indices, const at::Tensor& counts, const at::Tensor& records,
           const Place& at_place) {
@@ -77,10 +81,10 @@ bool mark(PyObject* indices, const at::Tensor& counts, const at::Tensor& records
   Py_DECREF(c);
   const at::Tensor& t = THPVariable_Unpack(indices);
   if (!records.defined() || t.is_inference()) return true;
-  PyObject* note = Py_BuildValue("(NKK)", THPVariable_Wrap(records),
-                                 (unsigned long long)t._version(),
-                                 (unsigned long long)reinterpret_cast<uintptr_t>(
-                                     at_place.handle()));
+  PyObject* note = Py_BuildValue(
+      "(NKKKK)", THPVariable_Wrap(records), (unsigned long long)t._version(),
+      address(at_place.handle()), address(t.data_ptr()),
+      (unsigned long long)brt_stream_capture_id(at_place.handle()));
   const bool ok = note != nullptr && PyObject_SetAttr(indices, g_records, note) == 0;
   Py_XDECREF(note);
   return ok;
@@ -104,21 +108,24 @@ const int32_t* dense_counts(PyObject* indices, int64_t paths) {
   return p;
 }
 // The route records noted on `indices`: false when a note is there that needs the slow road
-// (another stream); *out null when there is none or it no longer holds.
+// (another stream); *out null when there is none, it no longer holds or it is of another capture.
 bool route_records(PyObject* indices, int64_t cells, const Place& at_place, const void** out) {
   *out = nullptr;
   PyObject* note = attribute(indices, g_records);
   if (note == nullptr) return true;
   bool usable = true;
   const at::Tensor& t = THPVariable_Unpack(indices);
-  if (PyTuple_Check(note) && PyTuple_GET_SIZE(note) == 3) {
+  if (PyTuple_Check(note) && PyTuple_GET_SIZE(note) == 5) {
     const at::Tensor* records = plain(PyTuple_GET_ITEM(note, 0));
     const unsigned long long version = PyLong_AsUnsignedLongLong(PyTuple_GET_ITEM(note, 1));
     const unsigned long long stream = PyLong_AsUnsignedLongLong(PyTuple_GET_ITEM(note, 2));
+    const unsigned long long memory = PyLong_AsUnsignedLongLong(PyTuple_GET_ITEM(note, 3));
+    const unsigned long long capture = PyLong_AsUnsignedLongLong(PyTuple_GET_ITEM(note, 4));
     if (PyErr_Occurred()) PyErr_Clear();
     if (int32c(records, 1) && !t.is_inference() && version == t._version() &&
-        records->numel() == cells * 8 && same_device(t, records)) {
-      usable = stream == (unsigned long long)reinterpret_cast<uintptr_t>(at_place.handle());
+        memory == address(t.data_ptr()) && records->numel() == cells * 8 &&
+        same_device(t, records) && capture == brt_stream_capture_id(at_place.handle())) {
+      usable = stream == address(at_place.handle());
       if (usable) *out = records->data_ptr();
     }
   }

@@ -2148,6 +2148,17 @@ BRT_API size_t brt_route_record_bytes(int64_t cell_num, int path_num) {
   return (size_t)cell_num * kRecordRoutes * 8;
 }
 
+BRT_API uint64_t brt_stream_capture_id(void* stream) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  if (cudaStreamGetCaptureInfo(static_cast<cudaStream_t>(stream), &status, &id) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return UINT64_MAX;
+  }
+  if (status == cudaStreamCaptureStatusNone) return 0;
+  return status == cudaStreamCaptureStatusActive ? (uint64_t)id : UINT64_MAX;
+}
+
 BRT_API int brt_generate_indices_and_loads(const int32_t* hot_mask, int32_t* indices,
                                            int32_t* loads, int32_t* path_counts,
                                            int64_t cell_num, int path_num,

@@ -104,9 +104,14 @@ BRT_API int brt_generate_indices_and_loads(const int32_t* hot_mask, int32_t* ind
  *                          to 16 paths, where the index row is hardly longer, over 256, or a
  *                          mask that is too large for the single-launch scan): pass no
  *                          records then
+ * brt_stream_capture_id    the id of the capture that `stream` takes part in, 0 when there is
+ *                          none, UINT64_MAX when it cannot be told.  Records belong to the capture
+ *                          they were made in: a graph that reads records made outside
+ *                          it would not see an index tensor edited between two replays
  * The entry points are those without `records` in their names plus that argument (may be null).
  */
 BRT_API size_t brt_route_record_bytes(int64_t cell_num, int path_num);
+BRT_API uint64_t brt_stream_capture_id(void* stream);
 BRT_API int brt_generate_indices_loads_records(
     const int32_t* hot_mask, int32_t* indices, int32_t* loads, int32_t* path_counts,
     void* route_records, int64_t cell_num, int path_num, const int32_t* supported_capacities,

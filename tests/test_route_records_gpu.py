@@ -102,3 +102,41 @@ def test_records_used_on_another_stream_outlive_their_tensor():
     junk = [torch.full((65536 * 8,), -1, dtype=torch.int32, device="cuda") for _ in range(8)]
     side.synchronize()
     assert torch.equal(got, want) and len(junk) == 8
+
+
+def test_a_graph_does_not_keep_records_of_indices_made_before_it():
+    from brainstorm_b200._C import router as R
+
+    indices, loads = make(R, 65536, 32, [0.05], 11, None)
+    later, later_loads = make(R, 65536, 32, [0.05], 12, None)
+    assert R._records_of(indices, 65536, 32) is not None
+    rows = torch.randn((int(later_loads.max()) * 2 * 32, 8), device="cuda")
+
+    def run(at, n):
+        return R.combine_with_indices_and_loads(rows, at, n, None, None, True)[0]
+
+    run(indices, loads)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = run(indices, loads)
+        inside, _ = R.generate_indices_and_loads((indices > 0).to(torch.int32))
+        assert R._records_of(inside, 65536, 32) is not None
+    assert R._records_of(inside, 65536, 32) is None
+    indices.copy_(later)
+    loads.copy_(later_loads)
+    graph.replay()
+    assert torch.equal(out, run(later, later_loads))
+
+
+def test_notes_do_not_follow_a_tensor_to_other_memory():
+    from brainstorm_b200._C import router as R
+
+    indices, loads = make(R, 65536, 32, [0.05], 13, None)
+    later, _ = make(R, 65536, 32, [0.05], 14, None)
+    indices.data = later.clone()
+    assert R._records_of(indices, 65536, 32) is None
+    rows = torch.randn((65536 * 4, 8), device="cuda")
+    (a,) = R.combine_with_indices_and_loads(rows, indices, loads, None, None, True)
+    (b,) = R.combine_with_indices_and_loads(rows, indices.clone(), loads, None, None, True)
+    assert torch.equal(a, b)
