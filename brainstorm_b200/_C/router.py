@@ -451,8 +451,8 @@ def _dispatch(in_data, route_indices, loads, gates, tag_generating, tags, max_pa
             in_data.size(0) > 0:
         if not max_path_padding:
             if host_loads is None:
-                host_loads = loads.tolist()
-            slot, total = 0, sum(host_loads)
+                host_loads = loads.reshape(-1).tolist()
+            slot, total = 0, int(sum(host_loads))
         else:
             slot, total = max_path_load, max_path_load * route_indices.size(1)
         if slot > 0 or not max_path_padding:
@@ -493,7 +493,7 @@ def _dispatch(in_data, route_indices, loads, gates, tag_generating, tags, max_pa
         else:
             mpl = 0
             # the loads themselves cross over: a sum on the device takes two launches first
-            total = sum(loads.tolist() if host_loads is None else host_loads)
+            total = int(sum(loads.reshape(-1).tolist() if host_loads is None else host_loads))
         shape = list(in_data.shape)
         if is_1d_routing:
             shape[0] = total

@@ -155,3 +155,16 @@ def test_residual_is_returned_itself_and_notes_travel():
     base = torch.randn((65536, 8), device="cuda")
     (out,) = R.combine_with_indices_and_loads(rows, indices, loads, None, base)
     assert out is base
+
+
+@pytest.mark.parametrize("paths", [1, 30])
+def test_packed_dispatch_takes_loads_of_any_shape(paths):
+    from brainstorm_b200._C import router as R
+
+    indices, loads = R.generate_indices_and_loads(masks(500, paths)["plain"])
+    x = torch.randn((500, 64), device="cuda")
+    (want,) = R.dispatch_with_indices_and_loads(x, indices, loads)
+    shapes = [(1, paths), (paths, 1)] + ([()] if paths == 1 else [])
+    for shape in shapes:
+        (got,) = R.dispatch_with_indices_and_loads(x, indices, loads.reshape(shape))
+        assert torch.equal(got, want)
