@@ -1499,7 +1499,8 @@ __device__ __forceinline__ void write_routes(const ChainArgs& c, const TileCtx& 
       const int v = value_of<MODE>(seat, kLimited ? thr[col] : 0);
       if (v == 0) continue;
       if constexpr (MODE == Mode::kTag) {
-        if (seat <= x.cell_num)
+        // earlier runs may hold any int32: their sum, and with it the seat, may lie below 1
+        if (seat >= 1 && seat <= x.cell_num)
           c.t.out[(int64_t)(seat - 1) * x.path_num + (int64_t)x.chunk * x.ec + col] =
               (int)(row + 1);
       } else if (scatter) {

@@ -66,6 +66,29 @@ def test_scan_edges(cells, paths, kind):
         assert np.array_equal(prefix.cpu().numpy(), start_np)
 
 
+@pytest.mark.parametrize("paths", [5, 30, 32, 256, 260])
+@pytest.mark.parametrize("first", [-50, -9001, -46340])
+def test_tags_after_a_run_with_a_negative_sum(paths, first):
+    """A first run that sums to less than zero starts the 0/1 runs after it below seat 1: a cell
+    whose seat is not a row of the output goes nowhere."""
+    from brainstorm_b200._C import router as R
+
+    cells = 9001
+    rng = np.random.default_rng(paths)
+    mask = (rng.random((cells, paths)) < 0.1).astype(np.int32)
+    mask[0] = 0
+    mask[0, ::2] = first  # index first * first, past the rows that the later seats name
+    seat = np.cumsum(mask, axis=0, dtype=np.int64) * mask
+    assert first * first > seat[1:].max() and seat.min() < 0
+    want = np.zeros_like(mask)
+    cell, path = np.nonzero((seat >= 1) & (seat <= cells))
+    want[seat[cell, path] - 1, path] = cell + 1
+    dev = torch.from_numpy(mask).cuda()
+    got, loads = R.generate_indices_and_loads(dev, None, False, False, True)
+    assert np.array_equal(got.cpu().numpy(), want)
+    assert np.array_equal(loads.cpu().numpy(), mask.sum(axis=0))
+
+
 def test_scan_of_an_array_that_is_only_4_byte_aligned():
     from brainstorm_b200._C import router as R
 
