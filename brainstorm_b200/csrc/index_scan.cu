@@ -1160,13 +1160,24 @@ __device__ __forceinline__ void gate_words(const TileCtx& x, int* stage, int* bi
     const int64_t left = x.cell_num - row0;
     const int rows = left < x.rg * kGroupRows ? (int)left : x.rg * kGroupRows;
     const int total = rows * vec_per_row;
-    int4* const out = reinterpret_cast<int4*>(g.gates_out + row0 * x.path_num);
+    int* const out = reinterpret_cast<int*>(g.gates_out + row0 * x.path_num);
+    // the entry point takes gates at any float's alignment; rows are multiples of 16 bytes, so
+    // the first element decides for all of them
+    const bool wide = (reinterpret_cast<uintptr_t>(g.gates_out) & 15u) == 0;
     const int step_r = kTileThreads / vec_per_row;
     const int step_q = kTileThreads - step_r * vec_per_row;
     int r = threadIdx.x / vec_per_row;
     int q = threadIdx.x - r * vec_per_row;
     for (int i = threadIdx.x; i < total; i += kTileThreads) {
-      __stcs(out + i, *reinterpret_cast<const int4*>(stage + r * x.pitch + 4 * q));
+      const int4 four = *reinterpret_cast<const int4*>(stage + r * x.pitch + 4 * q);
+      if (wide) {
+        __stcs(reinterpret_cast<int4*>(out) + i, four);
+      } else {
+        __stcs(out + 4 * i, four.x);
+        __stcs(out + 4 * i + 1, four.y);
+        __stcs(out + 4 * i + 2, four.z);
+        __stcs(out + 4 * i + 3, four.w);
+      }
       r += step_r;
       q += step_q;
       if (q >= vec_per_row) { q -= vec_per_row; r += 1; }

@@ -275,14 +275,15 @@ typedef enum brt_route_output {
  *            brt_generate_indices_and_loads (the two SEAT_INDICES outputs); prefix and
  *            throttle_capacity as in brt_throttle_hotmask (the two THROTTLED outputs)
  *   gates_out optional fp32 [cell_num, path_num]: picked scores divided by their sum
- *            (clamped at FLT_EPSILON), zero elsewhere (protocol/swin_moe.py:193-204)
+ *            (clamped at FLT_EPSILON), zero elsewhere (protocol/swin_moe.py:193-204);
+ *            4-byte alignment is enough
  *   mask_out optional int32 [cell_num, path_num], the two SEAT_INDICES outputs only: the
  *            (throttled) hot mask beside its seat indices
  *   scratch  brt_index_scratch_bytes(cell_num, path_num) bytes
  *
  * Returns BRT_ERR_UNSUPPORTED (nothing launched) when path_num is not a multiple of 4 or
- * exceeds 256, an array is not 16-byte aligned, or the scores are too many for the
- * single-launch kernel; the caller then routes in two steps.
+ * exceeds 256, scores, out or mask_out is not 16-byte aligned, or the scores are too many for
+ * the single-launch kernel; the caller then routes in two steps.
  */
 BRT_API int brt_route_scores(const float* scores, int64_t cell_num, int path_num, int decision,
                              int top_k, float threshold, int residual_path, int output,

@@ -138,3 +138,52 @@ def test_gate_edges(cells, paths):
             want = oracle.threshold_hot_mask(score, 0.5, residual)
         got = R.route_scores(dev, "threshold", threshold=0.5, residual_path=residual)[0]
         assert np.array_equal(got.cpu().numpy(), want), residual
+
+
+def test_gates_go_to_an_array_of_any_float_alignment():
+    """Through the C entry point: torch's own allocations are always aligned further."""
+    from brainstorm_b200 import _lib
+
+    cells, paths, k = 1000, 20, 3
+    score = torch.from_numpy(np.random.default_rng(1).standard_normal(
+        (cells, paths)).astype(np.float32)).cuda()
+    nbytes = _lib.query("brt_index_scratch_bytes", cells, paths)
+    scratch = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+    found = []
+    for shift in range(4):
+        room = torch.full((cells * paths + 8,), -7.0, device="cuda")
+        out = torch.empty((cells, paths), dtype=torch.int32, device="cuda")
+        loads = torch.empty(paths, dtype=torch.int32, device="cuda")
+        _lib.call("brt_route_scores", score.data_ptr(), cells, paths, 0, k, 0.0, -1, 2,
+                  out.data_ptr(), loads.data_ptr(), None, None, 0, 0, 0, None, None,
+                  room.data_ptr() + 4 * shift, None, scratch.data_ptr(), nbytes,
+                  _lib.raw_stream(score.device))
+        room = room.cpu()
+        end = shift + cells * paths
+        assert torch.all(room[:shift] == -7) and torch.all(room[end:] == -7)
+        found.append(room[shift:end].reshape(cells, paths).numpy())
+    want = oracle.renormalised_topk_score(score.cpu().numpy(), k)
+    for got in found:
+        assert np.array_equal(got, found[0])
+    assert np.abs(found[0] - want).max() <= 1e-6
+
+
+def test_seats_of_an_array_that_is_only_4_byte_aligned_are_refused():
+    from brainstorm_b200 import _lib
+
+    score = torch.rand((64, 8), device="cuda")
+    nbytes = _lib.query("brt_index_scratch_bytes", 64, 8)
+    scratch = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+    out = torch.zeros(64 * 8 + 4, dtype=torch.int32, device="cuda")
+    loads = torch.empty(8, dtype=torch.int32, device="cuda")
+
+    def call(scores, to, mask_to):
+        return _lib.query("brt_route_scores", scores, 64, 8, 0, 1, 0.0, -1, 2, to,
+                          loads.data_ptr(), None, None, 0, 0, 0, None, None, None, mask_to,
+                          scratch.data_ptr(), nbytes, _lib.raw_stream(score.device))
+
+    good, bad = out.data_ptr(), out.data_ptr() + 4
+    for args in ((score.data_ptr() + 4, good, None), (score.data_ptr(), bad, None),
+                 (score.data_ptr(), good, bad)):
+        assert call(*args) == 4  # BRT_ERR_UNSUPPORTED, nothing is launched
+    assert not out.cpu().any()
