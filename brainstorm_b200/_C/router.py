@@ -89,51 +89,6 @@ def _mark_dense(indices: torch.Tensor, counts: torch.Tensor) -> None:
     setattr(indices, _DENSE, counts)
 
 
-_RECORDS = "_brt_route_records"
-
-
-def _new_records(cells: int, paths: int, device) -> Optional[torch.Tensor]:
-    """Room for the route records of such a mask, or None when its scan leaves none."""
-    if cells * paths < 1 << 21:  # brt_route_record_bytes gives 0 for these
-        return None
-    nbytes = _lib.query("brt_route_record_bytes", cells, paths)
-    return torch.empty(nbytes // 4, dtype=torch.int32, device=device) if nbytes else None
-
-
-def _mark_records(indices: torch.Tensor, records: Optional[torch.Tensor]) -> None:
-    """Remember on the tensor itself the route records that came with ``indices``, with the
-    tensor's version (an edit in place, of it or of a view, makes the note void), its memory,
-    the stream and the capture they were made in.  Inference tensors do not count their
-    edits, so they get no note."""
-    if records is not None and not indices.is_inference():
-        stream = _lib.raw_stream(indices.device)
-        setattr(indices, _RECORDS, (records, indices._version, stream, indices.data_ptr(),
-                                    _lib.query("brt_stream_capture_id", stream)))
-
-
-def _records_of(indices: torch.Tensor, cells: int, paths: int) -> Optional[torch.Tensor]:
-    """The route records of ``indices`` as long as they describe it.  A launch that is captured
-    takes them from its own capture only, and one that is not takes none of a capture: a
-    replay finds in the tensor what was copied there since, which the records would not show.
-    The caller of a stream they were not made on only vouches for ``indices``; their memory
-    is held for it here."""
-    note = getattr(indices, _RECORDS, None)
-    if note is None or not _USE_DENSE or getattr(indices, _DENSE, None) is None:
-        return None
-    records, version, stream, address, capture = note
-    if indices._version != version or indices.data_ptr() != address or \
-            records.device != indices.device or \
-            indices.size(0) != cells or indices.size(1) != paths or \
-            records.numel() != cells * 8:
-        return None
-    here = _lib.raw_stream(indices.device)
-    if _lib.query("brt_stream_capture_id", here) != capture:
-        return None
-    if here != stream:
-        records.record_stream(torch.cuda.current_stream(indices.device))
-    return records
-
-
 def check_index_status() -> None:
     """Raise (once) if an index scan enqueued earlier gave up a bounded wait: its indices and
     loads are wrong.  Reads a word of host memory that the kernels write, no device
@@ -205,15 +160,13 @@ def generate_indices_and_loads(
         loads, counts = both[0], both[1]
         nbytes = _lib.query("brt_index_scratch_bytes", T, E)
         scratch = _scratch.get("index", hot_mask.device, nbytes)
-        records = None if is_tag_index else _new_records(T, E, hot_mask.device)
-        _lib.call("brt_generate_indices_loads_records", _ptr(hot_mask), _ptr(indices),
-                  _ptr(loads), None if is_tag_index else _ptr(counts), _ptr(records), T, E, _ptr(caps), ncap,
+        _lib.call("brt_generate_indices_and_loads", _ptr(hot_mask), _ptr(indices), _ptr(loads),
+                  None if is_tag_index else _ptr(counts), T, E, _ptr(caps), ncap,
                   int(bool(capacity_padding)), int(bool(path_wise_padding)),
                   int(bool(is_tag_index)), _ptr(scratch), scratch.numel(),
                   _stream(hot_mask.device))
         if not is_tag_index:
             _mark_dense(indices, counts)
-            _mark_records(indices, records)
     return indices, loads
 
 
@@ -261,14 +214,12 @@ def throttle_and_generate_indices(
         throttled = torch.empty_like(hot_mask) if with_mask else None
         nbytes = _lib.query("brt_index_scratch_bytes", T, E)
         scratch = _scratch.get("index", dev, nbytes)
-        records = _new_records(T, E, dev)
         try:
-            _lib.call("brt_throttle_and_generate_records", _ptr(hot_mask), _ptr(indices),
-                      _ptr(loads), _ptr(counts), _ptr(records), _ptr(prefix), _ptr(threshold), _ptr(throttled),
+            _lib.call("brt_throttle_and_generate_indices", _ptr(hot_mask), _ptr(indices),
+                      _ptr(loads), _ptr(counts), _ptr(prefix), _ptr(threshold), _ptr(throttled),
                       T, E, _ptr(caps), ncap, int(bool(capacity_padding)),
                       int(bool(path_wise_padding)), _ptr(scratch), scratch.numel(), _stream(dev))
             _mark_dense(indices, counts)
-            _mark_records(indices, records)
         except _lib.BrtError as exc:
             if exc.status != 4:  # BRT_ERR_UNSUPPORTED: the two-step route takes every shape
                 raise
@@ -372,12 +323,10 @@ def route_scores(
                 raise RuntimeError("CHECK_EQ fails.")
         nbytes = _lib.query("brt_index_scratch_bytes", T, E)
         scratch = _scratch.get("index", dev, nbytes)
-        records = _new_records(T, E, dev) if seats else None
         try:
-            _lib.call("brt_route_scores_records", _ptr(score), T, E, _GATE[decision], int(top_k),
+            _lib.call("brt_route_scores", _ptr(score), T, E, _GATE[decision], int(top_k),
                       float(threshold), int(residual_path), _ROUTE_OUT[output], _ptr(out),
-                      _ptr(loads), _ptr(counts) if seats else None, _ptr(records), _ptr(caps),
-                      ncap,
+                      _ptr(loads), _ptr(counts) if seats else None, _ptr(caps), ncap,
                       int(bool(capacity_padding)),
                       int(bool(path_wise_padding)), _ptr(prefix), _ptr(thr), _ptr(gates),
                       _ptr(mask_out), _ptr(scratch), scratch.numel(), _stream(dev))
@@ -387,7 +336,6 @@ def route_scores(
             raise
         if seats:
             _mark_dense(out, counts)
-            _mark_records(out, records)
     if output == "throttled_seat_indices":
         res = (out, loads, prefix)
         if with_gates:
@@ -437,7 +385,11 @@ def dispatch_with_indices_and_loads(
     is_1d_routing: bool = True,
     is_tag_index: bool = False,
 ) -> List[torch.Tensor]:
-    """src/backend/torch/router.cc:131-273."""
+    """src/backend/torch/router.cc:131-273.
+
+    ``route_indices`` as an index operator returned them carry the cells per path: which rows of
+    the output stay empty is taken from there.  A program that drops or adds routes in such a
+    tensor in place deletes its ``_brt_dense_counts`` first (or passes a copy)."""
     return _dispatch(in_data, route_indices, loads, gates, tag_generating, tags,
                      max_path_padding, max_path_load, is_1d_routing, is_tag_index)
 
@@ -533,12 +485,8 @@ def _dispatch(in_data, route_indices, loads, gates, tag_generating, tags, max_pa
             nscratch = _lib.query("brt_dispatch_scratch_bytes", total, path_num)
             scratch = _scratch.get("dispatch", dev, nscratch)
             nscratch = scratch.numel()
-        # the records serve the 1-D kernel of 16-byte rows
-        records = None
-        if dense is not None and is_1d_routing:
-            records = _records_of(route_indices, cell_num, path_num)
-        _lib.call("brt_dispatch_with_records", _ptr(src), _ptr(out), _ptr(g),
-                  _ptr(route_indices), _ptr(records), _ptr(cuda_loads), _ptr(old_tags), _ptr(new_tags),
+        _lib.call("brt_dispatch_with_indices_and_loads", _ptr(src), _ptr(out), _ptr(g),
+                  _ptr(route_indices), _ptr(cuda_loads), _ptr(old_tags), _ptr(new_tags),
                   cell_num, cell_size, path_num, mpl, total, int(bool(is_1d_routing)),
                   int(bool(is_tag_index)), _DT[in_data.dtype], _ptr(dense), _ptr(scratch),
                   nscratch, _stream(dev))
@@ -733,9 +681,8 @@ def combine_with_indices_and_loads(
                 out = torch.empty((cell_num,) + tuple(in_data.shape[1:]), dtype=in_data.dtype,
                                   device=dev)
                 residual = 0
-            records = _records_of(route_indices, cell_num, path_num)
-            _lib.call("brt_combine_with_records", _ptr(src), _ptr(out), _ptr(g),
-                      _ptr(route_indices), _ptr(records), _ptr(cuda_loads), cell_num, cell_size, path_num, mpl,
+            _lib.call("brt_combine_with_indices_and_loads", _ptr(src), _ptr(out), _ptr(g),
+                      _ptr(route_indices), _ptr(cuda_loads), cell_num, cell_size, path_num, mpl,
                       residual, _DT[in_data.dtype], gdt, _stream(dev))
             return [out]
         # tag branch (router.cc:449-472): sum of rows per unique tag

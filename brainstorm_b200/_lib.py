@@ -29,21 +29,6 @@ SIGNATURES = {
     "brt_index_scratch_bytes": (_sz, [_i64, _int]),
     "brt_generate_indices_and_loads": (
         _int, [_vp, _vp, _vp, _vp, _i64, _int, _vp, _int, _int, _int, _int, _vp, _sz, _vp]),
-    "brt_route_record_bytes": (_sz, [_i64, _int]),
-    "brt_stream_capture_id": (ctypes.c_uint64, [_vp]),
-    "brt_generate_indices_loads_records": (
-        _int, [_vp, _vp, _vp, _vp, _vp, _i64, _int, _vp, _int, _int, _int, _int, _vp, _sz, _vp]),
-    "brt_throttle_and_generate_records": (
-        _int, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _int, _vp, _int, _int, _int, _vp,
-               _sz, _vp]),
-    "brt_route_scores_records": (
-        _int, [_vp, _i64, _int, _int, _int, ctypes.c_float, _int, _int, _vp, _vp, _vp, _vp, _vp,
-               _int, _int, _int, _vp, _vp, _vp, _vp, _vp, _sz, _vp]),
-    "brt_dispatch_with_records": (
-        _int, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _int, _i32, _i64, _int, _int,
-               _int, _vp, _vp, _sz, _vp]),
-    "brt_combine_with_records": (
-        _int, [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _int, _i32, _int, _int, _int, _vp]),
     "brt_sum_pieces_by_index": (
         _int, [_vp, _vp, _int, _vp, _vp, _i64, _i64, _int, _vp, _sz, _vp]),
     "brt_tag_group_bytes": (_sz, [_i64]),

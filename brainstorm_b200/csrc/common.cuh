@@ -96,12 +96,6 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-// ---- route records: the first routes of a cell, as the index scan leaves them ---------------
-// kRecordRoutes x (path, seat), ascending paths, seat 0 = none; kRecordMore in the first path:
-// the record does not hold all routes of the cell, read its index row instead.
-constexpr int kRecordRoutes = 4;
-constexpr int kRecordMore = 0x40000000;
-
 // ---- device-side conversion between storage types and fp32 ---------------------------------
 
 template <int DT>

@@ -21,7 +21,7 @@
 
 namespace {
 
-PyObject *g_dense, *g_records;  // attribute names on index tensors
+PyObject* g_dense;  // attribute name on index tensors
 
 // A plain torch.Tensor (no subclass, no functional wrapper) with memory on the GPU.
 const at::Tensor* plain(PyObject* o) {
@@ -66,27 +66,11 @@ bool same_device(const at::Tensor& a, const at::Tensor* b) {
   return b == nullptr || a.get_device() == b->get_device();
 }
 
-unsigned long long address(const void* p) {
-  return (unsigned long long)reinterpret_cast<uintptr_t>(p);
-}
-
-// The notes of an index operator on the tensor it returns, see _C/router.py.
-bool mark(PyObject* indices, const at::Tensor& counts, const at::Tensor& records,
-          const Place& at_place) {
+// The note of an index operator on the tensor it returns, see _C/router.py.
+bool mark(PyObject* indices, const at::Tensor& counts) {
   PyObject* c = THPVariable_Wrap(counts);
-  if (c == nullptr || PyObject_SetAttr(indices, g_dense, c) != 0) {
-    Py_XDECREF(c);
-    return false;
-  }
-  Py_DECREF(c);
-  const at::Tensor& t = THPVariable_Unpack(indices);
-  if (!records.defined() || t.is_inference()) return true;
-  PyObject* note = Py_BuildValue(
-      "(NKKKK)", THPVariable_Wrap(records), (unsigned long long)t._version(),
-      address(at_place.handle()), address(t.data_ptr()),
-      (unsigned long long)brt_stream_capture_id(at_place.handle()));
-  const bool ok = note != nullptr && PyObject_SetAttr(indices, g_records, note) == 0;
-  Py_XDECREF(note);
+  const bool ok = c != nullptr && PyObject_SetAttr(indices, g_dense, c) == 0;
+  Py_XDECREF(c);
   return ok;
 }
 // A new reference or null (no error set) when there is no such attribute.
@@ -107,32 +91,6 @@ const int32_t* dense_counts(PyObject* indices, int64_t paths) {
   Py_DECREF(note);
   return p;
 }
-// The route records noted on `indices`: false when a note is there that needs the slow road
-// (another stream); *out null when there is none, it no longer holds or it is of another capture.
-bool route_records(PyObject* indices, int64_t cells, const Place& at_place, const void** out) {
-  *out = nullptr;
-  PyObject* note = attribute(indices, g_records);
-  if (note == nullptr) return true;
-  bool usable = true;
-  const at::Tensor& t = THPVariable_Unpack(indices);
-  if (PyTuple_Check(note) && PyTuple_GET_SIZE(note) == 5) {
-    const at::Tensor* records = plain(PyTuple_GET_ITEM(note, 0));
-    const unsigned long long version = PyLong_AsUnsignedLongLong(PyTuple_GET_ITEM(note, 1));
-    const unsigned long long stream = PyLong_AsUnsignedLongLong(PyTuple_GET_ITEM(note, 2));
-    const unsigned long long memory = PyLong_AsUnsignedLongLong(PyTuple_GET_ITEM(note, 3));
-    const unsigned long long capture = PyLong_AsUnsignedLongLong(PyTuple_GET_ITEM(note, 4));
-    if (PyErr_Occurred()) PyErr_Clear();
-    if (int32c(records, 1) && !t.is_inference() && version == t._version() &&
-        memory == address(t.data_ptr()) && records->numel() == cells * 8 &&
-        same_device(t, records) && capture == brt_stream_capture_id(at_place.handle())) {
-      usable = stream == address(at_place.handle());
-      if (usable) *out = records->data_ptr();
-    }
-  }
-  Py_DECREF(note);
-  return usable;
-}
-
 struct Caps {
   const int32_t* ptr = nullptr;
   int num = 0;
@@ -167,10 +125,6 @@ PyObject* guarded(F&& body) {
   }
   return nullptr;
 }
-at::Tensor new_records(int64_t cells, int64_t paths, const Place& p) {
-  const size_t bytes = brt_route_record_bytes(cells, (int)paths);
-  return bytes != 0 ? empty({(int64_t)(bytes / 4)}, at::kInt, p.device) : at::Tensor();
-}
 void* data_or_null(const at::Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
 
 // scan(hot_mask, prefix | None, threshold | None, caps | None, capacity_padding, path_wise,
@@ -203,7 +157,6 @@ PyObject* scan(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const at::Tensor loads = both.select(0, 0), counts = both.select(0, 1);
     const at::Tensor throttled =
         with_mask ? empty(mask->sizes(), at::kInt, p.device) : at::Tensor();
-    const at::Tensor records = new_records(T, E, p);
     const int64_t bytes = (int64_t)brt_index_scratch_bytes(T, (int)E);
     const at::Tensor scratch = empty({bytes}, at::kByte, p.device);
     const auto m = static_cast<const int32_t*>(mask->data_ptr());
@@ -211,18 +164,17 @@ PyObject* scan(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const auto l = static_cast<int32_t*>(loads.data_ptr());
     const auto c = static_cast<int32_t*>(counts.data_ptr());
     const int rc =
-        throttle ? brt_throttle_and_generate_records(
-                       m, out, l, c, data_or_null(records),
-                       static_cast<int32_t*>(prefix->data_ptr()),
+        throttle ? brt_throttle_and_generate_indices(
+                       m, out, l, c, static_cast<int32_t*>(prefix->data_ptr()),
                        static_cast<const int32_t*>(threshold->data_ptr()),
                        static_cast<int32_t*>(data_or_null(throttled)), T, (int)E, caps.ptr,
                        caps.num, cpad, pwise, scratch.data_ptr(), (size_t)bytes, p.handle())
-                 : brt_generate_indices_loads_records(
-                       m, out, l, c, data_or_null(records), T, (int)E, caps.ptr, caps.num, cpad,
-                       pwise, 0, scratch.data_ptr(), (size_t)bytes, p.handle());
+                 : brt_generate_indices_and_loads(m, out, l, c, T, (int)E, caps.ptr, caps.num,
+                                                  cpad, pwise, 0, scratch.data_ptr(),
+                                                  (size_t)bytes, p.handle());
     if (rc != BRT_OK) return nullptr;  // nothing was enqueued: the operator says why
     PyObject* i = THPVariable_Wrap(indices);
-    if (i == nullptr || !mark(i, counts, records, p)) {
+    if (i == nullptr || !mark(i, counts)) {
       Py_XDECREF(i);
       return nullptr;
     }
@@ -278,22 +230,20 @@ PyObject* route_scores(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const at::Tensor gates =
         with_gates ? empty(score->sizes(), at::kFloat, p.device) : at::Tensor();
     const at::Tensor mask = with_mask ? empty(score->sizes(), at::kInt, p.device) : at::Tensor();
-    const at::Tensor records = seats ? new_records(T, E, p) : at::Tensor();
     const int64_t bytes = (int64_t)brt_index_scratch_bytes(T, (int)E);
     const at::Tensor scratch = empty({bytes}, at::kByte, p.device);
-    const int rc = brt_route_scores_records(
+    const int rc = brt_route_scores(
         static_cast<const float*>(score->data_ptr()), T, (int)E, (int)decision, (int)top_k,
         (float)threshold, (int)residual, (int)output, static_cast<int32_t*>(out.data_ptr()),
         static_cast<int32_t*>(loads.data_ptr()),
-        seats ? static_cast<int32_t*>(counts.data_ptr()) : nullptr, data_or_null(records),
-        caps.ptr, caps.num, cpad, pwise,
+        seats ? static_cast<int32_t*>(counts.data_ptr()) : nullptr, caps.ptr, caps.num, cpad, pwise,
         throttles ? static_cast<int32_t*>(prefix->data_ptr()) : nullptr,
         throttles ? static_cast<const int32_t*>(limit->data_ptr()) : nullptr,
         static_cast<float*>(data_or_null(gates)), static_cast<int32_t*>(data_or_null(mask)),
         scratch.data_ptr(), (size_t)bytes, p.handle());
     if (rc != BRT_OK) return nullptr;
     PyObject* o = THPVariable_Wrap(out);
-    if (o == nullptr || (seats && !mark(o, counts, records, p))) {
+    if (o == nullptr || (seats && !mark(o, counts))) {
       Py_XDECREF(o);
       return nullptr;
     }
@@ -335,14 +285,12 @@ PyObject* dispatch(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const int32_t* counts = dense_counts(a[1], E);
     if (counts == nullptr) return nullptr;
     const Place p(*x);
-    const void* records;
-    if (!route_records(a[1], T, p, &records)) return nullptr;
     c10::SmallVector<int64_t, 6> shape(x->sizes().begin(), x->sizes().end());
     shape[0] = total;
     const at::Tensor out = empty(shape, x->scalar_type(), p.device);
-    const int rc = brt_dispatch_with_records(
+    const int rc = brt_dispatch_with_indices_and_loads(
         x->data_ptr(), out.data_ptr(), gates != nullptr ? gates->data_ptr() : nullptr,
-        static_cast<const int32_t*>(indices->data_ptr()), records,
+        static_cast<const int32_t*>(indices->data_ptr()),
         static_cast<const int32_t*>(loads->data_ptr()), nullptr, nullptr, T, cell, (int)E,
         (int)mpl, total, 1, 0, dtype, counts, nullptr, 0, p.handle());
     if (rc != BRT_OK) return nullptr;
@@ -386,18 +334,16 @@ PyObject* combine(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const int64_t mpl = padded ? rows / E : 0;
     if (mpl > 0x7fffffffLL) return nullptr;
     const Place p(*x);
-    const void* records = nullptr;
-    if (dense_counts(a[1], E) != nullptr && !route_records(a[1], T, p, &records)) return nullptr;
     at::Tensor out;
     if (residual == nullptr) {
       c10::SmallVector<int64_t, 6> shape(x->sizes().begin(), x->sizes().end());
       shape[0] = T;
       out = empty(shape, x->scalar_type(), p.device);
     }
-    const int rc = brt_combine_with_records(
+    const int rc = brt_combine_with_indices_and_loads(
         x->data_ptr(), residual != nullptr ? residual->data_ptr() : out.data_ptr(),
         gates != nullptr ? gates->data_ptr() : nullptr,
-        static_cast<const int32_t*>(indices->data_ptr()), records,
+        static_cast<const int32_t*>(indices->data_ptr()),
         static_cast<const int32_t*>(loads->data_ptr()), T, cell, (int)E, (int32_t)mpl,
         residual != nullptr, dtype, gate_type, p.handle());
     if (rc != BRT_OK) return nullptr;
@@ -421,6 +367,5 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host_ops", nullptr, -1, methods,
 
 PyMODINIT_FUNC PyInit__host_ops() {
   g_dense = PyUnicode_InternFromString("_brt_dense_counts");
-  g_records = PyUnicode_InternFromString("_brt_route_records");
-  return g_dense != nullptr && g_records != nullptr ? PyModule_Create(&module) : nullptr;
+  return g_dense != nullptr ? PyModule_Create(&module) : nullptr;
 }

@@ -50,18 +50,10 @@ constexpr int kGroupRows = 32;  // cells per bit word
 
 // Where the launch under way writes the per-path cell counts of the indices it produces
 // (null: nowhere).  Set by the entry points around their call into the launch helpers.
-// The same for the cells' route records (chained path only).
 thread_local int32_t* t_counts_out = nullptr;
-thread_local void* t_records_out = nullptr;
 struct CountsScope {
-  explicit CountsScope(int32_t* counts, void* records = nullptr) {
-    t_counts_out = counts;
-    t_records_out = records;
-  }
-  ~CountsScope() {
-    t_counts_out = nullptr;
-    t_records_out = nullptr;
-  }
+  explicit CountsScope(int32_t* counts) { t_counts_out = counts; }
+  ~CountsScope() { t_counts_out = nullptr; }
 };
 
 // kMask: write the 0/1 mask itself.  kThrottleSeat: seat indices and loads of the throttled
@@ -1204,11 +1196,6 @@ __device__ __forceinline__ void gate_words(const TileCtx& x, int* stage, int* bi
 //
 // Any path count: V = 4 stages 16 bytes at a time and wants path_num % 4 == 0 and 16-byte
 // aligned arrays, V = 1 stages element by element.
-//
-// Beside the indices it can leave, per cell, a route record: the first kRecordRoutes routes
-// as (path, seat) in ascending path order, seat 0 where there are fewer, kRecordMore set in
-// the first path when the record does not hold them all (then the index row has to be read).
-// Dispatch and combine read 32 bytes per cell in place of its index row.
 struct ChainArgs {
   TiledArgs t;
   GateArgs gate;
@@ -1222,7 +1209,6 @@ struct ChainArgs {
   int first_ticket; // 0; a test passes 1 so that the first run is never published
   int tiles_per_cta;
   int ranges;
-  uint4* records;   // may be null; path_num <= 256 only
 };
 
 constexpr int kChainFly = 8;    // words a thread keeps in flight
@@ -1466,21 +1452,16 @@ __device__ __forceinline__ void write_tile(const TileCtx& x, int cols, const int
   }
 }
 
-// The routes of the 32 cells of a group, one cell per lane: their elements into a zeroed output
-// (`scatter`) and the cells' records.  Called by a whole warp.
+// The routes of the 32 cells of a group, one cell per lane, into a zeroed output.  Called by a
+// whole warp.
 template <Mode MODE>
 __device__ __forceinline__ void write_routes(const ChainArgs& c, const TileCtx& x, int cols,
                                              int64_t group, const int* bits, const int* base,
-                                             const int* thr, bool scatter) {
+                                             const int* thr) {
   const int lane = threadIdx.x & 31;
   const int64_t row = group * kGroupRows + lane;
   const uint32_t low = 0xffffffffu >> (31 - lane);
   const int64_t at = row * x.path_num + (int64_t)x.chunk * x.ec;
-  const bool records = (MODE == Mode::kSeat || MODE == Mode::kThrottleSeat) && c.records != nullptr;
-  int n = 0;
-  int path[kRecordRoutes], seats[kRecordRoutes];
-#pragma unroll
-  for (int k = 0; k < kRecordRoutes; k++) { path[k] = 0; seats[k] = 0; }
   // 128 paths at a time: four transposes in flight, and one turn of the loop takes a route of
   // every lane wherever in the 128 it lies
   for (int c0 = 0; c0 < cols; c0 += 128) {
@@ -1514,22 +1495,11 @@ __device__ __forceinline__ void write_routes(const ChainArgs& c, const TileCtx& 
         if (seat >= 1 && seat <= x.cell_num)
           c.t.out[(int64_t)(seat - 1) * x.path_num + (int64_t)x.chunk * x.ec + col] =
               (int)(row + 1);
-      } else if (scatter) {
+      } else {
         c.t.out[at + col] = v;
         if (c.t.mask_out != nullptr) c.t.mask_out[at + col] = 1;
       }
-      if (records) {
-#pragma unroll
-        for (int k = 0; k < kRecordRoutes; k++)
-          if (n == k) { path[k] = col; seats[k] = v; }
-        n++;
-      }
     }
-  }
-  if (records && row < x.cell_num) {
-    if (n > kRecordRoutes) path[0] |= kRecordMore;
-    c.records[2 * row] = make_uint4(path[0], seats[0], path[1], seats[1]);
-    c.records[2 * row + 1] = make_uint4(path[2], seats[2], path[3], seats[3]);
   }
 }
 
@@ -1695,12 +1665,6 @@ __global__ void __launch_bounds__(kTileThreads, 2) index_chain_kernel(const Chai
     for (int64_t t = tile0; t < tile1; t++) {
       x.tile = t;
       expand_general<MODE>(x, a.mask, run, a.out, a.threshold);
-      if (c.records != nullptr)  // seats of such a mask are not counts: read the index rows
-        for (int r = tid; r < rows_of(x); r += kTileThreads) {
-          const int64_t row = t * a.rg * kGroupRows + r;
-          c.records[2 * row] = make_uint4((unsigned)kRecordMore, 0u, 0u, 0u);
-          c.records[2 * row + 1] = make_uint4(0u, 0u, 0u, 0u);
-        }
     }
     return;
   }
@@ -1720,15 +1684,12 @@ __global__ void __launch_bounds__(kTileThreads, 2) index_chain_kernel(const Chai
     }
   }
   __syncthreads();
-  const bool with_records = c.records != nullptr;
   for (int g = tid >> 5; g < groups; g += kTileWarps) {
     const int i = g / a.rg;
     x.tile = tile0 + i;
-    const bool scatter =
-        MODE == Mode::kTag || sm.routed[i] * kSparse <= rows_of(x) * cols;  // warp-uniform
-    if (scatter || with_records)
+    if (MODE == Mode::kTag || sm.routed[i] * kSparse <= rows_of(x) * cols)  // warp-uniform
       write_routes<MODE>(c, x, cols, tile0 * a.rg + g, sm.bits + g * a.ec, sm.base + g * a.ec,
-                         sm.thr, scatter);
+                         sm.thr);
   }
   if constexpr (MODE != Mode::kTag) {
     for (int i = 0; i < tiles; i++) {
@@ -1847,8 +1808,6 @@ ChainPlan plan_chain(int64_t cell_num, int path_num, bool wide) {
   return plan;
 }
 
-constexpr int64_t kRecordMinElements = 1 << 21;
-
 bool forced_split() {
   static const bool forced = [] {
     const char* const v = getenv("BRT_INDEX_PATH");
@@ -1881,7 +1840,6 @@ int launch_chain(Mode mode, const ChainPlan& plan, bool wide, const int32_t* mas
   c.block = blocks ? c.status + (size_t)plan.ranges * path_num : nullptr;
   c.tiles_per_cta = plan.tiles_per_cta;
   c.ranges = plan.ranges;
-  c.records = static_cast<uint4*>(t_records_out);
   c.t.tile_flags = nullptr;
   c.t.tile_sums = nullptr;
   c.t.bits = nullptr;
@@ -1956,7 +1914,6 @@ int launch_tiled(Mode mode, const int32_t* mask, int32_t* out, int32_t* loads, i
     return set_error(BRT_ERR_UNSUPPORTED,
                      "a %lld x %d mask does not fit the single-launch scan; throttle and index "
                      "it in two steps", (long long)cell_num, path_num);
-  BRT_REQUIRE(t_records_out == nullptr, "this mask gets no route records");
   const TileGeom g = make_tile_geom(cell_num, path_num);
   BRT_REQUIRE(g.num_tiles <= 0x7fffffffLL && g.col_chunks <= 65535,
               "mask of %lld x %d cells is too large for one launch", (long long)cell_num,
@@ -2086,7 +2043,6 @@ int run_scan(Mode mode, const int32_t* mask, int32_t* out, int32_t* loads, int64
       return launch_chain(mode, plan, false, mask, out, loads, cell_num, path_num, caps, ncap,
                           capacity_padding, path_wise, prefix, threshold, scratch, stream);
   }
-  BRT_REQUIRE(t_records_out == nullptr, "this mask gets no route records");
   const bool a16 = aligned_to(mask, 16) && aligned_to(out, 16) &&
                    (threshold == nullptr || aligned_to(threshold, 16));
   const bool a8 = aligned_to(mask, 8) && aligned_to(out, 8) &&
@@ -2148,46 +2104,8 @@ BRT_API size_t brt_index_scratch_bytes(int64_t cell_num, int path_num) {
   return scratch_bytes_for(cell_num, path_num);
 }
 
-BRT_API size_t brt_route_record_bytes(int64_t cell_num, int path_num) {
-  // Up to 16 paths an index row is no longer than two records.  Below 8 MB of indices the rows
-  // come out of L2 and the records save little for what their allocation costs the host (4 us):
-  // 64 x 32, a step of 57 us took 64 with them; 32768 x 32, 84 us took 83, but the gate alone
-  // 27 -> 32.
-  if (cell_num * path_num < kRecordMinElements) return 0;
-  if (cell_num <= 0 || path_num <= 16 || path_num > 256 || forced_split()) return 0;
-  if (plan_chain(cell_num, path_num, false).smem == 0) return 0;
-  if (path_num % 4 == 0 && plan_chain(cell_num, path_num, true).smem == 0) return 0;
-  return (size_t)cell_num * kRecordRoutes * 8;
-}
-
-BRT_API uint64_t brt_stream_capture_id(void* stream) {
-  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-  unsigned long long id = 0;
-  if (cudaStreamGetCaptureInfo(static_cast<cudaStream_t>(stream), &status, &id) != cudaSuccess) {
-    (void)cudaGetLastError();
-    return UINT64_MAX;
-  }
-  if (status == cudaStreamCaptureStatusNone) return 0;
-  return status == cudaStreamCaptureStatusActive ? (uint64_t)id : UINT64_MAX;
-}
-
 BRT_API int brt_generate_indices_and_loads(const int32_t* hot_mask, int32_t* indices,
                                            int32_t* loads, int32_t* path_counts,
-                                           int64_t cell_num, int path_num,
-                                           const int32_t* supported_capacities,
-                                           int supported_capacity_num, int capacity_padding,
-                                           int path_wise_padding, int is_tag_index,
-                                           void* scratch, size_t scratch_bytes, void* stream) {
-  return brt_generate_indices_loads_records(hot_mask, indices, loads, path_counts, nullptr,
-                                            cell_num, path_num, supported_capacities,
-                                            supported_capacity_num, capacity_padding,
-                                            path_wise_padding, is_tag_index, scratch,
-                                            scratch_bytes, stream);
-}
-
-BRT_API int brt_generate_indices_loads_records(const int32_t* hot_mask, int32_t* indices,
-                                           int32_t* loads, int32_t* path_counts,
-                                           void* route_records,
                                            int64_t cell_num, int path_num,
                                            const int32_t* supported_capacities,
                                            int supported_capacity_num, int capacity_padding,
@@ -2217,9 +2135,7 @@ BRT_API int brt_generate_indices_loads_records(const int32_t* hot_mask, int32_t*
     return BRT_OK;
   }
   BRT_REQUIRE(hot_mask != nullptr && indices != nullptr, "hot_mask or indices is null");
-  BRT_REQUIRE(route_records == nullptr || (!is_tag_index && aligned_to(route_records, 16)),
-              "route_records go with seat indices and must be 16-byte aligned");
-  const CountsScope counts(path_counts, route_records);
+  const CountsScope counts(path_counts);
   return run_scan(is_tag_index ? Mode::kTag : Mode::kSeat, hot_mask, indices, loads, cell_num,
                   path_num, supported_capacities, supported_capacity_num, capacity_padding,
                   path_wise, nullptr, nullptr, scratch, scratch_bytes, st);
@@ -2242,18 +2158,6 @@ BRT_API int brt_throttle_hotmask(const int32_t* hotmask, int32_t* throttled, int
 BRT_API int brt_throttle_and_generate_indices(
     const int32_t* hot_mask, int32_t* indices, int32_t* loads, int32_t* path_counts,
     int32_t* prefix, const int32_t* threshold, int32_t* throttled_mask, int64_t cell_num,
-    int path_num, const int32_t* supported_capacities, int supported_capacity_num,
-    int capacity_padding, int path_wise_padding, void* scratch, size_t scratch_bytes,
-    void* stream) {
-  return brt_throttle_and_generate_records(
-      hot_mask, indices, loads, path_counts, nullptr, prefix, threshold, throttled_mask, cell_num,
-      path_num, supported_capacities, supported_capacity_num, capacity_padding,
-      path_wise_padding, scratch, scratch_bytes, stream);
-}
-
-BRT_API int brt_throttle_and_generate_records(
-    const int32_t* hot_mask, int32_t* indices, int32_t* loads, int32_t* path_counts,
-    void* route_records, int32_t* prefix, const int32_t* threshold, int32_t* throttled_mask, int64_t cell_num,
     int path_num,
     const int32_t* supported_capacities, int supported_capacity_num, int capacity_padding,
     int path_wise_padding, void* scratch, size_t scratch_bytes, void* stream) {
@@ -2291,8 +2195,7 @@ BRT_API int brt_throttle_and_generate_records(
   if (scratch_bytes < need)
     return set_error(BRT_ERR_SCRATCH_TOO_SMALL, "scratch holds %zu bytes, %zu needed",
                      scratch_bytes, need);
-  BRT_REQUIRE(aligned_to(route_records, 16), "route_records must be 16-byte aligned");
-  const CountsScope counts(path_counts, route_records);
+  const CountsScope counts(path_counts);
   return launch_tiled(Mode::kThrottleSeat, hot_mask, indices, loads, cell_num, path_num,
                       supported_capacities, supported_capacity_num, capacity_padding, path_wise,
                       prefix, threshold, scratch, st, nullptr, throttled_mask);
@@ -2301,21 +2204,6 @@ BRT_API int brt_throttle_and_generate_records(
 BRT_API int brt_route_scores(const float* scores, int64_t cell_num, int path_num, int decision,
                              int top_k, float threshold, int residual_path, int output,
                              int32_t* out, int32_t* loads, int32_t* path_counts,
-                             const int32_t* capacities, int capacity_num, int capacity_padding,
-                             int path_wise_padding, int32_t* prefix,
-                             const int32_t* throttle_capacity, float* gates_out,
-                             int32_t* mask_out, void* scratch, size_t scratch_bytes,
-                             void* stream) {
-  return brt_route_scores_records(scores, cell_num, path_num, decision, top_k, threshold,
-                                  residual_path, output, out, loads, path_counts, nullptr,
-                                  capacities, capacity_num, capacity_padding, path_wise_padding,
-                                  prefix, throttle_capacity, gates_out, mask_out, scratch,
-                                  scratch_bytes, stream);
-}
-
-BRT_API int brt_route_scores_records(const float* scores, int64_t cell_num, int path_num, int decision,
-                             int top_k, float threshold, int residual_path, int output,
-                             int32_t* out, int32_t* loads, int32_t* path_counts, void* route_records,
                              const int32_t* capacities,
                              int capacity_num, int capacity_padding, int path_wise_padding,
                              int32_t* prefix, const int32_t* throttle_capacity, float* gates_out,
@@ -2350,10 +2238,6 @@ BRT_API int brt_route_scores_records(const float* scores, int64_t cell_num, int 
   BRT_REQUIRE(path_counts == nullptr || output == BRT_ROUTE_SEAT_INDICES ||
                   output == BRT_ROUTE_THROTTLED_SEAT_INDICES,
               "path_counts goes with the seat-index outputs only");
-  BRT_REQUIRE(route_records == nullptr ||
-                  ((output == BRT_ROUTE_SEAT_INDICES ||
-                    output == BRT_ROUTE_THROTTLED_SEAT_INDICES) && aligned_to(route_records, 16)),
-              "route_records go with the seat-index outputs and must be 16-byte aligned");
   if (cell_num == 0) {
     if (output != BRT_ROUTE_THROTTLED_MASK)
       BRT_CUDA_TRY(cudaMemsetAsync(loads, 0, (size_t)path_num * 4, static_cast<cudaStream_t>(stream)));
@@ -2382,7 +2266,7 @@ BRT_API int brt_route_scores_records(const float* scores, int64_t cell_num, int 
                     : output == BRT_ROUTE_THROTTLED_MASK ? Mode::kThrottle
                     : output == BRT_ROUTE_THROTTLED_SEAT_INDICES ? Mode::kThrottleSeat
                                                                  : Mode::kSeat;
-  const CountsScope counts(path_counts, route_records);
+  const CountsScope counts(path_counts);
   return launch_tiled(mode, reinterpret_cast<const int32_t*>(scores), out, loads, cell_num,
                       path_num, capacities, capacity_num, capacity_padding, path_wise_padding,
                       prefix, throttle_capacity, scratch, static_cast<cudaStream_t>(stream), &gate,

@@ -269,28 +269,15 @@ __global__ void __launch_bounds__(kThreads) dispatch_tag_kernel(const MoveArgs a
 
 // ---------------------------------------------------------------------------------- combine
 // GMODE: 0 = no gates, 1 = fp32 gates, 2 = gates stored in the data type.
-// 16-byte rows only (VB == 16).  IV: paths per lane of an index row scan, or 0: the routes come
-// from the cells' records, 32 bytes per cell in place of an index and a gate row, and only the
-// gates of kept routes are read (262144 x 128, top-1, rows of 1.5 KB: 127 us -> 92).
-template <int IV>
-struct FoldStageOf {
-  using type = FoldStage;
-};
-template <>
-struct FoldStageOf<0> {
-  using type = RecordFoldStage;
-};
+// 16-byte rows only (VB == 16).
 template <int DT, int GMODE, int IV>
 __global__ void __launch_bounds__(kThreads, 3) combine_seat_async_kernel(const MoveArgs a) {
   constexpr int VB = 16;
-  constexpr bool kRecords = IV == 0;
-  constexpr int kScan = kRecords ? 1 : IV;  // a record that does not hold all routes
   using L = Lanes<VB, DT>;
   using V = typename L::V;
-  using Stage = typename FoldStageOf<IV>::type;
   extern __shared__ __align__(16) unsigned char s_raw[];
-  Stage* s_stage = reinterpret_cast<Stage*>(s_raw);  // [kWarps][kStages]
-  int* s_loads = reinterpret_cast<int*>(s_raw + sizeof(Stage) * kWarps * kStages);
+  FoldStage* s_stage = reinterpret_cast<FoldStage*>(s_raw);  // [kWarps][kStages]
+  int* s_loads = reinterpret_cast<int*>(s_raw + sizeof(FoldStage) * kWarps * kStages);
   int* s_base = s_loads + a.path_num;
   setup_tables(a.loads, nullptr, a.path_num, a.max_path_load, s_loads, s_base, nullptr, nullptr);
 
@@ -302,54 +289,26 @@ __global__ void __launch_bounds__(kThreads, 3) combine_seat_async_kernel(const M
   const V* __restrict__ src = static_cast<const V*>(a.src);
   V* __restrict__ dst = static_cast<V*>(a.dst);
   const int E = a.path_num;
-  Stage* my = s_stage + warp_in_cta * kStages;
+  FoldStage* my = s_stage + warp_in_cta * kStages;
 
-  int seat[kScan];
-  float gate[kScan];
-  uint2 record = make_uint2(0u, 0u);
-  // the gate of this lane's route travels in a register until the item is folded: [0] of the
-  // item being folded, [1] of the one issued after it
-  float held_gate_of[2] = {1.f, 1.f};
-  int held_slot_of[2] = {-1, -1};
+  int seat[IV];
+  float gate[IV];
   // the cell an item position stands for (positions are walked upwards either way)
   auto cell_at = [&](int64_t pos) { return a.newest_first ? a.cell_num - 1 - pos : pos; };
   auto fetch = [&](const ItemCursor& c) {
-    if constexpr (kRecords) {
-      record = make_uint2(0u, 0u);
-      if (c.cell < a.cell_num && lane < kRecordRoutes)
-        record = a.records[cell_at(c.cell) * kRecordRoutes + lane];
-    } else {
 #pragma unroll
-      for (int j = 0; j < kScan; j++) { seat[j] = 0; gate[j] = 1.f; }
-      if (c.cell < a.cell_num) {
-        load_index_chunk<kScan>(a.indices, cell_at(c.cell), E, 0, lane, seat);
-        load_gate_chunk<kScan, GMODE, DT>(a.gates, cell_at(c.cell), E, 0, lane, gate);
-      }
+    for (int j = 0; j < IV; j++) { seat[j] = 0; gate[j] = 1.f; }
+    if (c.cell < a.cell_num) {
+      load_index_chunk<IV>(a.indices, cell_at(c.cell), E, 0, lane, seat);
+      load_gate_chunk<IV, GMODE, DT>(a.gates, cell_at(c.cell), E, 0, lane, gate);
     }
   };
   // Build the route table of an item from the registers fetched for it and start the
   // asynchronous copies of its rows; always closes exactly one copy group.
-  auto issue = [&](Stage& st, const ItemCursor& c) {
-    if constexpr (kRecords) held_slot_of[1] = -1;
+  auto issue = [&](FoldStage& st, const ItemCursor& c) {
     if (c.cell < a.cell_num) {
-      const int64_t cell = cell_at(c.cell);
-      int count;
-      if constexpr (kRecords) {
-        const unsigned first = __shfl_sync(0xffffffffu, record.x, 0);
-        if ((first & (unsigned)kRecordMore) == 0u) {
-          int path;
-          count = record_routes(record, s_loads, s_base, st.route, lane, path, held_slot_of[1]);
-          if (held_slot_of[1] >= 0) held_gate_of[1] = gate_at<DT, GMODE>(a.gates, cell * E + path);
-        } else {
-          load_index_chunk<kScan>(a.indices, cell, E, 0, lane, seat);
-          load_gate_chunk<kScan, GMODE, DT>(a.gates, cell, E, 0, lane, gate);
-          count = build_routes<kScan, GMODE, DT, false>(a, cell, seat, gate, s_loads, s_base,
-                                                        st.route, lane, kRecordRoutes);
-        }
-      } else {
-        count = build_routes<kScan, GMODE, DT, false>(a, cell, seat, gate, s_loads, s_base,
-                                                      st.route, lane);
-      }
+      const int count = build_routes<IV, GMODE, DT, false>(a, cell_at(c.cell), seat, gate,
+                                                           s_loads, s_base, st.route, lane);
       if (lane == 0) st.count = count;
       __syncwarp();
       const int staged = count < kMaxRoutes ? count : kMaxRoutes;
@@ -376,18 +335,12 @@ __global__ void __launch_bounds__(kThreads, 3) combine_seat_async_kernel(const M
   issue(my[0], at);
   fetch(ahead);
   while (at.cell < a.cell_num) {
-    if constexpr (kRecords) {
-      held_gate_of[0] = held_gate_of[1];
-      held_slot_of[0] = held_slot_of[1];
-    }
     issue(my[stage ^ 1], ahead);
     fetch(ahead2);
     cp_async_wait<1>();
-    if constexpr (kRecords)
-      if (held_slot_of[0] >= 0) my[stage].route[held_slot_of[0]].gate = held_gate_of[0];
     __syncwarp();
 
-    const Stage& st = my[stage];
+    const FoldStage& st = my[stage];
     const int64_t cell = cell_at(at.cell);
     const int64_t first = (int64_t)at.piece * kFoldVecs;
     const int count = st.count;
@@ -428,10 +381,15 @@ __global__ void __launch_bounds__(kThreads, 3) combine_seat_async_kernel(const M
         V held0 = zero_chunk<V>(), held1 = zero_chunk<V>();
         float held_gate = 0.f;
         bool pending = false;
-        auto fold_row = [&](int64_t row, float next_gate) {
-          const V* rp = src + row * a.row_vecs + first;
+        int seen = 0;
+        for (int e = 0; e < E; e++) {
+          const int s = a.indices[cell * E + e];
+          if (s <= 0 || s > s_loads[e]) continue;
+          if (seen++ < kMaxRoutes) continue;
+          const V* rp = src + ((int64_t)s_base[e] + s - 1) * a.row_vecs + first;
           const V next0 = in0 ? load_stream(rp + v0) : zero_chunk<V>();
           const V next1 = in1 ? load_stream(rp + v1) : zero_chunk<V>();
+          const float next_gate = gate_at<DT, GMODE>(a.gates, cell * E + e);
           if (pending) {
             fold_chunk<VB, DT, GMODE>(acc0, held0, held_gate);
             fold_chunk<VB, DT, GMODE>(acc1, held1, held_gate);
@@ -440,17 +398,6 @@ __global__ void __launch_bounds__(kThreads, 3) combine_seat_async_kernel(const M
           held1 = next1;
           held_gate = next_gate;
           pending = true;
-        };
-        if (kRecords && count <= kRecordRoutes) {
-          for (int r = kMaxRoutes; r < count; r++) fold_row(st.route[r].row, st.route[r].gate);
-        } else {
-          int seen = 0;
-          for (int e = 0; e < E; e++) {
-            const int s = a.indices[cell * E + e];
-            if (s <= 0 || s > s_loads[e]) continue;
-            if (seen++ < kMaxRoutes) continue;
-            fold_row((int64_t)s_base[e] + s - 1, gate_at<DT, GMODE>(a.gates, cell * E + e));
-          }
         }
         if (pending) {
           fold_chunk<VB, DT, GMODE>(acc0, held0, held_gate);
@@ -474,17 +421,12 @@ __global__ void __launch_bounds__(kThreads, 3) combine_seat_async_kernel(const M
 // 1-D seat-index dispatch of 16-byte rows.  Same ownership as dispatch_seat_kernel (a warp
 // owns a (cell, 2 KB piece)), but the piece travels through shared memory: the asynchronous
 // copy of the warp's NEXT item is in flight while the current one is stored to its routes,
-// and cells that no path kept are never read.  IV: paths per lane of an index row scan, or 0: the
-// routes come from the cells' records (262144 x 128, top-1, rows of 1.5 KB: 192 us ->
-// 181; with the CTAs in order, see plan_dispatch, 145: 5.9 TB/s).  Zero rows are written before
-// the wait for the item's own row.
+// and cells that no path kept are never read.  Zero rows are written before the wait for the
+// item's own row.
 template <int DT, bool WEIGHTED, int IV>
 __global__ void __launch_bounds__(kThreads, WEIGHTED ? 3 : 4) dispatch_seat_async_kernel(const MoveArgs a) {
   constexpr int VB = 16;
   constexpr int GK = WEIGHTED ? 2 : 0;
-  constexpr bool kRecords = IV == 0;
-  constexpr int kScan = kRecords ? 1 : IV;  // a record that does not hold all routes
-  static_assert(kCopyRoutes == kRecordRoutes, "the route table takes a whole record");
   using V = uint4;
   extern __shared__ __align__(16) unsigned char s_raw[];
   CopyStage* s_stage = reinterpret_cast<CopyStage*>(s_raw);  // [kWarps][kStages]
@@ -501,49 +443,20 @@ __global__ void __launch_bounds__(kThreads, WEIGHTED ? 3 : 4) dispatch_seat_asyn
   const int E = a.path_num;
   CopyStage* my = s_stage + warp_in_cta * kStages;
   const unsigned long long evict_first = l2_evict_first_policy();
-  int seat[kScan];
-  float gate[kScan];
-  uint2 record = make_uint2(0u, 0u);
-  // as in combine_seat_async_kernel: [0] of the item being stored, [1] of the one issued after it
-  float held_gate_of[2] = {1.f, 1.f};
-  int held_slot_of[2] = {-1, -1};
+  int seat[IV];
+  float gate[IV];
   auto fetch = [&](const ItemCursor& c) {
-    if constexpr (kRecords) {
-      record = make_uint2(0u, 0u);
-      if (c.cell < a.cell_num && lane < kRecordRoutes)
-        record = a.records[c.cell * kRecordRoutes + lane];
-    } else {
 #pragma unroll
-      for (int j = 0; j < kScan; j++) { seat[j] = 0; gate[j] = 1.f; }
-      if (c.cell < a.cell_num) {
-        load_index_chunk<kScan>(a.indices, c.cell, E, 0, lane, seat);
-        load_gate_chunk<kScan, GK, DT>(a.gates, c.cell, E, 0, lane, gate);
-      }
+    for (int j = 0; j < IV; j++) { seat[j] = 0; gate[j] = 1.f; }
+    if (c.cell < a.cell_num) {
+      load_index_chunk<IV>(a.indices, c.cell, E, 0, lane, seat);
+      load_gate_chunk<IV, GK, DT>(a.gates, c.cell, E, 0, lane, gate);
     }
   };
   auto issue = [&](CopyStage& st, const ItemCursor& c) {
-    if constexpr (kRecords && WEIGHTED) held_slot_of[1] = -1;
     if (c.cell < a.cell_num) {
-      int count;
-      if constexpr (kRecords) {
-        const unsigned first = __shfl_sync(0xffffffffu, record.x, 0);
-        if ((first & (unsigned)kRecordMore) == 0u) {
-          int path, slot;
-          count = record_routes(record, s_loads, s_base, st.route, lane, path, slot);
-          if constexpr (WEIGHTED) {
-            held_slot_of[1] = slot;
-            if (slot >= 0) held_gate_of[1] = gate_at<DT, 2>(a.gates, c.cell * E + path);
-          }
-        } else {
-          load_index_chunk<kScan>(a.indices, c.cell, E, 0, lane, seat);
-          load_gate_chunk<kScan, GK, DT>(a.gates, c.cell, E, 0, lane, gate);
-          count = build_routes<kScan, GK, DT, false>(a, c.cell, seat, gate, s_loads, s_base,
-                                                     st.route, lane, kCopyRoutes);
-        }
-      } else {
-        count = build_routes<kScan, GK, DT, false>(a, c.cell, seat, gate, s_loads, s_base,
-                                                   st.route, lane, kCopyRoutes);
-      }
+      const int count = build_routes<IV, GK, DT, false>(a, c.cell, seat, gate, s_loads, s_base,
+                                                        st.route, lane, kCopyRoutes);
       if (lane == 0) st.count = count;
       if (count > 0) {
         const int64_t first = (int64_t)c.piece * kPieceVecs;
@@ -573,16 +486,10 @@ __global__ void __launch_bounds__(kThreads, WEIGHTED ? 3 : 4) dispatch_seat_asyn
   issue(my[0], at);
   fetch(ahead);
   while (at.cell < a.cell_num) {
-    if constexpr (kRecords && WEIGHTED) {
-      held_gate_of[0] = held_gate_of[1];
-      held_slot_of[0] = held_slot_of[1];
-    }
     issue(my[stage ^ 1], ahead);
     fetch(ahead2);
     if (dense) fill.run(a, fill.per_turn, s_base, s_written, s_fill, lane);
     cp_async_wait<1>();
-    if constexpr (kRecords && WEIGHTED)
-      if (held_slot_of[0] >= 0) my[stage].route[held_slot_of[0]].gate = held_gate_of[0];
     __syncwarp();
 
     const CopyStage& st = my[stage];
@@ -865,11 +772,7 @@ void launch_dispatch(const MoveArgs& a, bool is_tag, cudaStream_t st) {
       const size_t smem_async = sizeof(CopyStage) * kWarps * kStages + smem;
       MoveArgs b = a;
       const unsigned grid = plan_dispatch(b, WEIGHTED ? 3 : 4);
-      if (a.records != nullptr) {
-        configure_smem<dispatch_seat_async_kernel<DT, WEIGHTED, 0>>(sizeof(CopyStage) * kWarps *
-                                                                    kStages);
-        dispatch_seat_async_kernel<DT, WEIGHTED, 0><<<grid, kThreads, smem_async, st>>>(b), note_launch();
-      } else if (wide_rows(a.indices, a.gates, dtype_size(DT), a.path_num)) {
+      if (wide_rows(a.indices, a.gates, dtype_size(DT), a.path_num)) {
         configure_smem<dispatch_seat_async_kernel<DT, WEIGHTED, 4>>(sizeof(CopyStage) * kWarps *
                                                                     kStages);
         dispatch_seat_async_kernel<DT, WEIGHTED, 4><<<grid, kThreads, smem_async, st>>>(b), note_launch();
@@ -933,15 +836,14 @@ void launch_zero_fill(const MoveArgs& a, cudaStream_t st) {
 
 template <int DT, int GMODE, int IV>
 int launch_combine_async(const MoveArgs& a, cudaStream_t st) {
-  using Stage = typename FoldStageOf<IV>::type;
-  const size_t smem = sizeof(Stage) * kWarps * kStages + (size_t)a.path_num * 2 * sizeof(int);
+  const size_t smem = sizeof(FoldStage) * kWarps * kStages + (size_t)a.path_num * 2 * sizeof(int);
   static thread_local int configured_device = -1;
   int dev = 0;
   BRT_CUDA_TRY(cudaGetDevice(&dev));
   if (configured_device != dev) {
     BRT_CUDA_TRY(cudaFuncSetAttribute(combine_seat_async_kernel<DT, GMODE, IV>,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)(sizeof(Stage) * kWarps * kStages +
+                                      (int)(sizeof(FoldStage) * kWarps * kStages +
                                             (size_t)kMaxPaths * 2 * sizeof(int))));
     configured_device = dev;
   }
@@ -954,7 +856,6 @@ int launch_combine_async(const MoveArgs& a, cudaStream_t st) {
 template <int VB, int DT, int GMODE>
 int launch_combine(const MoveArgs& a, cudaStream_t st) {
   if constexpr (VB == 16) {
-    if (a.records != nullptr) return launch_combine_async<DT, GMODE, 0>(a, st);
     const int gate_bytes = GMODE == 1 ? 4 : dtype_size(DT);
     if (wide_rows(a.indices, a.gates, gate_bytes, a.path_num))
       return launch_combine_async<DT, GMODE, 4>(a, st);
@@ -1007,18 +908,6 @@ BRT_API int brt_dispatch_with_indices_and_loads(
     int64_t cell_size, int path_num, int32_t max_path_load, int64_t total_rows,
     int is_1d_routing, int is_tag_index, int dtype, const int32_t* dense_counts, void* scratch,
     size_t scratch_bytes, void* stream) {
-  return brt_dispatch_with_records(src_data, dst_data, gates, route_indices, nullptr, loads,
-                                   old_tags, new_tags, cell_num, cell_size, path_num,
-                                   max_path_load, total_rows, is_1d_routing, is_tag_index, dtype,
-                                   dense_counts, scratch, scratch_bytes, stream);
-}
-
-BRT_API int brt_dispatch_with_records(
-    const void* src_data, void* dst_data, const void* gates, const int32_t* route_indices,
-    const void* route_records, const int32_t* loads, const int32_t* old_tags, int32_t* new_tags, int64_t cell_num,
-    int64_t cell_size, int path_num, int32_t max_path_load, int64_t total_rows,
-    int is_1d_routing, int is_tag_index, int dtype, const int32_t* dense_counts, void* scratch,
-    size_t scratch_bytes, void* stream) {
   clear_error();
   BRT_REQUIRE(dtype == BRT_F32 || dtype == BRT_F16 || dtype == BRT_BF16, "bad dtype %d", dtype);
   BRT_REQUIRE(cell_num >= 0 && cell_size >= 0 && total_rows >= 0, "negative size");
@@ -1026,7 +915,6 @@ BRT_API int brt_dispatch_with_records(
               kMaxPaths);
   BRT_REQUIRE(max_path_load >= 0, "negative max_path_load");
   BRT_REQUIRE(total_rows <= 0x7fffffffLL, "more than 2^31-1 output rows");
-  BRT_REQUIRE(aligned_to(route_records, 8), "route_records must be 8-byte aligned");
   BRT_REQUIRE((old_tags == nullptr) == (new_tags == nullptr),
               "old_tags and new_tags must be given together");
   BRT_REQUIRE(gates == nullptr || is_1d_routing, "gates are only supported with 1-D routing");
@@ -1047,7 +935,6 @@ BRT_API int brt_dispatch_with_records(
   a.dst = dst_data;
   a.gates = gates;
   a.indices = route_indices;
-  a.records = is_tag_index ? nullptr : static_cast<const uint2*>(route_records);
   a.loads = loads;
   a.old_tags = old_tags;
   a.new_tags = new_tags;
@@ -1106,16 +993,6 @@ BRT_API int brt_combine_with_indices_and_loads(
     const void* src_data, void* dst_data, const void* gates, const int32_t* route_indices,
     const int32_t* loads, int64_t cell_num, int64_t cell_size, int path_num,
     int32_t max_path_load, int is_residual, int dtype, int gates_dtype, void* stream) {
-  return brt_combine_with_records(src_data, dst_data, gates, route_indices, nullptr, loads,
-                                  cell_num, cell_size, path_num, max_path_load, is_residual,
-                                  dtype, gates_dtype, stream);
-}
-
-BRT_API int brt_combine_with_records(
-    const void* src_data, void* dst_data, const void* gates, const int32_t* route_indices,
-    const void* route_records, const int32_t* loads, int64_t cell_num, int64_t cell_size,
-    int path_num, int32_t max_path_load, int is_residual, int dtype, int gates_dtype,
-    void* stream) {
   clear_error();
   BRT_REQUIRE(dtype == BRT_F32 || dtype == BRT_F16 || dtype == BRT_BF16, "bad dtype %d", dtype);
   BRT_REQUIRE(gates == nullptr || gates_dtype == BRT_F32 || gates_dtype == dtype,
@@ -1124,7 +1001,6 @@ BRT_API int brt_combine_with_records(
   BRT_REQUIRE(path_num > 0 && path_num <= kMaxPaths, "path_num %d outside [1, %d]", path_num,
               kMaxPaths);
   BRT_REQUIRE(max_path_load >= 0, "negative max_path_load");
-  BRT_REQUIRE(aligned_to(route_records, 8), "route_records must be 8-byte aligned");
   if (cell_num == 0 || cell_size == 0) return BRT_OK;
   BRT_REQUIRE(dst_data != nullptr && route_indices != nullptr && loads != nullptr,
               "null pointer argument");
@@ -1139,7 +1015,6 @@ BRT_API int brt_combine_with_records(
   a.dst = dst_data;
   a.gates = gates;
   a.indices = route_indices;
-  a.records = static_cast<const uint2*>(route_records);
   a.loads = loads;
   a.old_tags = nullptr;
   a.new_tags = nullptr;

@@ -265,7 +265,6 @@ struct MoveArgs {
   void* dst;
   const void* gates;
   const int* indices;
-  const uint2* records = nullptr;  // kRecordRoutes per cell (see common.cuh), or none
   const int* loads;
   const int* old_tags;       // dispatch only
   int* new_tags;             // dispatch only
@@ -372,20 +371,6 @@ __device__ __forceinline__ int build_routes(const MoveArgs& a, int64_t cell,
     }
   }
   return count;
-}
-
-// The same from a cell's route record: lane k < kRecordRoutes holds its k-th (path, seat).
-// Returns the number of kept routes, `slot` = where this lane's one went (-1: nowhere); the rows
-// are in slots[].row, the gates are for the caller to bring.
-__device__ __forceinline__ int record_routes(uint2 mine, const int* s_loads, const int* s_base,
-                                             RouteSlot* slots, int lane, int& path, int& slot) {
-  path = (int)(mine.x & (unsigned)(kRecordMore - 1));
-  const int seat = (int)mine.y;
-  const bool keep = lane < kRecordRoutes && seat > 0 && seat <= s_loads[path];
-  const unsigned kept = __ballot_sync(0xffffffffu, keep);
-  slot = keep ? __popc(kept & ((1u << lane) - 1u)) : -1;
-  if (keep) slots[slot].row = s_base[path] + seat - 1;
-  return __popc(kept);
 }
 
 // The items of a warp in a grid whose CTAs own kWarps * turns consecutive ones each, in order:
@@ -513,14 +498,6 @@ __device__ __forceinline__ float gate_at(const void* gates, int64_t at) {
 struct alignas(16) FoldStage {
   uint4 rows[kMaxRoutes][kFoldVecs];
   RouteSlot route[kMaxRoutes];
-  int count;
-  int pad[3];
-};
-
-// The same with room for all the routes of a record.
-struct alignas(16) RecordFoldStage {
-  uint4 rows[kMaxRoutes][kFoldVecs];
-  RouteSlot route[kRecordRoutes];
   int count;
   int pad[3];
 };

@@ -93,59 +93,6 @@ BRT_API int brt_generate_indices_and_loads(const int32_t* hot_mask, int32_t* ind
 /*
  * No counterpart in the reference.
  *
- * Route records: beside the seat indices the single-launch index scan can leave, per cell, its
- * first four routes as int32 pairs (path, seat) in ascending path order, seat 0 where there
- * are fewer; 0x40000000 set in the first path says that the record does not hold all routes
- * of the cell.  brt_dispatch_with_records and brt_combine_with_records read these 32 bytes per
- * cell in place of its rows of route_indices (and of gates).
- *
- * brt_route_record_bytes   the size of the records of such a mask (16-byte aligned device
- *                          memory), 0 when its scan leaves none (less than 2^21 elements, up
- *                          to 16 paths, where the index row is hardly longer, over 256, or a
- *                          mask that is too large for the single-launch scan): pass no
- *                          records then
- * brt_stream_capture_id    the id of the capture that `stream` takes part in, 0 when there is
- *                          none, UINT64_MAX when it cannot be told.  Records belong to the capture
- *                          they were made in: a graph that reads records made outside
- *                          it would not see an index tensor edited between two replays
- * The entry points are those without `records` in their names plus that argument (may be null).
- */
-BRT_API size_t brt_route_record_bytes(int64_t cell_num, int path_num);
-BRT_API uint64_t brt_stream_capture_id(void* stream);
-BRT_API int brt_generate_indices_loads_records(
-    const int32_t* hot_mask, int32_t* indices, int32_t* loads, int32_t* path_counts,
-    void* route_records, int64_t cell_num, int path_num, const int32_t* supported_capacities,
-    int supported_capacity_num, int capacity_padding, int path_wise_padding, int is_tag_index,
-    void* scratch, size_t scratch_bytes, void* stream);
-BRT_API int brt_throttle_and_generate_records(
-    const int32_t* hot_mask, int32_t* indices, int32_t* loads, int32_t* path_counts,
-    void* route_records, int32_t* prefix, const int32_t* threshold, int32_t* throttled_mask,
-    int64_t cell_num, int path_num, const int32_t* supported_capacities,
-    int supported_capacity_num, int capacity_padding, int path_wise_padding, void* scratch,
-    size_t scratch_bytes, void* stream);
-BRT_API int brt_route_scores_records(
-    const float* scores, int64_t cell_num, int path_num, int decision, int top_k, float threshold,
-    int residual_path, int output, int32_t* out, int32_t* loads, int32_t* path_counts,
-    void* route_records, const int32_t* capacities, int capacity_num, int capacity_padding,
-    int path_wise_padding, int32_t* prefix, const int32_t* throttle_capacity, float* gates_out,
-    int32_t* mask_out, void* scratch, size_t scratch_bytes, void* stream);
-/* route_records must belong to route_indices: made by the same call, with neither changed
- * since. */
-BRT_API int brt_dispatch_with_records(
-    const void* src_data, void* dst_data, const void* gates, const int32_t* route_indices,
-    const void* route_records, const int32_t* loads, const int32_t* old_tags, int32_t* new_tags,
-    int64_t cell_num, int64_t cell_size, int path_num, int32_t max_path_load, int64_t total_rows,
-    int is_1d_routing, int is_tag_index, int dtype, const int32_t* dense_counts, void* scratch,
-    size_t scratch_bytes, void* stream);
-BRT_API int brt_combine_with_records(
-    const void* src_data, void* dst_data, const void* gates, const int32_t* route_indices,
-    const void* route_records, const int32_t* loads, int64_t cell_num, int64_t cell_size,
-    int path_num, int32_t max_path_load, int is_residual, int dtype, int gates_dtype,
-    void* stream);
-
-/*
- * No counterpart in the reference.
- *
  * Same result as brt_generate_indices_and_loads, for callers that are not allowed to
  * obtain device memory themselves and therefore cannot supply the scratch buffer: code
  * running under a memory planner that owns the whole device heap, or a plugin host that
