@@ -1236,28 +1236,30 @@ __device__ __forceinline__ unsigned long long status_peek(const unsigned long lo
   return w;
 }
 
-// Shared memory of the chained kernel, in ints.  The base seats of every 32-cell group take
-// the place of the staged tiles once those are packed.
+// Shared memory of the chained kernel, in ints.  The base seats of the 32-cell groups take the
+// place of the staged tiles once those are packed, for as many tiles at a time as fit there
+// (64 and more of 16-byte rows).
 struct ChainSmem {
-  int* sum;             // [ec] column sums of the run
-  int* extra;           // [ec] what values other than 0/1 add to them
-  int* flag;            // [8]  flag[0]: such a value was seen
-  int* before;          // [ec] column sums of the earlier runs
-  int* thr;             // [ec]
-  int* routed;          // [tiles rounded up to 4] elements routed per tile
-  unsigned* row_words;  // [kTileThreads] picks of a gated tile
-  int* bits;            // [tiles][rg][ec] column bit words
-  int* stages;          // 2 x [rg * 32][pitch]
+  int* sum;               // [ec] column sums of the run
+  int* extra;             // [ec] what values other than 0/1 add to them
+  int* flag;              // [8]  flag[0]: such a value was seen; flag[2..3]: see routed()
+  int* before;            // [ec] column sums of the earlier runs
+  int* thr;               // [ec]
+  unsigned char* sparse;  // [tiles rounded up to 16] the tile is zeroed and scattered into
+  unsigned* row_words;    // [kTileThreads] picks of a gated tile
+  int* bits;              // [tiles][rg][ec] column bit words
+  int* stages;            // 2 x [rg * 32][pitch]
   int stage_ints;
-  int* base;            // [tiles][rg][ec], over the stages
+  int* base;              // [window][rg][ec], over the stages
   __device__ __forceinline__ int* stage(int i) const { return stages + (i & 1) * stage_ints; }
+  // elements routed in tile i, for as long as it is packed and zeroed
+  __device__ __forceinline__ int* routed(int i) const { return flag + 2 + (i & 1); }
 };
 __host__ __device__ inline int round4(int n) { return (n + 3) & ~3; }
+__host__ __device__ inline int sparse_ints(int tiles) { return (tiles + 15) / 16 * 4; }
 __host__ __device__ inline size_t chain_smem_ints(int ec, int rg, int pitch, int tiles) {
-  const size_t words = (size_t)tiles * rg * ec;
-  const size_t stages = 2 * (size_t)rg * kGroupRows * pitch;
-  return 4 * (size_t)ec + 8 + round4(tiles) + kTileThreads + words +
-         (stages > words ? stages : words);
+  return 4 * (size_t)ec + 8 + sparse_ints(tiles) + kTileThreads + (size_t)tiles * rg * ec +
+         2 * (size_t)rg * kGroupRows * pitch;
 }
 __device__ __forceinline__ ChainSmem carve_chain_smem(int* s, int ec, int rg, int pitch,
                                                       int tiles) {
@@ -1267,9 +1269,10 @@ __device__ __forceinline__ ChainSmem carve_chain_smem(int* s, int ec, int rg, in
   m.flag = s + 2 * ec;
   m.before = m.flag + 8;
   m.thr = m.before + ec;
-  m.routed = m.thr + ec;
-  m.row_words = reinterpret_cast<unsigned*>(m.routed + round4(tiles));
-  m.bits = m.routed + round4(tiles) + kTileThreads;
+  int* const after = m.thr + ec + sparse_ints(tiles);
+  m.sparse = reinterpret_cast<unsigned char*>(m.thr + ec);
+  m.row_words = reinterpret_cast<unsigned*>(after);
+  m.bits = after + kTileThreads;
   m.stages = m.bits + tiles * rg * ec;
   m.stage_ints = rg * kGroupRows * pitch;
   m.base = m.stages;
@@ -1512,8 +1515,7 @@ __global__ void __launch_bounds__(kTileThreads, 2) index_chain_kernel(const Chai
   const bool alone = c.ranges == 1;
   if (!alone && tid == 0) s_ticket = atomicAdd(c.ticket, 1);
   const ChainSmem sm = carve_chain_smem(s_dyn, a.ec, a.rg, a.pitch, c.tiles_per_cta);
-  for (int i = tid; i < 2 * a.ec + 1; i += kTileThreads) sm.sum[i] = 0;
-  for (int i = tid; i < c.tiles_per_cta; i += kTileThreads) sm.routed[i] = 0;
+  for (int i = tid; i < 2 * a.ec + 8; i += kTileThreads) sm.sum[i] = 0;
   __syncthreads();
   const int ticket = alone ? (int)blockIdx.x : s_ticket + c.first_ticket;
   const int range = ticket / a.chunks;
@@ -1562,11 +1564,16 @@ __global__ void __launch_bounds__(kTileThreads, 2) index_chain_kernel(const Chai
     x.tile = t;
     int* const bits = sm.bits + i * words_per_tile;
     if constexpr (GATED)  // the staged tile holds scores
-      gate_words(x, sm.stage(i), bits, sm.sum, sm.routed + i, sm.row_words, c.gate);
+      gate_words(x, sm.stage(i), bits, sm.sum, sm.routed(i), sm.row_words, c.gate);
     else
-      pack_words<V>(x, cols, sm, sm.stage(i), bits, sm.routed + i);
+      pack_words<V>(x, cols, sm, sm.stage(i), bits, sm.routed(i));
+    const bool sparse = *sm.routed(i) * kSparse <= rows_of(x) * cols;
+    if (tid == 0) {
+      sm.sparse[i] = sparse ? 1 : 0;
+      *sm.routed(i + 1) = 0;  // last read before this tile's first barrier, next added to after one
+    }
     // (the tag output is zeroed as a whole before the launch: its rows are not the tile's)
-    if (MODE != Mode::kTag && sm.routed[i] * kSparse <= rows_of(x) * cols) {
+    if (MODE != Mode::kTag && sparse) {
       zero_tile<V>(x, cols, a.out);
       if (a.mask_out != nullptr) zero_tile<V>(x, cols, a.mask_out);
     }
@@ -1668,35 +1675,40 @@ __global__ void __launch_bounds__(kTileThreads, 2) index_chain_kernel(const Chai
     }
     return;
   }
-  const int tiles = (int)(tile1 - tile0);
-  const int groups = tiles * a.rg;
-  if (tid < cols) {  // base seats of every group of the run, one path per thread
-    for (int g0 = 0; g0 < groups; g0 += 8) {
-      int n[8];
+  const int window = 2 * sm.stage_ints / words_per_tile;  // tiles whose base seats fit
+  for (int64_t t0 = tile0; t0 < tile1; t0 += window) {
+    if (t0 != tile0) __syncthreads();  // the base seats of the tiles before are no longer read
+    const int i0 = (int)(t0 - tile0);
+    const int tiles = (int)min((int64_t)window, tile1 - t0);
+    const int groups = tiles * a.rg;
+    const int* const bits = sm.bits + i0 * words_per_tile;
+    if (tid < cols) {  // base seats of these groups, one path per thread
+      for (int g0 = 0; g0 < groups; g0 += 8) {
+        int n[8];
 #pragma unroll
-      for (int u = 0; u < 8; u++)
-        n[u] = g0 + u < groups ? __popc(static_cast<uint32_t>(sm.bits[(g0 + u) * a.ec + tid])) : 0;
+        for (int u = 0; u < 8; u++)
+          n[u] = g0 + u < groups ? __popc(static_cast<uint32_t>(bits[(g0 + u) * a.ec + tid])) : 0;
 #pragma unroll
-      for (int u = 0; u < 8; u++) {
-        if (g0 + u < groups) sm.base[(g0 + u) * a.ec + tid] = run;
-        run += n[u];
+        for (int u = 0; u < 8; u++) {
+          if (g0 + u < groups) sm.base[(g0 + u) * a.ec + tid] = run;
+          run += n[u];
+        }
       }
     }
-  }
-  __syncthreads();
-  for (int g = tid >> 5; g < groups; g += kTileWarps) {
-    const int i = g / a.rg;
-    x.tile = tile0 + i;
-    if (MODE == Mode::kTag || sm.routed[i] * kSparse <= rows_of(x) * cols)  // warp-uniform
-      write_routes<MODE>(c, x, cols, tile0 * a.rg + g, sm.bits + g * a.ec, sm.base + g * a.ec,
-                         sm.thr);
-  }
-  if constexpr (MODE != Mode::kTag) {
-    for (int i = 0; i < tiles; i++) {
-      x.tile = tile0 + i;
-      if (sm.routed[i] * kSparse > rows_of(x) * cols)
-        write_tile<MODE, V>(x, cols, sm.bits + i * words_per_tile, sm.base + i * words_per_tile,
-                            sm.thr, a.out, a.mask_out);
+    __syncthreads();
+    for (int g = tid >> 5; g < groups; g += kTileWarps) {
+      const int i = g / a.rg;
+      x.tile = t0 + i;
+      if (MODE == Mode::kTag || sm.sparse[i0 + i] != 0)  // warp-uniform
+        write_routes<MODE>(c, x, cols, t0 * a.rg + g, bits + g * a.ec, sm.base + g * a.ec, sm.thr);
+    }
+    if constexpr (MODE != Mode::kTag) {
+      for (int i = 0; i < tiles; i++) {
+        x.tile = t0 + i;
+        if (sm.sparse[i0 + i] == 0)
+          write_tile<MODE, V>(x, cols, bits + i * words_per_tile, sm.base + i * words_per_tile,
+                              sm.thr, a.out, a.mask_out);
+      }
     }
   }
 }
@@ -1709,7 +1721,8 @@ size_t tiled_scratch_bytes(int64_t cell_num, int path_num) {
 }
 
 constexpr int kChainCtasPerSm = 2;
-constexpr size_t kChainSmemLimit = 110 * 1024;
+// two CTAs of an SM's 228 KB, 1 KB and the kernel's static words each aside
+constexpr size_t kChainSmemLimit = 113 * 1024 - 64;
 
 // A run-out look-back wait is reported through one word of host-mapped memory per process:
 // kernels write it, the host reads it without synchronising (brt_index_status).  The word is

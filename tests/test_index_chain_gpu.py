@@ -187,3 +187,43 @@ def test_seats_of_an_array_that_is_only_4_byte_aligned_are_refused():
                  (score.data_ptr(), good, bad)):
         assert call(*args) == 4  # BRT_ERR_UNSUPPORTED, nothing is launched
     assert not out.cpu().any()
+
+
+# The largest masks of these path counts whose bit words fit a CTA's shared memory on 148 SMs when
+# the base seats of a few tiles at a time are all that is kept beside them.
+@pytest.mark.parametrize("cells,paths", [(56756224, 4), (10381312, 16), (719872, 192),
+                                         (184704, 260)])
+def test_the_largest_masks_of_one_launch(cells, paths):
+    from brainstorm_b200 import _lib
+    from brainstorm_b200._C import router as R
+
+    g = torch.Generator(device="cuda").manual_seed(paths)
+    score = torch.rand((cells, paths), generator=g, device="cuda")
+    score[cells // 3:cells // 2] = score[cells // 3:cells // 2].bernoulli_()  # dense tiles below
+    best = score == score.max(dim=1, keepdim=True).values
+    first = (best.cumsum(dim=1, dtype=torch.int32) == 1) & best
+    del best
+
+    def seats_of(mask):
+        seats = mask.t().contiguous().cumsum(dim=1, dtype=torch.int32)
+        loads = seats[:, -1].contiguous()
+        return seats.t().contiguous().mul_(mask), loads
+
+    if paths <= 256:
+        want, loads = seats_of(first.to(torch.int32))
+        got, got_loads = R.route_scores(score, "topk", 1, output="seat_indices")
+        assert torch.equal(got, want) and torch.equal(got_loads, loads)
+        del got, want
+    mask = (first | (score >= 0.95)).to(torch.int32)
+    del first, score
+    want, loads = seats_of(mask)
+    before = _lib.query("brt_kernel_launch_count")
+    got, got_loads = R.generate_indices_and_loads(mask)
+    assert _lib.query("brt_kernel_launch_count") == before + 1
+    assert torch.equal(got, want) and torch.equal(got_loads, loads)
+    del got
+    limit = torch.full((paths,), cells // paths, dtype=torch.int32, device="cuda")
+    prefix = torch.zeros_like(limit)
+    got = R.throttle_hotmask(mask, prefix, limit)[0]
+    assert torch.equal(got, ((want > 0) & (want <= limit)).to(torch.int32))
+    assert torch.equal(prefix, torch.minimum(loads, limit))
