@@ -6,7 +6,9 @@
 // functions do the same for the calls that programs make all the time - contiguous tensors of
 // the right types on the current device, sizes known - and return None for any other
 // call, before anything has been enqueued: the Python operator then takes it and does the
-// checking and the explaining.  They call the same entry points of the C library.
+// checking and the explaining.  They call the same entry points of the C library, and like the
+// foreign calls they stand for they let other Python threads run meanwhile: an allocation may
+// synchronise, a launch waits while the queue of the stream is full.
 #include <Python.h>
 
 #include <ATen/core/Tensor.h>
@@ -66,6 +68,24 @@ bool same_device(const at::Tensor& a, const at::Tensor* b) {
   return b == nullptr || a.get_device() == b->get_device();
 }
 
+// Other Python threads run while this lives.  Everything that touches a Python object comes before
+// or after; what is made inside (tensors that no Python object wraps yet) needs no lock.
+struct Unlocked {
+  PyThreadState* const state = PyEval_SaveThread();
+  ~Unlocked() { PyEval_RestoreThread(state); }
+};
+// The addresses of a call's tensors, and the memory behind them kept until the call has been
+// enqueued: meanwhile another thread may drop a tensor or give it other memory.
+struct Memory {
+  c10::SmallVector<c10::Storage, 8> held;
+  void* of(const at::Tensor* t) {
+    if (t == nullptr) return nullptr;
+    held.push_back(t->storage());
+    return t->data_ptr();
+  }
+  int32_t* ints(const at::Tensor* t) { return static_cast<int32_t*>(of(t)); }
+};
+
 // The note of an index operator on the tensor it returns, see _C/router.py.
 bool mark(PyObject* indices, const at::Tensor& counts) {
   PyObject* c = THPVariable_Wrap(counts);
@@ -80,27 +100,28 @@ PyObject* attribute(PyObject* o, PyObject* name) {
   return v;
 }
 
-// The dense counts noted on `indices` (kept alive by it), or null.
-const int32_t* dense_counts(PyObject* indices, int64_t paths) {
+// The dense counts noted on `indices`, or null.
+const int32_t* dense_counts(PyObject* indices, int64_t paths, Memory& memory) {
   PyObject* note = attribute(indices, g_dense);
   if (note == nullptr) return nullptr;
   const at::Tensor* t = plain(note);
   const bool ok = int32c(t, 1) && t->numel() == paths &&
                   same_device(THPVariable_Unpack(indices), t);
-  const int32_t* p = ok ? static_cast<const int32_t*>(t->data_ptr()) : nullptr;
+  const int32_t* const p = ok ? memory.ints(t) : nullptr;
   Py_DECREF(note);
   return p;
 }
+
 struct Caps {
   const int32_t* ptr = nullptr;
   int num = 0;
   bool ok = true;
-  Caps(PyObject* o, const at::Tensor& like) {
+  Caps(PyObject* o, const at::Tensor& like, Memory& memory) {
     if (o == Py_None) return;
     const at::Tensor* t = plain(o);
     ok = int32c(t, 1) && same_device(like, t);
     if (!ok) return;
-    ptr = static_cast<const int32_t*>(t->data_ptr());
+    ptr = memory.ints(t);
     num = (int)t->numel();
   }
 };
@@ -146,32 +167,38 @@ PyObject* scan(PyObject*, PyObject* const* a, Py_ssize_t n) {
           !same_device(*mask, threshold))
         return nullptr;
     }
-    const Caps caps(a[3], *mask);
+    Memory memory;
+    const Caps caps(a[3], *mask, memory);
     if (!caps.ok) return nullptr;
     const int cpad = truth(a[4]), pwise = truth(a[5]), with_mask = truth(a[6]);
     if (cpad < 0 || pwise < 0 || with_mask < 0) return nullptr;
     if (throttle && E % 4 != 0) return nullptr;  // takes two launches
     const Place p(*mask);
-    const at::Tensor indices = empty(mask->sizes(), at::kInt, p.device);
-    const at::Tensor both = empty({2, E}, at::kInt, p.device);
-    const at::Tensor loads = both.select(0, 0), counts = both.select(0, 1);
-    const at::Tensor throttled =
-        with_mask ? empty(mask->sizes(), at::kInt, p.device) : at::Tensor();
-    const int64_t bytes = (int64_t)brt_index_scratch_bytes(T, (int)E);
-    const at::Tensor scratch = empty({bytes}, at::kByte, p.device);
-    const auto m = static_cast<const int32_t*>(mask->data_ptr());
-    const auto out = static_cast<int32_t*>(indices.data_ptr());
-    const auto l = static_cast<int32_t*>(loads.data_ptr());
-    const auto c = static_cast<int32_t*>(counts.data_ptr());
-    const int rc =
-        throttle ? brt_throttle_and_generate_indices(
-                       m, out, l, c, static_cast<int32_t*>(prefix->data_ptr()),
-                       static_cast<const int32_t*>(threshold->data_ptr()),
-                       static_cast<int32_t*>(data_or_null(throttled)), T, (int)E, caps.ptr,
-                       caps.num, cpad, pwise, scratch.data_ptr(), (size_t)bytes, p.handle())
-                 : brt_generate_indices_and_loads(m, out, l, c, T, (int)E, caps.ptr, caps.num,
-                                                  cpad, pwise, 0, scratch.data_ptr(),
-                                                  (size_t)bytes, p.handle());
+    const int32_t* const m = memory.ints(mask);
+    int32_t* const before = memory.ints(prefix);
+    const int32_t* const limit = memory.ints(threshold);
+    at::Tensor indices, loads, counts, throttled;
+    int rc;
+    {
+      const Unlocked unlocked;
+      indices = empty({T, E}, at::kInt, p.device);
+      const at::Tensor both = empty({2, E}, at::kInt, p.device);
+      loads = both.select(0, 0);
+      counts = both.select(0, 1);
+      if (with_mask) throttled = empty({T, E}, at::kInt, p.device);
+      const int64_t bytes = (int64_t)brt_index_scratch_bytes(T, (int)E);
+      const at::Tensor scratch = empty({bytes}, at::kByte, p.device);
+      const auto out = static_cast<int32_t*>(indices.data_ptr());
+      const auto l = static_cast<int32_t*>(loads.data_ptr());
+      const auto c = static_cast<int32_t*>(counts.data_ptr());
+      rc = throttle ? brt_throttle_and_generate_indices(
+                          m, out, l, c, before, limit,
+                          static_cast<int32_t*>(data_or_null(throttled)), T, (int)E, caps.ptr,
+                          caps.num, cpad, pwise, scratch.data_ptr(), (size_t)bytes, p.handle())
+                    : brt_generate_indices_and_loads(m, out, l, c, T, (int)E, caps.ptr, caps.num,
+                                                     cpad, pwise, 0, scratch.data_ptr(),
+                                                     (size_t)bytes, p.handle());
+    }
     if (rc != BRT_OK) return nullptr;  // nothing was enqueued: the operator says why
     PyObject* i = THPVariable_Wrap(indices);
     if (i == nullptr || !mark(i, counts)) {
@@ -205,7 +232,8 @@ PyObject* route_scores(PyObject*, PyObject* const* a, Py_ssize_t n) {
       return nullptr;
     }
     if (top_k != (int)top_k || residual != (int)residual) return nullptr;
-    const Caps caps(a[6], *score);
+    Memory memory;
+    const Caps caps(a[6], *score, memory);
     const int cpad = truth(a[7]), pwise = truth(a[8]);
     const int with_gates = truth(a[11]), with_mask = truth(a[12]);
     if (cpad < 0 || pwise < 0 || with_gates < 0 || with_mask < 0) return nullptr;
@@ -224,23 +252,29 @@ PyObject* route_scores(PyObject*, PyObject* const* a, Py_ssize_t n) {
     }
     if (with_mask && !seats) return nullptr;
     const Place p(*score);
-    const at::Tensor out = empty(score->sizes(), at::kInt, p.device);
-    const at::Tensor both = empty({2, E}, at::kInt, p.device);
-    const at::Tensor loads = both.select(0, 0), counts = both.select(0, 1);
-    const at::Tensor gates =
-        with_gates ? empty(score->sizes(), at::kFloat, p.device) : at::Tensor();
-    const at::Tensor mask = with_mask ? empty(score->sizes(), at::kInt, p.device) : at::Tensor();
-    const int64_t bytes = (int64_t)brt_index_scratch_bytes(T, (int)E);
-    const at::Tensor scratch = empty({bytes}, at::kByte, p.device);
-    const int rc = brt_route_scores(
-        static_cast<const float*>(score->data_ptr()), T, (int)E, (int)decision, (int)top_k,
-        (float)threshold, (int)residual, (int)output, static_cast<int32_t*>(out.data_ptr()),
-        static_cast<int32_t*>(loads.data_ptr()),
-        seats ? static_cast<int32_t*>(counts.data_ptr()) : nullptr, caps.ptr, caps.num, cpad, pwise,
-        throttles ? static_cast<int32_t*>(prefix->data_ptr()) : nullptr,
-        throttles ? static_cast<const int32_t*>(limit->data_ptr()) : nullptr,
-        static_cast<float*>(data_or_null(gates)), static_cast<int32_t*>(data_or_null(mask)),
-        scratch.data_ptr(), (size_t)bytes, p.handle());
+    const auto s = static_cast<const float*>(memory.of(score));
+    int32_t* const before = memory.ints(prefix);
+    const int32_t* const room = memory.ints(limit);
+    at::Tensor out, loads, counts, gates, mask;
+    int rc;
+    {
+      const Unlocked unlocked;
+      out = empty({T, E}, at::kInt, p.device);
+      const at::Tensor both = empty({2, E}, at::kInt, p.device);
+      loads = both.select(0, 0);
+      counts = both.select(0, 1);
+      if (with_gates) gates = empty({T, E}, at::kFloat, p.device);
+      if (with_mask) mask = empty({T, E}, at::kInt, p.device);
+      const int64_t bytes = (int64_t)brt_index_scratch_bytes(T, (int)E);
+      const at::Tensor scratch = empty({bytes}, at::kByte, p.device);
+      rc = brt_route_scores(
+          s, T, (int)E, (int)decision, (int)top_k, (float)threshold, (int)residual, (int)output,
+          static_cast<int32_t*>(out.data_ptr()), static_cast<int32_t*>(loads.data_ptr()),
+          seats ? static_cast<int32_t*>(counts.data_ptr()) : nullptr, caps.ptr, caps.num, cpad,
+          pwise, before, room, static_cast<float*>(data_or_null(gates)),
+          static_cast<int32_t*>(data_or_null(mask)), scratch.data_ptr(), (size_t)bytes,
+          p.handle());
+    }
     if (rc != BRT_OK) return nullptr;
     PyObject* o = THPVariable_Wrap(out);
     if (o == nullptr || (seats && !mark(o, counts))) {
@@ -282,17 +316,26 @@ PyObject* dispatch(PyObject*, PyObject* const* a, Py_ssize_t n) {
       return nullptr;
     }
     if (mpl < 0 || mpl > 0x7fffffffLL || total < 0) return nullptr;
-    const int32_t* counts = dense_counts(a[1], E);
+    Memory memory;
+    const int32_t* counts = dense_counts(a[1], E, memory);
     if (counts == nullptr) return nullptr;
     const Place p(*x);
     c10::SmallVector<int64_t, 6> shape(x->sizes().begin(), x->sizes().end());
     shape[0] = total;
-    const at::Tensor out = empty(shape, x->scalar_type(), p.device);
-    const int rc = brt_dispatch_with_indices_and_loads(
-        x->data_ptr(), out.data_ptr(), gates != nullptr ? gates->data_ptr() : nullptr,
-        static_cast<const int32_t*>(indices->data_ptr()),
-        static_cast<const int32_t*>(loads->data_ptr()), nullptr, nullptr, T, cell, (int)E,
-        (int)mpl, total, 1, 0, dtype, counts, nullptr, 0, p.handle());
+    const auto type = x->scalar_type();
+    const void* const src = memory.of(x);
+    const void* const g = memory.of(gates);
+    const int32_t* const at_rows = memory.ints(indices);
+    const int32_t* const l = memory.ints(loads);
+    at::Tensor out;
+    int rc;
+    {
+      const Unlocked unlocked;
+      out = empty(shape, type, p.device);
+      rc = brt_dispatch_with_indices_and_loads(src, out.data_ptr(), g, at_rows, l, nullptr, nullptr,
+                                               T, cell, (int)E, (int)mpl, total, 1, 0, dtype,
+                                               counts, nullptr, 0, p.handle());
+    }
     if (rc != BRT_OK) return nullptr;
     return THPVariable_Wrap(out);
   });
@@ -333,19 +376,28 @@ PyObject* combine(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (padded < 0) return nullptr;
     const int64_t mpl = padded ? rows / E : 0;
     if (mpl > 0x7fffffffLL) return nullptr;
+    Memory memory;
     const Place p(*x);
+    c10::SmallVector<int64_t, 6> shape(x->sizes().begin(), x->sizes().end());
+    shape[0] = T;
+    const auto type = x->scalar_type();
+    const void* const src = memory.of(x);
+    const void* const g = memory.of(gates);
+    const int32_t* const at_rows = memory.ints(indices);
+    const int32_t* const l = memory.ints(loads);
+    void* dst = memory.of(residual);
     at::Tensor out;
-    if (residual == nullptr) {
-      c10::SmallVector<int64_t, 6> shape(x->sizes().begin(), x->sizes().end());
-      shape[0] = T;
-      out = empty(shape, x->scalar_type(), p.device);
+    int rc;
+    {
+      const Unlocked unlocked;
+      if (residual == nullptr) {
+        out = empty(shape, type, p.device);
+        dst = out.data_ptr();
+      }
+      rc = brt_combine_with_indices_and_loads(src, dst, g, at_rows, l, T, cell, (int)E,
+                                              (int32_t)mpl, residual != nullptr, dtype, gate_type,
+                                              p.handle());
     }
-    const int rc = brt_combine_with_indices_and_loads(
-        x->data_ptr(), residual != nullptr ? residual->data_ptr() : out.data_ptr(),
-        gates != nullptr ? gates->data_ptr() : nullptr,
-        static_cast<const int32_t*>(indices->data_ptr()),
-        static_cast<const int32_t*>(loads->data_ptr()), T, cell, (int)E, (int32_t)mpl,
-        residual != nullptr, dtype, gate_type, p.handle());
     if (rc != BRT_OK) return nullptr;
     return residual != nullptr ? Py_NewRef(a[4]) : THPVariable_Wrap(out);
   });

@@ -167,3 +167,52 @@ def test_packed_dispatch_takes_loads_of_any_shape(paths):
     for shape in shapes:
         (got,) = R.dispatch_with_indices_and_loads(x, indices, loads.reshape(shape))
         assert torch.equal(got, want)
+
+
+def test_other_threads_run_while_a_launch_waits():
+    """With the stream busy and its queue full an operator waits; the process must not."""
+    import threading
+    import time
+
+    from brainstorm_b200._C import router as R
+
+    mask = masks(64, 32)["plain"]
+    indices, loads = R.generate_indices_and_loads(mask)
+    x = torch.randn((64, 16), device="cuda")
+    slot = int(loads.max())
+
+    def step():
+        R.generate_indices_and_loads(mask)
+        (rows,) = R.dispatch_with_indices_and_loads(x, indices, loads, None, False, None, True,
+                                                    slot)
+        R.combine_with_indices_and_loads(rows, indices, loads, None, None, True)
+        R.route_scores(x, "topk", 1, output="seat_indices")
+
+    step()
+    torch.cuda.synchronize()
+    ticks, stop = [], threading.Event()
+
+    def tick():
+        while not stop.is_set():
+            ticks.append(time.perf_counter())
+            time.sleep(0.001)
+
+    thread = threading.Thread(target=tick)
+    thread.start()
+    longest = 0.0
+    try:
+        torch.cuda._sleep(2_000_000_000)  # about a second
+        begin = time.perf_counter()
+        while time.perf_counter() - begin < 2.0:  # more launches than any queue holds
+            at = time.perf_counter()
+            step()
+            longest = max(longest, time.perf_counter() - at)
+            if longest > 0.3:
+                break
+    finally:
+        stop.set()
+        thread.join()
+    torch.cuda.synchronize()
+    assert longest > 0.3, "no launch had to wait"
+    gaps = [b - a for a, b in zip(ticks, ticks[1:])]
+    assert max(gaps) < 0.5 * longest
