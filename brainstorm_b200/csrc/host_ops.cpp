@@ -17,6 +17,7 @@
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include "../../include/brt_b200.h"
@@ -133,14 +134,15 @@ int truth(PyObject* o) {
   return v;
 }
 
+// Errors keep the kind that torch gives them in Python: torch.OutOfMemoryError above all.
 template <typename F>
 PyObject* guarded(F&& body) {
   try {
     PyObject* r = body();
     if (r != nullptr || PyErr_Occurred()) return r;
     Py_RETURN_NONE;
-  } catch (const std::exception& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
+  } catch (const std::exception&) {
+    torch::translate_exception_to_python(std::current_exception());
   } catch (...) {
     PyErr_SetString(PyExc_RuntimeError, "unknown error in a router operator");
   }

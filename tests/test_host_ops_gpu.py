@@ -216,3 +216,41 @@ def test_other_threads_run_while_a_launch_waits():
     assert longest > 0.3, "no launch had to wait"
     gaps = [b - a for a, b in zip(ticks, ticks[1:])]
     assert max(gaps) < 0.5 * longest
+
+
+def test_running_out_of_memory_keeps_its_kind():
+    """What a program catches to free something and try again."""
+    from brainstorm_b200._C import router as R
+
+    cells = torch.arange(1 << 18, device="cuda")
+    mask = torch.zeros((1 << 18, 64), dtype=torch.int32, device="cuda")
+    mask[cells, cells % 64] = 1  # 4096 cells for every path
+    score = torch.rand((1 << 18, 64), device="cuda")
+    limit = torch.full((64,), 5, dtype=torch.int32, device="cuda")
+    indices, loads = R.generate_indices_and_loads(mask)
+    x = torch.randn((1 << 18, 64), device="cuda")
+    slot = 1 << 18
+    rows = torch.randn((64 * 4096, 64), device="cuda")
+    calls = [
+        lambda: R.generate_indices_and_loads(mask),
+        lambda: R.throttle_and_generate_indices(mask, torch.zeros_like(limit), limit),
+        lambda: R.route_scores(score, "topk", 1, output="seat_indices", with_gates=True),
+        lambda: R.dispatch_with_indices_and_loads(x, indices, loads, None, False, None, True, slot),
+        lambda: R.combine_with_indices_and_loads(rows, indices, loads, None, None, True),
+    ]
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    try:  # nothing beyond what is allocated now
+        torch.cuda.set_per_process_memory_fraction(
+            torch.cuda.memory_reserved() / torch.cuda.mem_get_info()[1])
+        for call in calls:
+            with pytest.raises(torch.OutOfMemoryError):
+                held = []
+                for _ in range(8):  # what the reserved blocks still have room for
+                    held.append(call())
+            held = None
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    for call in calls[:3]:
+        call()
+    torch.cuda.synchronize()
