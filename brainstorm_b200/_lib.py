@@ -1,10 +1,12 @@
 """ctypes binding of ``libbrt_b200.so`` (the C ABI declared in ``include/brt_b200.h``).
 
 There is no fallback: if the library is missing or a call fails, a ``RuntimeError`` says
-so.  Pointers are passed as integers (``tensor.data_ptr()``), streams as
+so.  (The native host side of the hot operators is an extra: without it their Python does the same
+calls.)  Pointers are passed as integers (``tensor.data_ptr()``), streams as
 ``torch.cuda.current_stream().cuda_stream``.
 """
 import ctypes
+import warnings
 from pathlib import Path
 
 _PKG = Path(__file__).resolve().parent
@@ -139,17 +141,37 @@ def load():
 _host = None
 
 
+class _DeclinesAll:
+    """Stands in for the native host side where there is none: the Python operators take all."""
+
+    @staticmethod
+    def scan(*args):
+        return None
+
+    route_scores = dispatch = combine = scan
+
+
 def host_ops():
-    """The native host side of the hot operators (``csrc/host_ops.cpp``); raises if missing."""
+    """The native host side of the hot operators (``csrc/host_ops.cpp``).  It is built against one
+    torch; where it is missing or belongs to another one, a warning says so (once) and the Python
+    operators, which call the same library, take every call."""
     global _host
     if _host is None:
+        import torch
+
         load()
         try:
             from . import _host_ops
+
+            built_for, here = _host_ops.torch_version, torch.__version__.split("+")[0]
+            problem = None if built_for == here else f"is built for torch {built_for}, not {here}"
         except ImportError as exc:
-            raise BrtError(f"{_PKG / '_host_ops.so'} does not load ({exc}): build it with "
-                           "`python -m brainstorm_b200.build`") from None
-        _host = _host_ops
+            problem = f"does not load ({exc})"
+        if problem is not None:
+            warnings.warn(f"{_PKG / '_host_ops.so'} {problem}: the router operators take 5 to 12 us "
+                          "longer each; build it with `python -m brainstorm_b200.build`",
+                          RuntimeWarning, stacklevel=3)
+        _host = _host_ops if problem is None else _DeclinesAll()
     return _host
 
 

@@ -5,7 +5,8 @@
 
 The library has no Python or torch dependency; ``brainstorm_b200._lib`` loads it
 with ctypes.  nvcc cross-compiles without a GPU.  ``_host_ops.so``, the native host side of the
-router's hot operators, is a small extension module on top of it (g++, torch's headers).
+router's hot operators, is a small extension module on top of it (g++, torch's headers); it is left
+out where torch is not installed, and built again when torch has changed.
 """
 import os
 import shutil
@@ -21,6 +22,7 @@ LIB = PKG / "libbrt_b200.so"
 HOST_SRC = CSRC / "host_ops.cpp"
 HOST_LIB = PKG / "_host_ops.so"
 OBJ_DIR = PKG / "build"
+HOST_STAMP = OBJ_DIR / "host_ops.torch"  # the torch that HOST_LIB was built against
 
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC,-fvisibility=hidden",
@@ -68,15 +70,25 @@ def _stale() -> bool:
     return LIB.stat().st_mtime < newest
 
 
-def build_host(force: bool = False) -> Path:
-    if not force and HOST_LIB.exists() and \
-            HOST_LIB.stat().st_mtime >= max(p.stat().st_mtime for p in
-                                            [HOST_SRC, LIB, *INCLUDE.glob("*.h")]):
-        return HOST_LIB
+def _host_stale(torch_version: str) -> bool:
+    if not HOST_LIB.exists() or not HOST_STAMP.exists() or \
+            HOST_STAMP.read_text() != torch_version:
+        return True
+    newest = max(p.stat().st_mtime for p in [HOST_SRC, LIB, *INCLUDE.glob("*.h")])
+    return HOST_LIB.stat().st_mtime < newest
+
+
+def build_host(force: bool = False):
+    """The path of the extension module, or None without torch."""
     import sysconfig
 
-    import torch
-
+    try:
+        import torch
+    except ImportError:
+        print("[build] no torch: the library is built without _host_ops.so", file=sys.stderr)
+        return None
+    if not force and not _host_stale(torch.__version__):
+        return HOST_LIB
     base = Path(torch.__file__).resolve().parent
     cuda = Path(_nvcc()).resolve().parent.parent
     cxx = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else "g++"
@@ -90,6 +102,8 @@ def build_host(force: bool = False) -> Path:
     proc = subprocess.run(cmd, capture_output=True, text=True)
     if proc.returncode != 0:
         raise RuntimeError(f"$ {' '.join(cmd)}\n{proc.stdout}\n{proc.stderr}")
+    OBJ_DIR.mkdir(exist_ok=True)
+    HOST_STAMP.write_text(torch.__version__)
     return HOST_LIB
 
 

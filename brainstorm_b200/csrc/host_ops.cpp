@@ -19,6 +19,7 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/version.h>
 
 #include "../../include/brt_b200.h"
 
@@ -421,5 +422,10 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host_ops", nullptr, -1, methods,
 
 PyMODINIT_FUNC PyInit__host_ops() {
   g_dense = PyUnicode_InternFromString("_brt_dense_counts");
-  return g_dense != nullptr ? PyModule_Create(&module) : nullptr;
+  PyObject* const m = g_dense != nullptr ? PyModule_Create(&module) : nullptr;
+  if (m != nullptr && PyModule_AddStringConstant(m, "torch_version", TORCH_VERSION) != 0) {
+    Py_DECREF(m);
+    return nullptr;
+  }
+  return m;
 }
