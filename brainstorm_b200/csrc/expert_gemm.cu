@@ -19,8 +19,9 @@
 // walks the list of (expert, row tile, feature tile) work items that it derives from `loads`
 // itself.  Roles inside a CTA (192 threads):
 //   warp 0     one elected lane issues the TMA loads (cp.async.bulk.tensor, 128B swizzle, no
-//              multicast) of its weight tile [128 x 64] and of its rows in boxes of 32 x 64 into
-//              a shared-memory ring; the bytes of both CTAs count on the first CTA's mbarrier;
+//              multicast) of its weight tile [128 x 64] and of its rows, in one box of 32, 64, 96
+//              or 128 x 64, into a shared-memory ring; the bytes of both CTAs count on the first
+//              CTA's mbarrier;
 //   warp 1     allocates tensor memory (2 accumulators of 128 lanes x 256 fp32 columns); one
 //              elected lane of the first CTA issues tcgen05.mma (K = 16) four times per k-block
 //              for the pair, releasing ring slots and publishing accumulators in both CTAs with

@@ -883,8 +883,7 @@ __device__ __forceinline__ void expand_binary(const TileCtx& x, const TileSmem& 
 }
 
 // Write the indices (or the throttled mask) of one tile from its bit words and the tile's
-// exclusive prefix in global memory.  `bits_in` != null: the words are first fetched from
-// global memory (separate-launch path); null: pack left them in shared memory.
+// exclusive prefix, both in global memory.
 template <Mode MODE>
 __device__ __forceinline__ void expand_tile(const TileCtx& x, const TileSmem& sm,
                                             const int* __restrict__ mask,
@@ -903,14 +902,12 @@ __device__ __forceinline__ void expand_tile(const TileCtx& x, const TileSmem& sm
     expand_general<MODE>(x, mask, run, out, threshold);
     return;
   }
-  if (bits_in != nullptr) {
-    for (int i = tid; i < x.rg * cols; i += kTileThreads) {
-      const int g = i / cols;
-      const int c = i - g * cols;
-      const int64_t group = x.tile * x.rg + g;
-      sm.bits[g * x.ec + c] =
-          group < num_groups ? static_cast<int>(bits_in[group * x.path_num + col0 + c]) : 0;
-    }
+  for (int i = tid; i < x.rg * cols; i += kTileThreads) {
+    const int g = i / cols;
+    const int c = i - g * cols;
+    const int64_t group = x.tile * x.rg + g;
+    sm.bits[g * x.ec + c] =
+        group < num_groups ? static_cast<int>(bits_in[group * x.path_num + col0 + c]) : 0;
   }
   if constexpr (MODE == Mode::kThrottle)
     for (int c = tid; c < cols; c += kTileThreads) sm.thr[c] = threshold[col0 + c];
@@ -977,9 +974,9 @@ __global__ void __launch_bounds__(kTileThreads) index_expand_tiled_kernel(const 
 }
 
 // ------------------------------------------------------------------------------- gate rows
-// Route decision of a staged tile of fp32 scores.  A warp (or a part of it, for narrow rows)
-// decides one row at a time and keeps the outcome as bits of the column words of the row's
-// 32-cell group; the words of all warps meet in shared memory, so no mask is ever written.
+// Route decision of a staged tile of fp32 scores.  One to eight neighbouring threads decide a row
+// and leave its picks as bits, 32 paths a word; a warp transposes the words of a 32-cell group
+// into the column words that `pack` makes of a mask, so no mask is ever written.
 //   kind 1: ones at the top_k largest scores of the row (python/brt/router/protocol/topk.py:
 //           26-31); equal scores go to the lower path index;
 //   kind 2: ones where score > threshold; a row without any goes to residual_path when that

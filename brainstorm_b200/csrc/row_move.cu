@@ -767,20 +767,18 @@ void launch_dispatch(const MoveArgs& a, bool is_tag, cudaStream_t st) {
   if (is_tag) {
     dispatch_tag_kernel<VB, DT, WEIGHTED, IS_1D>
         <<<grid_for_items(a.total_rows * a.pieces_per_row), kThreads, smem, st>>>(a), note_launch();
-  } else if (VB == 16 && IS_1D) {
-    if constexpr (VB == 16 && IS_1D) {
-      const size_t smem_async = sizeof(CopyStage) * kWarps * kStages + smem;
-      MoveArgs b = a;
-      const unsigned grid = plan_dispatch(b, WEIGHTED ? 3 : 4);
-      if (wide_rows(a.indices, a.gates, dtype_size(DT), a.path_num)) {
-        configure_smem<dispatch_seat_async_kernel<DT, WEIGHTED, 4>>(sizeof(CopyStage) * kWarps *
-                                                                    kStages);
-        dispatch_seat_async_kernel<DT, WEIGHTED, 4><<<grid, kThreads, smem_async, st>>>(b), note_launch();
-      } else {
-        configure_smem<dispatch_seat_async_kernel<DT, WEIGHTED, 1>>(sizeof(CopyStage) * kWarps *
-                                                                    kStages);
-        dispatch_seat_async_kernel<DT, WEIGHTED, 1><<<grid, kThreads, smem_async, st>>>(b), note_launch();
-      }
+  } else if constexpr (VB == 16 && IS_1D) {
+    const size_t smem_async = sizeof(CopyStage) * kWarps * kStages + smem;
+    MoveArgs b = a;
+    const unsigned grid = plan_dispatch(b, WEIGHTED ? 3 : 4);
+    if (wide_rows(a.indices, a.gates, dtype_size(DT), a.path_num)) {
+      configure_smem<dispatch_seat_async_kernel<DT, WEIGHTED, 4>>(sizeof(CopyStage) * kWarps *
+                                                                  kStages);
+      dispatch_seat_async_kernel<DT, WEIGHTED, 4><<<grid, kThreads, smem_async, st>>>(b), note_launch();
+    } else {
+      configure_smem<dispatch_seat_async_kernel<DT, WEIGHTED, 1>>(sizeof(CopyStage) * kWarps *
+                                                                  kStages);
+      dispatch_seat_async_kernel<DT, WEIGHTED, 1><<<grid, kThreads, smem_async, st>>>(b), note_launch();
     }
   } else {
     MoveArgs b = a;

@@ -1,7 +1,8 @@
 """The pipelined dispatch at the edges of the items a CTA owns: cell counts around a CTA's span and
 around one resident wave, rows of one and of several pieces, slots and capacities that leave rows to
-zero, up to more paths than a CTA has threads.  Against the same call on a copy of the indices,
-which takes the general kernels; whole bytes."""
+zero, up to more paths than a CTA has threads.  Rows, tags and zeros against torch, for the indices
+as the scan returned them and for a copy of them, whose empty rows a second launch zeroes; whole
+bytes (a weighted row is one product, rounded once)."""
 import pytest
 import torch
 
@@ -26,12 +27,21 @@ def test_spans(cells, paths, width, layout):
     padded = "slots" in layout
     x = torch.randn((cells, width), generator=g, device="cuda").bfloat16()
     gates = torch.rand((cells, paths), generator=g, device="cuda").bfloat16()
+    base = torch.arange(paths, device="cuda") * slot if padded else loads.cumsum(0) - loads
+    total = slot * paths if padded else int(loads.sum())
+    cell, path = mask.nonzero(as_tuple=True)
+    at = base[path] + mask.cumsum(dim=0)[cell, path] - 1
+    want_tags = torch.zeros(total, dtype=torch.int32, device="cuda")
+    want_tags[at] = (cell + 1).to(torch.int32)
     for weights in (None, gates):
-        for tags in (False, True):
-            got = R.dispatch_with_indices_and_loads(x, indices, loads, weights, tags, None, padded,
-                                                    slot if padded else 0)
-            want = R.dispatch_with_indices_and_loads(x, indices.clone(), loads, weights, tags,
-                                                     None, padded, slot if padded else 0)
-            for a, b in zip(got, want):
-                assert a.shape == b.shape
-                assert torch.equal(a.view(torch.uint8), b.view(torch.uint8))
+        want = torch.zeros((total, width), dtype=torch.bfloat16, device="cuda")
+        want[at] = x[cell] if weights is None else \
+            (x[cell].float() * weights[cell, path].float()[:, None]).bfloat16()
+        for idx in (indices, indices.clone()):
+            for tags in (False, True):
+                got = R.dispatch_with_indices_and_loads(x, idx, loads, weights, tags, None, padded,
+                                                        slot if padded else 0)
+                assert got[0].shape == want.shape
+                assert torch.equal(got[0].view(torch.int16), want.view(torch.int16))
+                if tags:
+                    assert torch.equal(got[1], want_tags)

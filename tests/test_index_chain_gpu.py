@@ -140,6 +140,25 @@ def test_gate_edges(cells, paths):
         assert np.array_equal(got.cpu().numpy(), want), residual
 
 
+@pytest.mark.parametrize("paths", [4, 8, 12, 20, 32, 36, 64, 68, 100, 128, 132, 200, 256])
+@pytest.mark.parametrize("cells", [1, 33, 300, 5003, 40000])
+def test_gate_values(cells, paths):
+    """The renormalised gates of every row shape and of partial last tiles: the same sums in the same
+    order and one division; 1e-6 leaves either side a rounding of each."""
+    from brainstorm_b200._C import router as R
+
+    score = np.random.default_rng(7 * cells + paths).random((cells, paths)).astype(np.float32)
+    dev = torch.from_numpy(score).cuda()
+    for k in sorted({1, 2, min(5, paths), paths}):
+        idx, _, gates, mask = R.route_scores(dev, "topk", k, output="seat_indices", with_gates=True,
+                                             with_mask=True)
+        want = oracle.renormalised_topk_score(score, k)
+        np.testing.assert_allclose(gates.cpu().numpy(), want, rtol=1e-6, atol=0)
+        picked = picks_by_key(score, k)
+        assert np.array_equal(mask.cpu().numpy(), picked), k
+        assert np.array_equal(idx.cpu().numpy(), np.cumsum(picked, axis=0) * picked), k
+
+
 def test_gates_go_to_an_array_of_any_float_alignment():
     """Through the C entry point: torch's own allocations are always aligned further."""
     from brainstorm_b200 import _lib
