@@ -483,7 +483,11 @@ int max_row_groups(int ec) {
   return rg < 1 ? 1 : rg;
 }
 
-// rg == 0: pick the tile height that yields at least two CTAs per SM when possible.
+// rg == 0: the tallest tile that still makes a tile for every third SM.  Few large runs beat many
+// small ones: each waits for all before it.  At 8192 x 128, 256 tiles of one 32-cell group against
+// 64 of four: gate 18.5 -> 9.5 us, scan 16.3 -> 8.3; 32768 x 8: 11.2 -> 8.0 and 8.4 -> 7.1.  (Tiles for
+// a quarter or half of the SMs measure the same but for sizes where one of them leaves
+// single-group runs, which keep no block sums: 4096 x 128, half: 11.5 against 9.4.)
 TileGeom make_tile_geom(int64_t cell_num, int path_num, int rg = 0) {
   TileGeom g;
   g.ec = path_num < 256 ? path_num : 256;
@@ -492,7 +496,7 @@ TileGeom make_tile_geom(int64_t cell_num, int path_num, int rg = 0) {
   g.num_groups = (cell_num + kGroupRows - 1) / kGroupRows;
   if (rg == 0) {
     rg = max_row_groups(g.ec);
-    const int64_t want = (int64_t)sm_count() * 2;
+    const int64_t want = sm_count() / 3;
     while (rg > 1 && (g.num_groups + rg - 1) / rg * g.col_chunks < want) rg >>= 1;
   }
   g.rg = rg;
@@ -1183,13 +1187,15 @@ __device__ __forceinline__ void gate_words(const TileCtx& x, int* stage, int* bi
 // have started by construction, so the kernel needs no co-residency guarantee.  A mask that
 // one CTA takes needs neither tickets nor published sums (nor the memset that prepares them).
 //
-// Almost all of the output of a sparse mask is zero and known before any sum is: a tile with at
-// most 1/kSparse of its elements routed is zeroed while the next one is loaded, so that the
+// Almost all of the output of a sparse mask is zero and known before any sum is: a tile with less
+// than 1/kSparse of its elements routed is zeroed while the next one is loaded, so that the
 // reads and most of the writes share the memory system, and what is left after the wait is
-// one 4-byte store per route.  Denser tiles are written whole, 16 bytes at a time, after the
-// wait.  (All tiles written after the wait: 262144 x 128 in 78 us, reads and writes one after
-// the other; now 60 us: 51 for reads and zeros, 5.2 TB/s, the rest for the wait and the routes.
-// From scores, top-1: 112 us with a warp per row in the gate, now 71.)
+// one 4-byte store per route.  Denser tiles, and those of runs with no other tile to load
+// meanwhile, are written whole, 16 bytes at a time, after the wait (256 x 256: scan 9.5 us against
+// 8.2 whole; 524288 x 8, top-1, a route in every 32-byte sector: 20.8 against 18.6).
+// (All tiles written after the wait: 262144 x 128 in 82 us, memset included, reads and writes
+// one after the other; now 62: 51 for reads and zeros, 5.2 TB/s, the rest for the wait and the
+// routes.  From scores, top-1: 114 us with a warp per row in the gate, now 74.)
 //
 // Any path count: V = 4 stages 16 bytes at a time and wants path_num % 4 == 0 and 16-byte
 // aligned arrays, V = 1 stages element by element.
@@ -1208,10 +1214,12 @@ struct ChainArgs {
   int ranges;
 };
 
-constexpr int kChainFly = 8;    // words a thread keeps in flight
+// Words a thread keeps in flight: 8 where block sums leave few of them, 16 where there are none
+// (2048 x 256, 64 runs: gate 13.0 -> 11.8 us; 16 for all cost 524288 x 8, top-4, 3 %).
+constexpr int kFlyBlocks = 8, kFlyRuns = 16;
 constexpr int kBlockRuns = 16;  // a run then adds up at most ranges / 16 + 15 words per column
 constexpr int kChainSpinLimit = 1 << 20;  // default number of polls
-constexpr int kSparse = 8;  // 4-byte stores into zeroed sectors beat whole vectors below this
+constexpr int kSparse = 8;  // 4-byte stores into zeroed sectors beat whole vectors below 1/8
 
 // A published word: the sum (any int32) above a byte that counts the runs in it.
 __device__ __forceinline__ unsigned long long status_word(int value) {
@@ -1503,6 +1511,48 @@ __device__ __forceinline__ void write_routes(const ChainArgs& c, const TileCtx& 
   }
 }
 
+// The sum of every parts-th of the words before a run, from `part` on: whole blocks of runs, then
+// the runs of this run's block.  FLY loads in flight at a time.
+template <int FLY>
+__device__ __forceinline__ int sum_before(const ChainArgs& c, const unsigned long long* blocks,
+                                          const unsigned long long* runs, int my_block, int words,
+                                          int part, int parts) {
+  const int stride = c.t.path_num;
+  int acc = 0;
+  for (int j0 = part; j0 < words; j0 += parts * FLY) {
+    unsigned long long w[FLY];
+    int spins = 0;
+    for (;;) {
+      bool ready = true;
+#pragma unroll
+      for (int u = 0; u < FLY; u++) {
+        const int j = j0 + u * parts;
+        // word j is block j, or run my_block * kBlockRuns + (j - my_block)
+        w[u] = j < words ? status_peek((j < my_block ? blocks : runs) + (int64_t)j * stride)
+                         : (unsigned long long)kBlockRuns;
+      }
+#pragma unroll
+      for (int u = 0; u < FLY; u++) {
+        const int need = j0 + u * parts < my_block ? kBlockRuns : 1;
+        ready = ready && (int)(w[u] & 0xffu) >= need;
+      }
+      if (ready) break;
+      if (++spins > c.spin_limit) {  // give up: report it and carry on with what is there
+        *c.error = 1;
+        if (c.host_error != nullptr) {
+          *reinterpret_cast<volatile int*>(c.host_error) = BRT_ERR_TIMEOUT;
+          __threadfence_system();
+        }
+        break;
+      }
+      __nanosleep(64);
+    }
+#pragma unroll
+    for (int u = 0; u < FLY; u++) acc += status_value(w[u]);
+  }
+  return acc;
+}
+
 template <Mode MODE, bool GATED, int V>
 __global__ void __launch_bounds__(kTileThreads, 2) index_chain_kernel(const ChainArgs c) {
   extern __shared__ __align__(16) int s_dyn[];
@@ -1564,7 +1614,7 @@ __global__ void __launch_bounds__(kTileThreads, 2) index_chain_kernel(const Chai
       gate_words(x, sm.stage(i), bits, sm.sum, sm.routed(i), sm.row_words, c.gate);
     else
       pack_words<V>(x, cols, sm, sm.stage(i), bits, sm.routed(i));
-    const bool sparse = *sm.routed(i) * kSparse <= rows_of(x) * cols;
+    const bool sparse = tile1 - tile0 > 1 && *sm.routed(i) * kSparse < rows_of(x) * cols;
     if (tid == 0) {
       sm.sparse[i] = sparse ? 1 : 0;
       *sm.routed(i + 1) = 0;  // last read before this tile's first barrier, next added to after one
@@ -1588,8 +1638,7 @@ __global__ void __launch_bounds__(kTileThreads, 2) index_chain_kernel(const Chai
         status_add(c.block + (int64_t)my_block * a.path_num + col0 + tid, own);
     }
     __syncthreads();
-    // sum of the runs before this one: whole blocks of them, then those of this run's block.
-    // Thread (part, path) takes every parts-th word, kChainFly loads in flight at a time.
+    // sum of the runs before this one; thread (part, path) takes every parts-th word
     const int parts = kTileThreads / cols;
     const int part = tid / cols;
     const int path = tid - part * cols;
@@ -1598,38 +1647,9 @@ __global__ void __launch_bounds__(kTileThreads, 2) index_chain_kernel(const Chai
       const unsigned long long* const blocks = c.block + col0 + path;
       const unsigned long long* const runs =
           c.status + (int64_t)my_block * (kBlockRuns - 1) * a.path_num + col0 + path;
-      int acc = 0;
-      for (int j0 = part; j0 < words; j0 += parts * kChainFly) {
-        unsigned long long w[kChainFly];
-        int spins = 0;
-        for (;;) {
-          bool ready = true;
-#pragma unroll
-          for (int u = 0; u < kChainFly; u++) {
-            const int j = j0 + u * parts;
-            // word j is block j, or run my_block * kBlockRuns + (j - my_block)
-            w[u] = j < words ? status_peek((j < my_block ? blocks : runs) + (int64_t)j * a.path_num)
-                             : (unsigned long long)kBlockRuns;
-          }
-#pragma unroll
-          for (int u = 0; u < kChainFly; u++) {
-            const int need = j0 + u * parts < my_block ? kBlockRuns : 1;
-            ready = ready && (int)(w[u] & 0xffu) >= need;
-          }
-          if (ready) break;
-          if (++spins > c.spin_limit) {  // give up: report it and carry on with what is there
-            *c.error = 1;
-            if (c.host_error != nullptr) {
-              *reinterpret_cast<volatile int*>(c.host_error) = BRT_ERR_TIMEOUT;
-              __threadfence_system();
-            }
-            break;
-          }
-          __nanosleep(64);
-        }
-#pragma unroll
-        for (int u = 0; u < kChainFly; u++) acc += status_value(w[u]);
-      }
+      const int acc = c.block != nullptr
+                          ? sum_before<kFlyBlocks>(c, blocks, runs, my_block, words, part, parts)
+                          : sum_before<kFlyRuns>(c, blocks, runs, 0, words, part, parts);
       if (acc != 0) atomicAdd(&sm.before[path], acc);
     }
   }
@@ -1790,16 +1810,22 @@ struct ChainPlan {
   size_t smem;
 };
 
-// Masks of at most this many full tiles are scanned by one CTA (per 256 paths): what it saves is
-// the memset in front of the launch, the ticket and the wait.  (256 x 32: 4.7 us of GPU time;
-// 2048 x 32 with 64 CTAs takes 6.0 plus 1.4 for the memset)
+// Masks of at most two full tiles are scanned by one CTA (per 256 paths): what it saves is the
+// memset in front of the launch, the ticket and the wait, and the host the memset's enqueueing.
+// It pays for gates up to one tile of 32 KB (256 x 32: 10.2 -> 6.6 us against a chain; two tiles take
+// 10.0 and 7.7), for scans up to one and a half, or two with few rows (300 x 32: an eager step 26.3
+// and 27.5; 128 x 128: 7.3 and 7.2 of GPU time, the step 26.7 and 28.1; 512 x 32: 7.7 and 6.6,
+// 32.0 and 28.9).
 constexpr int64_t kAloneTiles = 2;
+constexpr int64_t kAloneGate = 8192, kAloneScan = 12288, kAloneCells = 256;
 
-ChainPlan plan_chain(int64_t cell_num, int path_num, bool wide) {
+ChainPlan plan_chain(int64_t cell_num, int path_num, bool wide, bool gated) {
   ChainPlan plan;
   TileGeom& g = plan.geom;
   g = make_tile_geom(cell_num, path_num, max_row_groups(path_num < 256 ? path_num : 256));
-  const bool alone = g.num_tiles <= kAloneTiles;
+  const bool alone = g.num_tiles <= kAloneTiles &&
+                     (cell_num * path_num <= (gated ? kAloneGate : kAloneScan) ||
+                      (!gated && cell_num <= kAloneCells));
   if (!alone) g = make_tile_geom(cell_num, path_num);
   if (!wide) {  // element by element: an odd pitch keeps a column walk free of bank conflicts
     g.ec = round4(g.ec);
@@ -1808,7 +1834,10 @@ ChainPlan plan_chain(int64_t cell_num, int path_num, bool wide) {
   int64_t target = alone ? 1 : (int64_t)sm_count() * kChainCtasPerSm / g.col_chunks;
   if (target < 1) target = 1;
   const int64_t ranges0 = g.num_tiles < target ? g.num_tiles : target;
-  const int64_t tiles_per_cta = (g.num_tiles + ranges0 - 1) / ranges0;
+  int64_t tiles_per_cta = (g.num_tiles + ranges0 - 1) / ranges0;
+  // Runs of a single 32-cell group leave the scratch no room for block sums: no more of them than
+  // SMs, then two a run (8192 x 256: gate 33.3 -> 14.7 us, scan 27.6 -> 12.1).
+  if (g.rg * tiles_per_cta < 2 && ranges0 * g.col_chunks > sm_count()) tiles_per_cta = 2;
   plan.smem = 0;
   if (tiles_per_cta > (int64_t)kChainSmemLimit) return plan;
   plan.tiles_per_cta = (int)tiles_per_cta;
@@ -1816,6 +1845,13 @@ ChainPlan plan_chain(int64_t cell_num, int path_num, bool wide) {
   const size_t smem = chain_smem_ints(g.ec, g.rg, g.pitch, plan.tiles_per_cta) * sizeof(int);
   if (smem <= kChainSmemLimit && (wide || g.col_chunks == 1)) plan.smem = smem;
   return plan;
+}
+
+constexpr size_t kGraphZeros = 4352;
+bool capturing(cudaStream_t stream) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) (void)cudaGetLastError();
+  return status == cudaStreamCaptureStatusActive;
 }
 
 bool forced_split() {
@@ -1871,8 +1907,14 @@ int launch_chain(Mode mode, const ChainPlan& plan, bool wide, const int32_t* mas
   c.t.pitch = g.pitch;
   c.t.num_tiles = g.num_tiles;
   c.t.chunks = g.col_chunks;
-  if (plan.ranges > 1)
-    BRT_CUDA_TRY(cudaMemsetAsync(p, 0, 256 + run_bytes + (blocks ? block_bytes : 0), stream));
+  if (plan.ranges > 1) {
+    size_t zeros = 256 + run_bytes + (blocks ? block_bytes : 0);
+    // A graph's memset node of up to 4 KB takes 1.5 to 2 us longer than a larger one (4.4 and 2.8 us
+    // with a small kernel after it); enqueued eagerly it is the larger that does (4.2 and 6.2).
+    if (zeros <= 4096 && scratch_bytes_for(cell_num, path_num) >= kGraphZeros && capturing(stream))
+      zeros = kGraphZeros;
+    BRT_CUDA_TRY(cudaMemsetAsync(p, 0, zeros, stream));
+  }
   if (mode == Mode::kTag)
     BRT_CUDA_TRY(cudaMemsetAsync(out, 0, (size_t)cell_num * path_num * 4, stream));
   const unsigned grid = (unsigned)plan.ranges * (unsigned)g.col_chunks;
@@ -1910,7 +1952,7 @@ int launch_tiled(Mode mode, const int32_t* mask, int32_t* out, int32_t* loads, i
   // One chained launch when the bit words of a CTA's tiles fit in shared memory, else three
   // launches (pack, scan, expand).  BRT_INDEX_PATH=split forces the latter (for tests).
   if (gate != nullptr || !forced_split() || mode == Mode::kThrottleSeat) {
-    const ChainPlan plan = plan_chain(cell_num, path_num, true);
+    const ChainPlan plan = plan_chain(cell_num, path_num, true, gate != nullptr);
     if (plan.smem != 0)
       return launch_chain(mode, plan, true, mask, out, loads, cell_num, path_num, caps, ncap,
                           capacity_padding, path_wise, prefix, threshold, scratch, stream, gate,
@@ -2048,7 +2090,7 @@ int run_scan(Mode mode, const int32_t* mask, int32_t* out, int32_t* loads, int64
   // paths (9001 x 30: memset and three strip launches took 16.8 us of GPU time, memset and this
   // one 10.4)
   if (!forced_split()) {
-    const ChainPlan plan = plan_chain(cell_num, path_num, false);
+    const ChainPlan plan = plan_chain(cell_num, path_num, false, false);
     if (plan.smem != 0)
       return launch_chain(mode, plan, false, mask, out, loads, cell_num, path_num, caps, ncap,
                           capacity_padding, path_wise, prefix, threshold, scratch, stream);

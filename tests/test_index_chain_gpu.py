@@ -208,6 +208,39 @@ def test_seats_of_an_array_that_is_only_4_byte_aligned_are_refused():
     assert not out.cpu().any()
 
 
+@pytest.mark.parametrize("cells,paths", [(600, 8), (1024, 8), (4096, 4), (16384, 4), (2048, 9),
+                                         (4900, 256)])
+def test_a_captured_scan_clears_its_words_for_every_replay(cells, paths):
+    """Small masks: a graph's memset covers more than the words, within the scratch."""
+    from brainstorm_b200 import _lib
+
+    rng = np.random.default_rng(cells)
+    mask = torch.zeros((cells, paths), dtype=torch.int32, device="cuda")
+    out = torch.empty_like(mask)
+    loads = torch.empty(paths, dtype=torch.int32, device="cuda")
+    nbytes = _lib.query("brt_index_scratch_bytes", cells, paths)
+    room = torch.full((nbytes + 256,), 7, dtype=torch.uint8, device="cuda")
+
+    def scan():
+        _lib.call("brt_generate_indices_and_loads", mask.data_ptr(), out.data_ptr(),
+                  loads.data_ptr(), None, cells, paths, None, 0, 0, 0, 0, room.data_ptr(), nbytes,
+                  _lib.raw_stream(mask.device))
+
+    scan()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        scan()
+    for density in (0.02, 0.5, 0.02):
+        new = (rng.random((cells, paths)) < density).astype(np.int32)
+        mask.copy_(torch.from_numpy(new))
+        graph.replay()
+        want = oracle.generate_indices_and_loads(new)
+        assert np.array_equal(out.cpu().numpy(), want[0])
+        assert np.array_equal(loads.cpu().numpy(), want[1])
+    assert bool((room[nbytes:] == 7).all())
+
+
 # The largest masks of these path counts whose bit words fit a CTA's shared memory on 148 SMs when
 # the base seats of a few tiles at a time are all that is kept beside them.
 @pytest.mark.parametrize("cells,paths", [(56756224, 4), (10381312, 16), (719872, 192),
