@@ -698,16 +698,18 @@ unsigned grid_for_resident(int64_t items, int ctas_per_sm) {
 // SMs work inside one narrow window that advances through memory.  CTAs that stay and stride
 // over the grid's width drift apart, which costs DRAM bandwidth (a plain fill of 800 MB: 5.8 TB/s
 // striding, 7.1 in order).  How many items: enough to hide a CTA's start, few enough to keep the
-// window narrow.  Measured, striding / 2 / 4 / 8 items per warp: 65536 x 64 packed rows of 4 KB
-// 147 / 129 / 133 / 136 us; 64 samples of 3 MiB 185 / 166 / 171 / 185; with capacity padding, where
-// a turn is mostly zero rows, 262144 x 128 181 / 173 / 145 / 150 and 32768 x 32 36.4 / 35.6 / 35.0 /
-// 35.0.  So 2 for packed rows, 4 with slots of a fixed size, and more when an item is less than 2 KB.
+// window narrow.  Measured, striding / 2 / 4 / 8 items per warp, several launches in a graph: 65536 x
+// 64 packed rows of 4 KB 146 / 128 / 131 / 135 us; 64 samples of 3 MiB 185 / 166 / 171 / 185; with
+// capacity padding, where a turn is mostly zero rows, 262144 x 128 194 / 202 / 165 / 165 and 32768 x
+// 32 38.8 / 36.4 / 36.6 / 39.4 (the rule below: 37.5).  So 2 for packed rows, 4 with slots of a fixed
+// size, and more when an item is less than 2 KB.
 // A grid of a few waves takes the count near that which leaves the last wave fullest (20000 rows of
-// 4000 bytes, 32 slots: 4 items make 2.1 waves, 34.9 us; 8 make 1.06, 38.5; 5 make 2.8, 32.5).  When SMs would stay
-// idle although there are rows to move or to zero, the items are spread over one resident wave.
-// (The combine was measured in the same way and keeps its resident CTAs: 26 / 33 / 31 / 33 us at
-// 32768 x 32, 92 / 157 / 127 / 115 at 262144 x 128: its three CTAs per SM have little beside them
-// to cover a start, and it reads more than it writes.)
+// 4000 bytes, 32 slots: 4 items make 2.1 waves, 34.9 us; 8 make 1.06, 38.5; 5 make 2.8, 32.5).
+// When SMs would stay idle although there are rows to move or to zero, the items are spread over
+// one resident wave.
+// (The combine was measured in the same way and keeps its resident CTAs, 26 / 33 / 31 / 33 us at
+// 32768 x 32: its three CTAs per SM have little beside them to cover a start, and it reads more
+// than it writes.)
 unsigned plan_dispatch(MoveArgs& a, int ctas_per_sm) {
   const int64_t items = a.cell_num * a.pieces_per_row;
   const int64_t fills = a.dense_counts != nullptr ? a.total_rows * a.pieces_per_row : 0;

@@ -10,7 +10,7 @@
 // read once, every output row is written once (rows nobody points at as zeros); no atomics on
 // data, no pre-zeroed output.  The input may lie in several pieces (one tensor per path): the
 // list holds addresses, so nothing has to be concatenated first (64 samples of 3 MiB over 8
-// paths: the concatenation alone took 253 us, the sum takes 168).
+// paths: the concatenation alone took 253 us, the sum takes 158).
 //
 // Grouping by a given index: count, scan, fill, per-destination sort of the usually very short
 // lists.  Grouping by tag (the destination of a row is the rank of its tag among the distinct
