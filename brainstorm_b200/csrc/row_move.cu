@@ -75,7 +75,6 @@ __global__ void __launch_bounds__(kThreads, 4) dispatch_seat_kernel(const MoveAr
     const int64_t v0 = (int64_t)piece * (32 * U) + lane;
     const int left = (int)min(a.row_vecs - (int64_t)piece * (32 * U), (int64_t)(32 * U));
     const int live = (left + 31) >> 5;  // rounds of this piece that hold anything
-    constexpr int kRounds = U == kCopyUnroll ? 1 : 4;  // looked at so many at a time
     V regs[U];
     bool loaded = false;
     for (int c = 0; c < chunks; c++) {
@@ -116,7 +115,7 @@ __global__ void __launch_bounds__(kThreads, 4) dispatch_seat_kernel(const MoveAr
               const V* sp = src + src_row * a.row_vecs;
 #pragma unroll
               for (int u = 0; u < U; u++) {
-                if (u % kRounds == 0 && u >= live) break;
+                if (U > kAllRounds && u % 4 == 0 && u >= live) break;
                 if (u * 32 + lane < left) regs[u] = load_stream(sp + v0 + u * 32);
               }
               loaded = true;
@@ -126,14 +125,14 @@ __global__ void __launch_bounds__(kThreads, 4) dispatch_seat_kernel(const MoveAr
               const float g = __shfl_sync(0xffffffffu, gate[j], l);
 #pragma unroll
               for (int u = 0; u < U; u++) {
-                if (u % kRounds == 0 && u >= live) break;
+                if (U > kAllRounds && u % 4 == 0 && u >= live) break;
                 if (u * 32 + lane < left)
                   store_stream(dp + v0 + u * 32, scale_chunk<VB, DT>(regs[u], g));
               }
             } else {
 #pragma unroll
               for (int u = 0; u < U; u++) {
-                if (u % kRounds == 0 && u >= live) break;
+                if (U > kAllRounds && u % 4 == 0 && u >= live) break;
                 if (u * 32 + lane < left) store_stream(dp + v0 + u * 32, regs[u]);
               }
             }
@@ -582,7 +581,6 @@ __global__ void __launch_bounds__(kThreads) combine_seat_kernel(const MoveArgs a
     const int64_t v0 = piece * (32 * U) + lane;
     const int left = (int)min(a.row_vecs - piece * (32 * U), (int64_t)(32 * U));
     const int live = (left + 31) >> 5;  // rounds of this piece that hold anything
-    constexpr int kRounds = U == kCopyUnroll ? 1 : 4;  // looked at so many at a time
     float acc[U][L::N];
 #pragma unroll
     for (int u = 0; u < U; u++)
@@ -603,24 +601,31 @@ __global__ void __launch_bounds__(kThreads) combine_seat_kernel(const MoveArgs a
         const int seat_b = __shfl_sync(0xffffffffu, seat, b);
         const float g = __shfl_sync(0xffffffffu, gate, b);
         const V* sp = src + ((int64_t)s_base[p + b] + seat_b - 1) * a.row_vecs + v0;
-        V row[U];
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-          if (u % kRounds == 0 && u >= live) break;
-          row[u] = u * 32 + lane < left ? load_stream(sp + u * 32) : zero_chunk<V>();
-        }
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-          if (u % kRounds == 0 && u >= live) break;
-          fold_chunk<VB, DT, GMODE>(acc[u], row[u], g);
-        }
         routed = true;
+        if constexpr (U <= kAllRounds) {
+#pragma unroll
+          for (int u = 0; u < U; u++)
+            if (u * 32 + lane < left)
+              fold_chunk<VB, DT, GMODE>(acc[u], load_stream(sp + u * 32), g);
+        } else {
+          V row[U];
+#pragma unroll
+          for (int u = 0; u < U; u++) {
+            if (u % 4 == 0 && u >= live) break;
+            row[u] = u * 32 + lane < left ? load_stream(sp + u * 32) : zero_chunk<V>();
+          }
+#pragma unroll
+          for (int u = 0; u < U; u++) {
+            if (u % 4 == 0 && u >= live) break;
+            fold_chunk<VB, DT, GMODE>(acc[u], row[u], g);
+          }
+        }
       }
     }
     if (routed || !a.is_residual) {
 #pragma unroll
       for (int u = 0; u < U; u++) {
-        if (u % kRounds == 0 && u >= live) break;
+        if (U > kAllRounds && u % 4 == 0 && u >= live) break;
         if (u * 32 + lane < left)
           store_stream(dst + cell * a.row_vecs + v0 + u * 32, pack_chunk<VB, DT>(acc[u]));
       }
@@ -707,10 +712,13 @@ unsigned grid_for_resident(int64_t items, int ctas_per_sm) {
 // 4000 bytes, 32 slots: 4 items make 2.1 waves, 34.9 us; 8 make 1.06, 38.5; 5 make 2.8, 32.5).
 // When SMs would stay idle although there are rows to move or to zero, the items are spread over
 // one resident wave.
+// Rows of more than 256 and at most 1024 bytes that are no multiple of 16 keep one resident wave
+// that strides: striding / in order 42 / 45 us for 79393 x 52 rows of 460 bytes, 51 / 58 for 1000;
+// 220 bytes 39 / 37, 1028 100 / 68.
 // (The combine was measured in the same way and keeps its resident CTAs, 26 / 33 / 31 / 33 us at
 // 32768 x 32: its three CTAs per SM have little beside them to cover a start, and it reads more
 // than it writes.)
-unsigned plan_dispatch(MoveArgs& a, int ctas_per_sm) {
+unsigned plan_dispatch(MoveArgs& a, int ctas_per_sm, int vec_bytes) {
   const int64_t items = a.cell_num * a.pieces_per_row;
   const int64_t fills = a.dense_counts != nullptr ? a.total_rows * a.pieces_per_row : 0;
   const int64_t resident = (int64_t)sm_count() * ctas_per_sm;
@@ -732,7 +740,11 @@ unsigned plan_dispatch(MoveArgs& a, int ctas_per_sm) {
     ctas = ctas_for(turns);
   }
   const int64_t useful = std::min((std::max(items, fills) + kWarps - 1) / kWarps, resident);
-  if (ctas < useful) {
+  if (vec_bytes < 16 && a.row_bytes > 256 && a.row_bytes <= 1024) {
+    ctas = std::max(useful, (int64_t)1);
+    turns = std::max((items + ctas * kWarps - 1) / (ctas * kWarps), (int64_t)1);
+    a.strided = 1;
+  } else if (ctas < useful) {
     ctas = useful;
     turns = std::max((items + ctas * kWarps - 1) / (ctas * kWarps), (int64_t)1);
   }
@@ -772,7 +784,7 @@ void launch_dispatch(const MoveArgs& a, bool is_tag, cudaStream_t st) {
   } else if constexpr (VB == 16 && IS_1D) {
     const size_t smem_async = sizeof(CopyStage) * kWarps * kStages + smem;
     MoveArgs b = a;
-    const unsigned grid = plan_dispatch(b, WEIGHTED ? 3 : 4);
+    const unsigned grid = plan_dispatch(b, WEIGHTED ? 3 : 4, VB);
     if (wide_rows(a.indices, a.gates, dtype_size(DT), a.path_num)) {
       configure_smem<dispatch_seat_async_kernel<DT, WEIGHTED, 4>>(sizeof(CopyStage) * kWarps *
                                                                   kStages);
@@ -784,7 +796,7 @@ void launch_dispatch(const MoveArgs& a, bool is_tag, cudaStream_t st) {
     }
   } else {
     MoveArgs b = a;
-    const unsigned grid = plan_dispatch(b, 4);
+    const unsigned grid = plan_dispatch(b, 4, VB);
     const bool wide = wide_rows(a.indices, a.gates, dtype_size(DT), a.path_num);
     constexpr int U = unroll_of(VB);
     if (U != kCopyUnroll && a.row_vecs <= kShortRow) {
@@ -866,6 +878,8 @@ int launch_combine(const MoveArgs& a, cudaStream_t st) {
     const unsigned grid = grid_for_items(a.cell_num * a.pieces_per_row);
     if (a.row_vecs <= kShortRow)
       combine_seat_kernel<VB, DT, GMODE, kCopyUnroll><<<grid, kThreads, smem, st>>>(a), note_launch();
+    else if (a.row_vecs <= kMidRow)
+      combine_seat_kernel<VB, DT, GMODE, 8><<<grid, kThreads, smem, st>>>(a), note_launch();
     else
       combine_seat_kernel<VB, DT, GMODE, unroll_of(VB)><<<grid, kThreads, smem, st>>>(a), note_launch();
     return BRT_OK;

@@ -19,9 +19,15 @@ constexpr int kCopyUnroll = kPieceVecs / 32;
 constexpr int unroll_of(int vec_bytes) {
   return vec_bytes == 16 ? kCopyUnroll : vec_bytes == 8 ? 8 : 16;
 }
-// Rows of at most this many vectors take the variants with kCopyUnroll rounds (one piece either
-// way; 16 rounds that mostly hold nothing cost rows of 36 and 72 bytes a third of their time).
+// Rows of at most this many vectors take the variants with kCopyUnroll rounds, and in the combine
+// those of at most kMidRow the ones with 8 (one piece either way; 16 rounds that mostly hold
+// nothing cost rows of 36 and 72 bytes a third of their time; 516 bytes: combine 66 -> 52 us).
 constexpr int kShortRow = 32 * kCopyUnroll;
+constexpr int kMidRow = 32 * 8;
+// Up to so many rounds all of them are looked at, each vector under its own condition; more are
+// skipped four at a time.  (A branch out of four rounds keeps their loads from being issued
+// together: 79393 rows of 460 bytes, combine 33 -> 47 us, dispatch 45 -> 56.)
+constexpr int kAllRounds = 8;
 constexpr int kMaxRoutes = 2;      // routes per combine item staged in shared memory (the
                                    // fold below is written out for exactly two)
 constexpr int kFoldVecs = 128;     // vectors per combine item (2 KB at 16 bytes)
@@ -282,7 +288,8 @@ struct MoveArgs {
   int max_path_load;
   int64_t total_rows;  // dispatch: output rows
   int64_t row_bytes = 0;
-  int turns = 0;       // pipelined dispatch: items per warp; a CTA owns kWarps * turns of them
+  int turns = 0;       // dispatch: items per warp; a CTA owns kWarps * turns of them
+  int strided = 0;     // dispatch: those items lie the grid's warps apart
   int is_residual;     // combine only
 };
 
@@ -374,7 +381,8 @@ __device__ __forceinline__ int build_routes(const MoveArgs& a, int64_t cell,
 }
 
 // The items of a warp in a grid whose CTAs own kWarps * turns consecutive ones each, in order:
-// the CTA's first + warp, + kWarps, ...  A cursor past the last one has cell == cell_num.
+// the CTA's first + warp, + kWarps, ...; or, strided, its own number + the warps of the grid, ...
+// A cursor past the last one has cell == cell_num.
 struct WarpItems {
   ItemStep step;
   int64_t cell_num;
@@ -382,12 +390,13 @@ struct WarpItems {
   ItemCursor last;
   __device__ __forceinline__ explicit WarpItems(const MoveArgs& a) {
     const int64_t items = a.cell_num * a.pieces_per_row;
-    step = step_of(kWarps, a.pieces_per_row);
+    const int64_t stride = a.strided ? (int64_t)gridDim.x * kWarps : kWarps;
+    step = step_of(stride, a.pieces_per_row);
     cell_num = a.cell_num;
-    const int64_t span = (int64_t)kWarps * a.turns;
+    const int64_t span = a.strided ? kWarps : (int64_t)kWarps * a.turns;
     const int64_t first = blockIdx.x * span + (threadIdx.x >> 5);
-    const int64_t end = min((int64_t)(blockIdx.x + 1) * span, items);
-    mine = first < end ? (int)((end - first + kWarps - 1) / kWarps) : 0;
+    const int64_t end = a.strided ? items : min((int64_t)(blockIdx.x + 1) * span, items);
+    mine = first < end ? (int)((end - first + stride - 1) / stride) : 0;
     given = 0;
     last = cursor_at(mine > 0 ? first : 0, a.pieces_per_row);
   }

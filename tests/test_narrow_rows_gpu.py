@@ -12,11 +12,24 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("padded", [False, True])
 def test_narrow_rows(width, dtype, padded):
+    check(777, 5, width, dtype, padded)
+
+
+@pytest.mark.parametrize("width,dtype", [(130, torch.bfloat16), (230, torch.float16),
+                                         (301, torch.bfloat16), (500, torch.float16),
+                                         (506, torch.bfloat16), (514, torch.float16),
+                                         (65, torch.float32), (255, torch.float32)])
+@pytest.mark.parametrize("padded", [False, True])
+def test_narrow_rows_of_many_cells(width, dtype, padded):
+    """More items than a resident wave of warps, between and around 256 and 1024 bytes a row."""
+    check(9473, 7, width, dtype, padded)
+
+
+def check(cells, paths, width, dtype, padded):
     from brainstorm_b200._C import router as R
 
     if dtype == torch.float16 and width % 2:
         pytest.skip("odd fp16 cells are refused")
-    cells, paths = 777, 5
     g = torch.Generator(device="cuda").manual_seed(width)
     mask = (torch.rand((cells, paths), generator=g, device="cuda") < 0.4).to(torch.int32)
     indices, loads = R.generate_indices_and_loads(mask)
